@@ -9,6 +9,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <numeric>
 #include <vector>
@@ -84,6 +85,7 @@ struct sg_grid_plan {
     // axis 0: off0[c] = number of (sample, control point) incidences of control points
     // below c (offsets of the fused adjoint's weight list); device, n_basis[0] + 1 values
     int32_t *off0 = nullptr;
+    int64_t line_support = 0;  // Nin = 1 with long supports (adj_line_*): the longest; else 0
     // device status word: SG_ERR_TIMEOUT when a bounded wait of a streaming pass gave up
     int *status = nullptr;
     // adjoint stream chunk size per axis chosen by sg_grid_plan_tune (0: heuristic)
@@ -91,6 +93,16 @@ struct sg_grid_plan {
     // Nin = 2: the fused single-launch path (sg_fused2d.cuh) when the grid fits it
     int32_t strategy = SG_STRATEGY_AUTO;
     bool f2_fwd_ok = false, f2_adj_ok = false;
+    // AUTO: the separable adjoint all the same (large, chunked axis 0).  Its intermediate is
+    // a buffer of its own, in use by one stream at a time: a call on another stream while
+    // the last user's work is in flight, and a call under capture, take the fused path,
+    // which needs none.
+    bool f2_adj_skip = false;
+    void *auto_scratch = nullptr;
+    cudaEvent_t auto_done = nullptr;          // after the last use
+    unsigned long long auto_stream = 0;       // its stream's id
+    bool auto_used = false;
+    std::mutex auto_mutex;
     sg::F2Tiling f2_fwd, f2_adj;
     int64_t f2_adj_target = 0;      // cotangent values per adjoint tile (0: the wave model)
     std::vector<int32_t> lb0_host;  // axis-0 support table (host copy, for re-tiling)
@@ -167,9 +179,10 @@ static int validate_desc(const sg_grid_desc *d) {
 // element offsets, no weights; the adjoint also needs sorted samples on both axes and
 // axis-0 supports that fit a tile.  The grid runs alone, so the tilings are sized for
 // whole waves of the resident units.
+constexpr int64_t kSeparableAdjValues = 1 << 21;
 static void plan_fused_tilings(sg_grid_plan *p) {
     const sg_grid_desc &d = p->desc;
-    p->f2_fwd_ok = p->f2_adj_ok = false;
+    p->f2_fwd_ok = p->f2_adj_ok = p->f2_adj_skip = false;
     if (d.nin != 2 || d.has_weights || d.degree[0] > 3 || d.degree[1] > 3) return;
     if (d.n_samples[0] < 1 || d.n_samples[1] < 1) return;
     if (!f2_offsets_fit(d.n_samples[0], d.n_samples[1], d.n_basis[0], d.n_basis[1], d.nout)) return;
@@ -191,6 +204,13 @@ static void plan_fused_tilings(sg_grid_plan *p) {
                                          f2_align_elems(dt), p->f2_adj_target,
                                          p->f2_adj_target > 0 ? 0 : f2_slots(dt, 1),
                                          p->f2_adj);
+    // AUTO: rows of two tiles and more would be cut into chunks, and chunks along both axes
+    // re-read (and re-sum) their neighbours' boundary spans.  From kSeparableAdjValues on,
+    // two passes are faster: their axis-1 units have a halo along one axis only, and the
+    // intermediate (n1 / ns1 of the cotangent) stays in L2.  (4096, 4096) x 3: Float32 52 us
+    // against 66, Float64 460 against 527; (2048, 2048): 12 against 23.
+    p->f2_adj_skip = d.n_samples[0] >= 2 * np &&
+                     d.n_samples[0] * d.n_samples[1] * d.nout >= kSeparableAdjValues;
 }
 
 static int plan_scan_indices(sg_grid_plan *p, cudaStream_t s) {
@@ -259,6 +279,11 @@ static int plan_scan_indices(sg_grid_plan *p, cudaStream_t s) {
             p->lb1_host = lb;
         }
         if (k == 0) {
+            p->line_support = 0;
+            if (d.nin == 1 && dk <= 5) {
+                const int64_t longest = longest_support(lb.data(), n, dk);
+                if (longest > kLineSupport) p->line_support = longest;
+            }
             const std::vector<int32_t> off = f2_weight_offsets(lb.data(), n, dk);
             dev_free(p->off0);
             p->off0 = nullptr;
@@ -306,6 +331,10 @@ extern "C" int sg_grid_plan_create(const sg_grid_desc *desc, sg_stream_t stream,
         const size_t es = (p->desc.dtype == SG_F64) ? 8 : 4;
         for (int b = 0; b < nbuf && !rc; ++b)
             rc = dev_alloc(&p->scratch[b], (size_t)p->scratch_elems * es, "plan: scratch allocation");
+    }
+    if (!rc && p->f2_adj_skip) {
+        rc = dev_alloc(&p->auto_scratch, (size_t)p->scratch_elems * elem_size(p->desc.dtype), "plan: adjoint intermediate");
+        if (!rc) rc = cuda_check(cudaEventCreateWithFlags(&p->auto_done, cudaEventDisableTiming), "plan: event");
     }
     if (!rc) rc = dev_alloc((void **)&p->status, sizeof(int), "plan: status");
     if (!rc) rc = cuda_check(cudaMemsetAsync(p->status, 0, sizeof(int), s), "plan: status");
@@ -368,6 +397,8 @@ extern "C" void sg_grid_plan_destroy(sg_grid_plan *p) {
         if (p->events[i]) cudaEventDestroy(p->events[i]);
     for (int b = 0; b < 2; ++b)
         dev_free(p->scratch[b]);
+    dev_free(p->auto_scratch);
+    if (p->auto_done) cudaEventDestroy(p->auto_done);
     for (int k = 0; k < SG_MAX_NIN; ++k) {
         dev_free(p->perm[k]);
         dev_free(p->lb[k]);
@@ -379,7 +410,7 @@ extern "C" void sg_grid_plan_destroy(sg_grid_plan *p) {
 extern "C" int64_t sg_grid_plan_workspace_bytes(const sg_grid_plan *p) {
     if (!p) return 0;
     const int nbuf = p->desc.nin >= 3 ? 2 : (p->desc.nin == 2 ? 1 : 0);
-    return nbuf * p->scratch_elems * (p->desc.dtype == SG_F64 ? 8 : 4);
+    return (nbuf + (p->auto_scratch ? 1 : 0)) * p->scratch_elems * (p->desc.dtype == SG_F64 ? 8 : 4);
 }
 
 // derivative_order checks of src/validation.jl:52-88 with the reference's messages.
@@ -421,6 +452,7 @@ static AxisPass axis_pass(const sg_grid_desc &d, const sg_grid_plan *p, int k,
     const size_t bes = (d.dtype == SG_F64) ? 8 : 4;  // basis tables are F32 in BF16 mode
     a.B = (const char *)d.basis_eval[k] + bes * (size_t)(a.ns * (a.d + 1) * (int64_t)ord[k]);
     a.cc = p->tuned_cc[k];
+    a.support = p->line_support;
     return a;
 }
 
@@ -451,6 +483,10 @@ static F2Grid f2_grid(const sg_grid_plan *p, const int32_t *ord, const void *X, 
 
 static bool use_fused(const sg_grid_plan *p, bool ok) {
     return ok && p->strategy != SG_STRATEGY_SEPARABLE;
+}
+static bool use_fused_adjoint(const sg_grid_plan *p) {
+    return use_fused(p, p->f2_adj_ok) &&
+           (p->strategy == SG_STRATEGY_FUSED || !p->f2_adj_skip || !p->auto_scratch);
 }
 
 // Forward pass k (contract axis k) of one derivative order: X -> Y.  Only order[k] is
@@ -605,6 +641,35 @@ extern "C" int sg_evaluate_multi(sg_grid_plan *p, int32_t n_orders, const int32_
                         timer);
 }
 
+// The passes of evaluate_adjoint!, last axis first, through scratch[0] and scratch[1].
+static int separable_adjoint(sg_grid_plan *p, const int32_t *derivative_order, const void *eval_bar,
+                             void *control_points_bar, void *const *scratch, cudaStream_t s, PassTimer &timer) {
+    const sg_grid_desc &d = p->desc;
+    const bool f64 = d.dtype == SG_F64;
+    int rc = SG_OK;
+    const void *X = eval_bar;
+    int buf = 0;
+    for (int k = d.nin - 1; k >= 0; --k) {
+        AxisPass a = axis_pass(d, p, k, derivative_order);
+        a.X = X;
+        a.Y = (k == 0) ? control_points_bar : scratch[buf];
+        buf ^= 1;
+        int64_t M = 1, Q = d.nout;
+        for (int i = 0; i < k; ++i) M *= d.n_samples[i];
+        for (int i = k + 1; i < d.nin; ++i) Q *= d.n_basis[i];
+        a.M = M;
+        a.Q = Q;
+        timer.begin();
+        if (k > 0) rc = f64 ? adj_axis_f64(a, s) : adj_axis_f32(a, s);
+        else if (p->line_support) rc = f64 ? adj_line_f64(a, s) : adj_line_f32(a, s);
+        else rc = f64 ? adj_axis0_f64(a, s) : adj_axis0_f32(a, s);
+        timer.end();
+        if (rc) return rc;
+        X = a.Y;
+    }
+    return SG_OK;
+}
+
 extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_order,
                                    const void *eval_bar, void *control_points_bar,
                                    sg_stream_t stream) {
@@ -618,7 +683,6 @@ extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_or
         return set_error(SG_ERR_INVALID_ARGUMENT, "control_points_bar is NULL");
     cudaStream_t s = (cudaStream_t)stream;
     // SG_BF16_F32 grids take a Float32 cotangent and return a Float32 gradient.
-    const bool f64 = d.dtype == SG_F64;
     int64_t V = 1, NCP = 1;
     for (int k = 0; k < d.nin; ++k) {
         V *= d.n_samples[k];
@@ -631,7 +695,37 @@ extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_or
     if (!eval_bar) return set_error(SG_ERR_INVALID_ARGUMENT, "eval_bar is NULL");
 
     PassTimer timer(p, s);
-    if (use_fused(p, p->f2_adj_ok)) {  // Nin = 2: both axes in one launch
+    bool fused = use_fused_adjoint(p);
+    if (!fused && use_fused(p, p->f2_adj_ok)) {  // AUTO, separable: when its buffer is free
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        rc = cuda_check(cudaStreamIsCapturing(s, &cap), "adjoint: capture status");
+        if (!rc && cap == cudaStreamCaptureStatusNone) {
+            rc = cuda_check(cudaStreamGetId(s, &id), "adjoint: stream id");
+            std::lock_guard<std::mutex> lock(p->auto_mutex);
+            bool free_now = true;
+            if (!rc && p->auto_used && id != p->auto_stream) {
+                const cudaError_t e = cudaEventQuery(p->auto_done);
+                if (e == cudaErrorNotReady) {
+                    (void)cudaGetLastError();
+                    free_now = false;
+                } else {
+                    rc = cuda_check(e, "adjoint: intermediate");
+                }
+            }
+            if (!rc && free_now) {
+                void *const bufs[2] = {p->auto_scratch, nullptr};
+                rc = separable_adjoint(p, derivative_order, eval_bar, control_points_bar, bufs, s, timer);
+                const int rc2 = cuda_check(cudaEventRecord(p->auto_done, s), "adjoint: intermediate");
+                p->auto_used = true;
+                p->auto_stream = id;
+                return rc ? rc : rc2;
+            }
+        }
+        if (rc) return rc;
+        fused = true;
+    }
+    if (fused) {  // Nin = 2: both axes in one launch
         timer.begin();
         rc = f2_launch_grid(d.dtype == SG_F64 ? SG_F64 : SG_F32,
                             f2_grid(p, derivative_order, eval_bar, control_points_bar), p->f2_adj, 1,
@@ -639,26 +733,7 @@ extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_or
         timer.end();
         return rc;
     }
-    const void *X = eval_bar;
-    int buf = 0;
-    for (int k = d.nin - 1; k >= 0; --k) {
-        AxisPass a = axis_pass(d, p, k, derivative_order);
-        a.X = X;
-        a.Y = (k == 0) ? control_points_bar : p->scratch[buf];
-        buf ^= 1;
-        int64_t M = 1, Q = d.nout;
-        for (int i = 0; i < k; ++i) M *= d.n_samples[i];
-        for (int i = k + 1; i < d.nin; ++i) Q *= d.n_basis[i];
-        a.M = M;
-        a.Q = Q;
-        timer.begin();
-        if (k > 0) rc = f64 ? adj_axis_f64(a, s) : adj_axis_f32(a, s);
-        else rc = f64 ? adj_axis0_f64(a, s) : adj_axis0_f32(a, s);
-        timer.end();
-        if (rc) return rc;
-        X = a.Y;
-    }
-    return SG_OK;
+    return separable_adjoint(p, derivative_order, eval_bar, control_points_bar, p->scratch, s, timer);
 }
 
 // Measured choice of the adjoint stream's chunk size per axis k >= 1: each candidate
@@ -728,7 +803,7 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     rc = cuda_check(cudaEventCreate(&e0), "tune: event");
     if (!rc) rc = cuda_check(cudaEventCreate(&e1), "tune: event");
-    if (!rc && use_fused(p, p->f2_adj_ok)) {
+    if (!rc && use_fused_adjoint(p)) {
         rc = tune_fused_adjoint(p, derivative_order, eval_bar, control_points_bar, s, e0, e1, chosen);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -806,6 +881,6 @@ extern "C" int sg_grid_plan_set_strategy(sg_grid_plan *p, int32_t strategy) {
 extern "C" int sg_grid_plan_paths(const sg_grid_plan *p, int32_t *forward, int32_t *adjoint) {
     if (!p) return set_error(SG_ERR_INVALID_ARGUMENT, "plan is NULL");
     if (forward) *forward = use_fused(p, p->f2_fwd_ok) ? SG_STRATEGY_FUSED : SG_STRATEGY_SEPARABLE;
-    if (adjoint) *adjoint = use_fused(p, p->f2_adj_ok) ? SG_STRATEGY_FUSED : SG_STRATEGY_SEPARABLE;
+    if (adjoint) *adjoint = use_fused_adjoint(p) ? SG_STRATEGY_FUSED : SG_STRATEGY_SEPARABLE;
     return SG_OK;
 }

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "sg_passes.cuh"
+#include "sg_stream.cuh"
 #include "sg_fused2d_host.h"
 
 namespace sg {
@@ -286,6 +287,9 @@ struct sg_batch_plan {
     std::vector<int32_t *> off0;                   // device, per grid: fused adjoint weight offsets
     std::vector<void *> fwd_scratch, adj_scratch;  // device, per grid (ping-pong x2)
     std::vector<int64_t> scratch_elems;
+    // Nin = 1 grids with long supports: the longest (else 0).  Their adjoint is one launch
+    // of its own per grid, the per-grid call's (adj_line_*), not a pass of the queue.
+    std::vector<int64_t> line_support;
     // host copies of the pass tables for the three run modes; device copies below
     std::vector<BatchPass> host_passes[4];
     BatchPass *dev_passes[4] = {};
@@ -372,6 +376,7 @@ extern "C" int sg_batch_plan_create(int32_t n_grids, const sg_grid_desc *grids,
     p->fwd_scratch.assign(2 * n_grids, nullptr);
     p->adj_scratch.assign(2 * n_grids, nullptr);
     p->scratch_elems.assign(n_grids, 0);
+    p->line_support.assign(n_grids, 0);
     p->f2_ok.assign(n_grids, 0);
     p->f2_fwd.assign(n_grids, F2Tiling());
     p->f2_adj.assign(n_grids, F2Tiling());
@@ -453,6 +458,8 @@ extern "C" int sg_batch_plan_create(int32_t n_grids, const sg_grid_desc *grids,
             sorted_all = sorted_all && sorted;
             if (k == 0) {  // the fused adjoint's weight-list offsets
                 p->lb0_host[g] = lb;
+                const int64_t longest = d.nin == 1 ? longest_support(lb.data(), n, dk) : 0;
+                if (longest > kLineSupport) p->line_support[g] = longest;
                 const std::vector<int32_t> off = f2_weight_offsets(lb.data(), n, dk);
                 void *doff;
                 rc = batch_alloc(p, &doff, off.size() * 4, "batch: weight offsets");
@@ -641,7 +648,7 @@ static void build_passes(sg_batch_plan *p, const void *const *cps, void *const *
                 if (g < 0 || g >= p->n_grids || level >= p->desc[g].nin) continue;
                 if (grid_fused(p, g)) continue;  // in the fused lists instead
                 if (do_fwd && cps[g] && evals[g]) fwd_pass(g, level);
-                if (do_adj && ebars[g] && cpbars[g]) adj_pass(g, p->desc[g].nin - 1 - level);
+                if (do_adj && ebars[g] && cpbars[g] && !p->line_support[g]) adj_pass(g, p->desc[g].nin - 1 - level);
             }
         }
         p->n_items[mode] = first;
@@ -870,7 +877,10 @@ extern "C" int sg_batch_run(sg_batch_plan *p, int32_t what, sg_stream_t stream) 
     if (!p->arrays_set) return set_error(SG_ERR_INVALID_ARGUMENT, "batch: sg_batch_set_arrays first");
     const auto &h = p->host_passes[what];
     const int64_t nf = (what & 1) ? p->n_f2[0] : 0, na = (what & 2) ? p->n_f2[1] : 0;
-    if (h.empty() && nf == 0 && na == 0)
+    int64_t lines = 0;
+    for (int g = 0; (what & 2) && g < p->n_grids; ++g)
+        lines += p->line_support[g] && p->a_ebar[g] && p->a_cpbar[g] ? 1 : 0;
+    if (h.empty() && nf == 0 && na == 0 && lines == 0)
         return set_error(SG_ERR_INVALID_ARGUMENT, "batch: no arrays for this mode");
     cudaStream_t s = (cudaStream_t)stream;
     int rc = cuda_check(cudaMemsetAsync(p->status, 0, sizeof(int), s), "batch: reset");
@@ -881,6 +891,22 @@ extern "C" int sg_batch_run(sg_batch_plan *p, int32_t what, sg_stream_t stream) 
         rc = cuda_check(cudaMemsetAsync(p->f2_head, 0, sizeof(unsigned long long), s), "batch: reset");
         if (!rc)
             rc = f2_launch_batch(p->dtype, 1, p->dev_f2_grids, p->dev_f2_tiles[1], na, p->f2_head, p->status, s);
+    }
+    for (int g = 0; lines && !rc && g < p->n_grids; ++g) {
+        if (!p->line_support[g] || !p->a_ebar[g] || !p->a_cpbar[g]) continue;
+        const sg_grid_desc &d = p->desc[g];
+        AxisPass a;
+        a.perm = p->perm[g][0];
+        a.lb = p->lb[g][0];
+        a.ns = d.n_samples[0];
+        a.d = d.degree[0];
+        a.n = d.n_basis[0];
+        a.B = (const char *)d.basis_eval[0] + (p->dtype == SG_F64 ? 8 : 4) * (size_t)(a.ns * (a.d + 1) * (int64_t)p->orders[g][0]);
+        a.Q = d.nout;
+        a.X = p->a_ebar[g];
+        a.Y = p->a_cpbar[g];
+        a.support = p->line_support[g];
+        rc = p->dtype == SG_F64 ? adj_line_f64(a, s) : adj_line_f32(a, s);
     }
     if (rc || h.empty()) return rc;
     rc = cuda_check(cudaMemsetAsync(p->done, 0, h.size() * sizeof(int), s), "batch: reset");
@@ -954,7 +980,10 @@ extern "C" int64_t sg_batch_plan_workspace_bytes(const sg_batch_plan *p) {
 
 extern "C" int64_t sg_batch_items(const sg_batch_plan *p, int32_t what) {
     if (!p || what < 1 || what > 3) return 0;
-    return p->n_items[what] + ((what & 1) ? p->n_f2[0] : 0) + ((what & 2) ? p->n_f2[1] : 0);
+    int64_t lines = 0;
+    for (int g = 0; (what & 2) && g < p->n_grids; ++g)
+        lines += p->line_support[g] && p->has_adj && p->a_ebar[g] && p->a_cpbar[g] ? 1 : 0;
+    return p->n_items[what] + ((what & 1) ? p->n_f2[0] : 0) + ((what & 2) ? p->n_f2[1] : 0) + lines;
 }
 
 // One cudaMemcpyAsync per entry, issued from here so that a host-data step of many grids

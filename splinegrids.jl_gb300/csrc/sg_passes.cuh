@@ -6,7 +6,7 @@
 
 #include "sg_contract.cuh"
 #include "sg_warp.cuh"
-#include "sg_stream.cuh"
+#include "sg_ring.cuh"
 
 namespace sg {
 
@@ -29,7 +29,8 @@ struct AxisPass {
     bool final_pass = false;        // writes eval
     int x_dtype = SG_F32;           // element type of X on the axis-0 forward pass
     int *status = nullptr;          // device status word of bounded waits
-    int cc = 0;                     // adjoint stream: control points per chunk (0: heuristic)
+    int cc = 0;                     // adjoint: control points per chunk (0: heuristic)
+    int64_t support = 0;            // Nin = 1 adjoint: samples in the longest support (adj_line_*)
 };
 
 int fwd_axis0_f32(const AxisPass &p, cudaStream_t s);
@@ -40,6 +41,15 @@ int adj_axis_f32(const AxisPass &p, cudaStream_t s);
 int adj_axis_f64(const AxisPass &p, cudaStream_t s);
 int adj_axis0_f32(const AxisPass &p, cudaStream_t s);
 int adj_axis0_f64(const AxisPass &p, cudaStream_t s);
+// Nin = 1 with supports longer than kLineSupport, degrees 0..5 (p.support set)
+int adj_line_f32(const AxisPass &p, cudaStream_t s);
+int adj_line_f64(const AxisPass &p, cudaStream_t s);
+// Samples in the longest support of an axis (lb: its support table).
+inline int64_t longest_support(const int32_t *lb, int64_t n, int d) {
+    int64_t m = 0;
+    for (int64_t c = 0; c < n; ++c) m = lb[c + 1 + d] - lb[c] > m ? lb[c + 1 + d] - lb[c] : m;
+    return m;
+}
 
 constexpr int64_t kMaxGridYZ = 65535;
 constexpr int64_t kNumSMs = 152;                 // GB300
@@ -121,6 +131,7 @@ inline void launch_fwd_axis0_m(const AxisPass &p, cudaStream_t s) {
     else launch_fwd_axis0_d<T, TX, kRational>(p, s);
 }
 
+
 // ------------------------------------------------------------------ forward axis k
 template <typename T, int D, int VEC, int MODE, int NC, bool FINAL, bool ST>
 inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
@@ -140,13 +151,23 @@ inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
     }
 }
 
-// kPlain passes of degree <= 3 run as warp tasks (sg_warp.cuh)
+// kPlain passes of degree <= 5 run as warp tasks (sg_warp.cuh), or one thread per output up
+// to kThreadFwdValues outputs, where the tasks leave most of the GPU idle ((50, 50, 25) x 4,
+// Float64, all three axes: 6.7 us against 24.5; at 6 M outputs the threads take 35 against 19)
+constexpr int64_t kThreadFwdValues = 1 << 19;
 template <typename T, int D, bool ST, bool FINAL>
 inline void launch_fwd_warp(const AxisPass &p, cudaStream_t s) {
     const int64_t gxw = (p.M + warp_width<T>() - 1) / warp_width<T>();
     const int64_t tasks = gxw * ((p.ns + kFwdGridRows - 1) / kFwdGridRows) * p.Q;
     const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (blocks == 0) return;
+    const int64_t total = p.M * p.ns * p.Q;
+    if (total <= kThreadFwdValues) {
+        k_fwd_thread<D, T><<<(unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s>>>(
+            p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
+            (T *)p.Y);
+        return;
+    }
     k_fwd_warp<D, T, ST, FINAL><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
         p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.Q, gxw, (T *)p.Y);
 }
@@ -172,6 +193,19 @@ inline void launch_fwd_axis_d(const AxisPass &p, cudaStream_t s) {
     else launch_fwd_axis_v<T, D, V, true>(p, s);
 }
 
+// degrees 4 and 5 (NURBS take the generic rational kernel)
+template <typename T, int D>
+inline void launch_fwd_axis_plain(const AxisPass &p, cudaStream_t s) {
+    constexpr int V = 16 / (int)sizeof(T);
+    if (vec_width<T>(p) == V) {
+        if (p.final_pass) launch_fwd_warp<T, D, false, true>(p, s);
+        else launch_fwd_warp<T, D, false, false>(p, s);
+    } else {
+        if (p.final_pass) launch_fwd_warp<T, D, true, true>(p, s);
+        else launch_fwd_warp<T, D, true, false>(p, s);
+    }
+}
+
 template <typename T>
 inline void launch_fwd_axis(const AxisPass &p, cudaStream_t s) {
     if (p.mode == kRational && (p.nch + 1 > 4 || p.d > 3)) {
@@ -185,6 +219,8 @@ inline void launch_fwd_axis(const AxisPass &p, cudaStream_t s) {
         case 1: launch_fwd_axis_d<T, 2>(p, s); break;
         case 2: launch_fwd_axis_d<T, 3>(p, s); break;
         case 3: launch_fwd_axis_d<T, 4>(p, s); break;
+        case 4: launch_fwd_axis_plain<T, 5>(p, s); break;
+        case 5: launch_fwd_axis_plain<T, 6>(p, s); break;
         default:  // any degree: runtime-degree kernel, scalar accesses
             if (p.final_pass) launch_fwd_axis_t<T, 0, 1, kPlain, 1, true, false>(p, s);
             else launch_fwd_axis_t<T, 0, 1, kPlain, 1, false, false>(p, s);
@@ -217,76 +253,89 @@ inline void launch_adj_axis_t(const AxisPass &p, cudaStream_t s) {
                                                      (T *)p.Y);
 }
 
-// Warp tasks (sg_warp.cuh): chunks of CC control points, CC as wide as possible (the
-// halo of d knot spans shared with the neighbour chunk is re-read) while the tasks
-// still fill every SM with ~32 warps.
-template <typename T, int D, bool ST>
-inline void launch_adj_warp(const AxisPass &p, cudaStream_t s) {
-    const int64_t gxw = (p.M + warp_width<T>() - 1) / warp_width<T>();
-    const int64_t per_chunk = gxw * p.Q;  // tasks per chunk
-    const int64_t want_chunks = (kNumSMs * 32 * 2 + per_chunk - 1) / per_chunk;
-    int64_t CC = (p.n + want_chunks - 1) / want_chunks;
-    CC = CC < 8 ? 8 : (CC > 64 ? 64 : CC);
-    const int64_t chunks = (p.n + CC - 1) / CC;
-    const int64_t blocks = (per_chunk * chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    if (blocks == 0) return;
-    k_adj_warp<D, T, ST><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        p.idx, p.perm, p.lb, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.Q, (int)CC, gxw,
-        chunks, (T *)p.Y);
+// One thread per output (sg_ring.cuh).
+template <typename T, int D>
+inline void launch_adj_thread(const AxisPass &p, cudaStream_t s) {
+    const int64_t total = p.M * p.n * p.Q;
+    if (total == 0) return;
+    k_adj_thread<D, T><<<(unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s>>>(
+        p.perm, p.lb, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
+        (T *)p.Y);
 }
 
-// Bulk-copy stream (sg_stream.cuh): tiles of up to stream_width<T>() values of m (all
-// of M when it fits) x CC control points x one column; CC as wide as possible while
-// the tiles still give every SM ~2 waves of resident CTAs.
-// Stream tiles of an adjoint pass: m blocks x chunks of CC control points x columns.
-// CC (8..64) is the largest chunk that still gives enough tiles: about 2.5 per SM when
-// a chunk has few tiles (few columns: longer chunks re-read fewer halo rows), two per
-// CTA slot when it has many (long m).
-template <typename T>
-inline int64_t stream_tiles(const AxisPass &p, int64_t &CC, int64_t &chunks) {
-    constexpr int64_t W = stream_width<T>();
-    const int64_t per_chunk = ((p.M + W - 1) / W) * p.Q;
-    const int64_t target = per_chunk <= 64 ? 384 : kNumSMs * 3 * 2;
-    const int64_t min_chunks = (target + per_chunk - 1) / per_chunk;
-    CC = p.n / min_chunks;
-    CC = CC < 8 ? 8 : (CC > 64 ? 64 : CC);
-    if (p.cc > 0) CC = p.cc;  // measured by sg_grid_plan_tune
-    chunks = (p.n + CC - 1) / CC;
-    return per_chunk * chunks;
+// Cotangent values up to which a pass over an axis k >= 1 runs one thread per output: it
+// reads every value d + 1 times, so it loses once the pass is long enough to be bound by
+// memory ((2048, 2048): 31 us against 14; (50, 50, 25) x 4 values: 24 against 50).
+constexpr int64_t kThreadAdjValues = 1 << 20;
+
+// Control points per chunk of an adjoint pass whose units are warps (k_adj_ring,
+// k_adj_cols): per_chunk units per chunk.  A unit walks the rows of CC + d knot spans (the
+// d last ones are read again by the next chunk), every row costs it at least `lat` cycles,
+// and `per` cycles of its SM sub-partition (each has its own FP64 pipe and a quarter of the
+// SM's share of the memory bandwidth), where ceil(units / sub-partitions) units share it.
+// The chunk count with the smallest (CC + d) * max(lat, units per sub-partition * per).
+inline int64_t adj_chunk(const AxisPass &p, int64_t per_chunk, int64_t lat, int64_t per) {
+    int64_t best = p.n, best_cost = INT64_MAX, prev = 0;
+    const int64_t kmax = p.n < 512 ? p.n : 512;
+    for (int64_t k = 1; k <= kmax; ++k) {
+        const int64_t CC = (p.n + k - 1) / k;
+        if (CC == prev) continue;
+        prev = CC;
+        const int64_t units = per_chunk * ((p.n + CC - 1) / CC);
+        const int64_t share = (units + kNumSMs * 4 - 1) / (kNumSMs * 4);
+        const int64_t cost = (CC + p.d) * (lat > share * per ? lat : share * per);
+        if (cost < best_cost && units <= INT32_MAX) {
+            best_cost = cost;
+            best = CC;
+        }
+    }
+    return p.cc > 0 && per_chunk * ((p.n + p.cc - 1) / p.cc) <= INT32_MAX ? p.cc : best;  // cc: measured by sg_grid_plan_tune
 }
+// Cycles of adj_chunk's model, fitted to sweeps on (256, 256) x (4096, 4096) x 3,
+// (2048, 2048) and (1999, 1501) x 3 (each within 5 % of its best chunk count).
+constexpr int64_t kRingLat = 170, kRingPer = 60;
+constexpr int64_t kColsLat = 120, kColsPer = 12;
 
 template <typename T, int D>
-inline void launch_adj_stream(const AxisPass &p, cudaStream_t s) {
-    constexpr int64_t W = stream_width<T>();
-    const int64_t nmb = (p.M + W - 1) / W;
-    const int64_t L = p.M < W ? p.M : W;
-    int64_t CC = 0, chunks = 0;
-    const int64_t tiles = stream_tiles<T>(p, CC, chunks);
-    const int smem = (int)stream_smem_bytes<D, T>();
-    static bool attr_set = false;  // one instance per template instantiation
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_adj_stream<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr_set = true;
-    }
-    if (tiles == 0) return;
-    k_adj_stream<D, T><<<(unsigned)tiles, kStreamThreads, smem, s>>>(
-        p.idx, p.perm, p.lb, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.Q, (int)CC, nmb,
-        chunks, stream_rows_per_stage(L, (int)sizeof(T)), (T *)p.Y, p.status);
+inline void launch_adj_ring(const AxisPass &p, cudaStream_t s) {
+    constexpr int64_t W = warp_width<T>();
+    const int64_t gxw = (p.M + W - 1) / W, per_chunk = gxw * p.Q;
+    if (per_chunk == 0) return;
+    const int64_t CC = adj_chunk(p, per_chunk, kRingLat, kRingPer);
+    const int64_t chunks = (p.n + CC - 1) / CC;
+    k_adj_ring<D, T><<<(unsigned)(per_chunk * chunks), 32, (ring_smem<D, T>()), s>>>(
+        p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, (T *)p.Y);
+}
+template <typename T, int D>
+inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
+    const int64_t gxw = (p.M + 31) / 32, per_chunk = gxw * p.Q;
+    if (per_chunk == 0) return;
+    // Float64: a warp FMA holds a sub-partition's FP64 pipe for 64 cycles
+    const int64_t CC = sizeof(T) == 4 ? adj_chunk(p, per_chunk, kColsLat, kColsPer)
+                                      : adj_chunk(p, per_chunk, 64 * D + kColsLat, 64 * D);
+    const int64_t chunks = (p.n + CC - 1) / CC, units = per_chunk * chunks;
+    k_adj_cols<D, T, 8><<<(unsigned)((units + kColsWarps - 1) / kColsWarps), 32 * kColsWarps, 0, s>>>(
+        p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
 }
 
 template <typename T, int D>
 inline void launch_adj_axis_d(const AxisPass &p, cudaStream_t s) {
-    constexpr int V = 16 / (int)sizeof(T);
     if constexpr (D == 0) {
         launch_adj_axis_t<T, D, 1, false>(p, s);  // runtime degree: one value a thread
     } else {
-        // the stream needs a 16-byte aligned source; with fewer tiles than SMs (few
-        // long columns, e.g. Nout = 1 on a large grid) the warp tasks spread wider
-        int64_t CC = 0, chunks = 0;
-        if ((uintptr_t)p.X % 16 == 0 && stream_tiles<T>(p, CC, chunks) >= kNumSMs)
-            launch_adj_stream<T, D>(p, s);
-        else if (vec_width<T>(p) == V) launch_adj_warp<T, D, false>(p, s);
-        else launch_adj_warp<T, D, true>(p, s);
+        if (p.M * p.ns * p.Q <= kThreadAdjValues && p.M * p.n * p.Q <= INT32_MAX) {
+            launch_adj_thread<T, D>(p, s);
+            return;
+        }
+        if constexpr (sizeof(T) == 4) {
+            // rings copy 16 bytes per lane; Float64 passes are bound by the FP64 pipe, which
+            // the finer units of k_adj_cols fill more evenly
+            if (vec_width<T>(p) == 16 / (int)sizeof(T)) {
+                launch_adj_ring<T, D>(p, s);
+                return;
+            }
+        }
+        launch_adj_cols<T, D>(p, s);
     }
 }
 
@@ -297,6 +346,8 @@ inline void launch_adj_axis(const AxisPass &p, cudaStream_t s) {
         case 1: launch_adj_axis_d<T, 2>(p, s); break;
         case 2: launch_adj_axis_d<T, 3>(p, s); break;
         case 3: launch_adj_axis_d<T, 4>(p, s); break;
+        case 4: launch_adj_axis_d<T, 5>(p, s); break;
+        case 5: launch_adj_axis_d<T, 6>(p, s); break;
         default: launch_adj_axis_d<T, 0>(p, s); break;
     }
 }
@@ -320,37 +371,72 @@ inline void launch_adj_axis0_t(const AxisPass &p, cudaStream_t s) {
                                                        (T *)p.Y);
 }
 
-// degrees <= 3: warp tasks of 32 columns x a chunk of control points (sg_warp.cuh);
-// few columns get short chunks (at least 4 control points) so the tasks fill the GPU
+// degrees <= 5: shared-memory tiles of 32 columns x kA0Cp control points, or one thread
+// per output when half of a tile's lanes would idle or the tiles leave most SMs idle
+// ((1999, 131) x 3: tiles 8 us against 18; (50, 10, 5) x 4: one thread per output 6 against 8)
+constexpr int64_t kA0Tiles = 64;
 template <typename T, int D>
-inline void launch_adj0_warp(const AxisPass &p, cudaStream_t s) {
-    const int64_t groups = (p.Q + 31) / 32;
-    if (groups == 0 || p.n == 0) return;
-    const int64_t want = (kAxis0Tasks + groups - 1) / groups;  // chunks wanted
-    int64_t CC = (p.n + want - 1) / want;
-    CC = CC < 4 ? 4 : CC;
-    const int64_t tasks = groups * ((p.n + CC - 1) / CC);
-    const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    const int smem = kWarpsPerBlock * warp_adj0_smem<D, T>();
-    static bool attr_set = false;  // one instance per template instantiation
-    if (!attr_set) {
-        cudaFuncSetAttribute(k_adj0_warp<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr_set = true;
+inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
+    const int64_t groups = (p.Q + 31) / 32, tiles = groups * ((p.n + kA0Cp - 1) / kA0Cp);
+    if (tiles == 0) return;
+    if ((p.Q < 16 || tiles < kA0Tiles) && p.n * p.Q <= INT32_MAX) {
+        launch_adj_thread<T, D>(p, s);
+        return;
     }
-    if (blocks == 0) return;
-    k_adj0_warp<D, T><<<(unsigned)blocks, 32 * kWarpsPerBlock, smem, s>>>(
-        p.idx, p.perm, p.lb, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.n, p.Q, CC, (T *)p.Y);
+    const int smem = a0_smem<D, T>();
+    k_adj0_tile<D, T><<<(unsigned)tiles, 32 * kA0Warps, smem, s>>>(p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X,
+                                                                   p.n, p.Q, groups, (T *)p.Y);
 }
 
-// Degrees <= 3 run as warp tasks; other degrees (runtime-degree path) as CTA tiles.
+// Higher degrees (runtime-degree path) run as CTA tiles.
 template <typename T>
 inline void launch_adj_axis0(const AxisPass &p, cudaStream_t s) {
     switch (p.d) {
-        case 0: launch_adj0_warp<T, 1>(p, s); break;
-        case 1: launch_adj0_warp<T, 2>(p, s); break;
-        case 2: launch_adj0_warp<T, 3>(p, s); break;
-        case 3: launch_adj0_warp<T, 4>(p, s); break;
+        case 0: launch_adj0<T, 1>(p, s); break;
+        case 1: launch_adj0<T, 2>(p, s); break;
+        case 2: launch_adj0<T, 3>(p, s); break;
+        case 3: launch_adj0<T, 4>(p, s); break;
+        case 4: launch_adj0<T, 5>(p, s); break;
+        case 5: launch_adj0<T, 6>(p, s); break;
         default: launch_adj_axis0_t<T, 0>(p, s); break;
+    }
+}
+
+// Nin = 1 with long supports: one cluster per (control point, column group)
+template <typename T, int D, int QT>
+inline int launch_adj_line_q(const AxisPass &p, cudaStream_t s) {
+    const int64_t units = p.n * ((p.Q + QT - 1) / QT);
+    int S = 1;  // more CTAs per control point while SMs are free and threads have several rounds
+    while (S < 8 && units * S < kNumSMs * 4 && p.support > (int64_t)S * kLineThreads * 8) S *= 2;
+    if (units * S > INT32_MAX) return set_error(SG_ERR_UNSUPPORTED, "adjoint: too many control points");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(units * S));
+    cfg.blockDim = dim3(kLineThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)S;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cuda_check(cudaLaunchKernelEx(&cfg, k_adj_line<D, T, QT>, p.perm, p.lb, (const T *)p.B, p.ns,
+                                         (const T *)p.X, p.n, p.Q, S, (T *)p.Y),
+                      "adjoint launch");
+}
+template <typename T, int D>
+inline int launch_adj_line_d(const AxisPass &p, cudaStream_t s) {
+    return p.Q == 1 ? launch_adj_line_q<T, D, 1>(p, s) : p.Q == 2 ? launch_adj_line_q<T, D, 2>(p, s)
+                                                                  : launch_adj_line_q<T, D, 4>(p, s);
+}
+template <typename T>
+inline int launch_adj_line(const AxisPass &p, cudaStream_t s) {
+    switch (p.d) {
+        case 0: return launch_adj_line_d<T, 1>(p, s);
+        case 1: return launch_adj_line_d<T, 2>(p, s);
+        case 2: return launch_adj_line_d<T, 3>(p, s);
+        case 3: return launch_adj_line_d<T, 4>(p, s);
+        case 4: return launch_adj_line_d<T, 5>(p, s);
+        default: return launch_adj_line_d<T, 6>(p, s);
     }
 }
 

@@ -24,5 +24,6 @@ int adj_axis0_f32(const AxisPass &p, cudaStream_t s) {
     launch_adj_axis0<float>(p, s);
     return cuda_check(cudaGetLastError(), "adj_axis0_f32 launch");
 }
+int adj_line_f32(const AxisPass &p, cudaStream_t s) { return launch_adj_line<float>(p, s); }
 
 }  // namespace sg

@@ -22,5 +22,6 @@ int adj_axis0_f64(const AxisPass &p, cudaStream_t s) {
     launch_adj_axis0<double>(p, s);
     return cuda_check(cudaGetLastError(), "adj_axis0_f64 launch");
 }
+int adj_line_f64(const AxisPass &p, cudaStream_t s) { return launch_adj_line<double>(p, s); }
 
 }  // namespace sg

@@ -451,21 +451,4 @@ adj_stream_tile(int64_t m_lo, int64_t L, int64_t chunk, int64_t q, int R, unsign
         }
 }
 
-// Per-grid kernel: block -> tile (m block fastest, then the chunk, then q).
-template <int D, typename T>
-__global__ void __launch_bounds__(kStreamThreads, 3)
-k_adj_stream(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
-             const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
-             const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int CC, int64_t nmb,
-             int64_t chunks, int R, T *__restrict__ Y, int *status) {
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    const int64_t tile = blockIdx.x;
-    const int64_t mb = tile % nmb, r = tile / nmb;
-    constexpr int64_t W = stream_width<T>();
-    const int64_t m_lo = mb * W;
-    const int64_t L = (M - m_lo) < W ? (M - m_lo) : W;
-    adj_stream_tile<D, T>(m_lo, L, r % chunks, r / chunks, R, s_dyn, idx, perm, lb, B, ns, d, X, M,
-                          n, CC, Y, status);
-}
-
 }  // namespace sg

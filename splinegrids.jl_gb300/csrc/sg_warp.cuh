@@ -244,7 +244,7 @@ fwd_axis_warp(int64_t mw, int64_t jchunk, int rows, int64_t q, int lane, unsigne
               const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns, int d,
               const T *__restrict__ X, int64_t M, int64_t n, T *__restrict__ Y) {
     using DT = DegreeTraits<D>;
-    static_assert(D >= 1 && D <= 4, "warp tasks take degrees 0..3");
+    static_assert(D >= 1 && D <= 6, "forward warp tasks take degrees 0..5");
     constexpr int DA = DT::DA;
     constexpr int DP = DT::DP;
     constexpr int VEC = 16 / (int)sizeof(T);
@@ -278,6 +278,8 @@ fwd_axis_warp(int64_t mw, int64_t jchunk, int rows, int64_t q, int lane, unsigne
                 case 0: win[0] = nxt; break;
                 case 1: win[1 % DA] = nxt; break;
                 case 2: win[2 % DA] = nxt; break;
+                case 4: if constexpr (DA > 4) win[4 % DA] = nxt; break;
+                case 5: if constexpr (DA > 5) win[5 % DA] = nxt; break;
                 default: win[3 % DA] = nxt; break;
             }
             p = (p + 1 == DA) ? 0 : p + 1;
@@ -294,12 +296,13 @@ fwd_axis_warp(int64_t mw, int64_t jchunk, int rows, int64_t q, int lane, unsigne
         T bv[DA];                                                              \
         basis_row<T, DA, DP>(s_B + t * DP, bv);                                \
         stw<FINAL, ST, T, VEC>(yq + M * t, rot_dot_pack<(P) % DA>(win, bv), ln.nv); \
-    }                                                                          \
-    break;
-            case 0: SG_FWD_RUN(0)
-            case 1: SG_FWD_RUN(1)
-            case 2: SG_FWD_RUN(2)
-            default: SG_FWD_RUN(3)
+    }
+            case 0: SG_FWD_RUN(0) break;
+            case 1: SG_FWD_RUN(1) break;
+            case 2: SG_FWD_RUN(2) break;
+            case 4: if constexpr (DA > 4) { SG_FWD_RUN(4) } break;
+            case 5: if constexpr (DA > 5) { SG_FWD_RUN(5) } break;
+            default: SG_FWD_RUN(3) break;
 #undef SG_FWD_RUN
         }
     }
@@ -551,38 +554,6 @@ fwd0_warp(int64_t q0, int64_t s_begin, int64_t s_end, int lane, unsigned char *w
 // segments of the same rows.
 // ---------------------------------------------------------------------------------
 constexpr int kWarpsPerBlock = 4;
-
-template <int D, typename T, bool ST>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-k_adj_warp(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
-           const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
-           const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int CC, int64_t gxw,
-           int64_t chunks, T *__restrict__ Y) {
-    __shared__ __align__(16) unsigned char smem[kWarpsPerBlock * warp_adj_smem<D, T>()];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w;
-    if (task >= gxw * chunks * Q) return;
-    const int64_t mw = task % gxw, r = task / gxw;
-    adj_axis_warp<D, T, ST>(mw, r % chunks, r / chunks, lane, smem + w * warp_adj_smem<D, T>(), idx,
-                            perm, lb, B, ns, d, X, M, n, CC, Y);
-}
-
-// task = column group (fastest) x chunk of CC control points
-template <int D, typename T>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-k_adj0_warp(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
-            const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
-            const T *__restrict__ X, int64_t n, int64_t Q, int64_t CC, T *__restrict__ Y) {
-    extern __shared__ __align__(16) unsigned char s_dyn[];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w;
-    const int64_t groups = (Q + 31) / 32, chunks = (n + CC - 1) / CC;
-    if (task >= groups * chunks) return;
-    const int64_t cg = task % groups, c_lo = (task / groups) * CC;
-    const int64_t c_hi = c_lo + CC < n ? c_lo + CC : n;
-    adj0_warp<D, T>(cg * 32, c_lo, c_hi, lane, s_dyn + w * warp_adj0_smem<D, T>(), idx, perm, lb,
-                    B, ns, d, X, n, Q, Y);
-}
 
 // task = column group (fastest) x chunk of SC samples
 template <int D, typename T>

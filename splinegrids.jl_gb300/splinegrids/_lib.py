@@ -6,6 +6,7 @@ Loading fails loudly when the library has not been built or CUDA is unavailable.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 
 import torch
@@ -170,14 +171,37 @@ def check(rc: int) -> None:
         raise SplineGridsError(rc, last_error())
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", None)
+_streams_ready = False  # CUDA is initialised (by the first stream asked for)
+
+
 def stream_handle(device: torch.device | None = None) -> int:
-    """The current torch CUDA stream of `device` as a cudaStream_t value."""
-    return torch.cuda.current_stream(device).cuda_stream
+    """The current torch CUDA stream of `device` as a cudaStream_t value.  (The stream
+    object of torch.cuda.current_stream costs 3 us a call, its handle alone 0.2.)"""
+    global _streams_ready
+    if device is None and _streams_ready:
+        return _raw_stream(_current_device())
+    h = torch.cuda.current_stream(device).cuda_stream
+    _streams_ready = _raw_stream is not None and _current_device is not None
+    return h
+
+
+# Small constant arrays (sizes, derivative orders): one object per value, which callers
+# only read.
+@functools.lru_cache(maxsize=1024)
+def _i64(vals):
+    return (C.c_int64 * max(1, len(vals)))(*vals)
+
+
+@functools.lru_cache(maxsize=1024)
+def _i32(vals):
+    return (C.c_int32 * max(1, len(vals)))(*vals)
 
 
 def i64_array(vals):
-    return (C.c_int64 * max(1, len(vals)))(*[int(v) for v in vals])
+    return _i64(tuple(map(int, vals)))
 
 
 def i32_array(vals):
-    return (C.c_int32 * max(1, len(vals)))(*[int(v) for v in vals])
+    return _i32(tuple(map(int, vals)))

@@ -26,14 +26,14 @@ def colmajor_strides(shape) -> tuple:
     st, acc = [], 1
     for s in shape:
         st.append(acc)
-        acc *= max(int(s), 1)
+        if s > 1:
+            acc *= int(s)
     return tuple(st)
 
 
 def empty(shape, dtype=torch.float32, device="cuda") -> torch.Tensor:
     shape = tuple(int(s) for s in shape)
-    base = torch.empty(tuple(reversed(shape)), dtype=dtype, device=device)
-    return base.permute(*reversed(range(len(shape)))) if shape else base
+    return torch.empty_strided(shape, colmajor_strides(shape), dtype=dtype, device=device)
 
 
 def zeros(shape, dtype=torch.float32, device="cuda") -> torch.Tensor:
@@ -57,10 +57,15 @@ def from_any(x, dtype=None, device="cuda") -> torch.Tensor:
 
 
 def is_colmajor(t: torch.Tensor) -> bool:
-    if t.numel() <= 1:
-        return True
-    exp = colmajor_strides(t.shape)
-    return all(st == e for st, e, n in zip(t.stride(), exp, t.shape) if n > 1)
+    exp, same, empty = 1, True, False
+    for st, n in zip(t.stride(), t.shape):
+        if n > 1:
+            if st != exp:
+                same = False
+            exp *= n
+        elif n == 0:
+            empty = True
+    return same or empty
 
 
 def ptr(t: torch.Tensor | None, what: str = "array") -> int | None:

@@ -34,8 +34,11 @@ class _Evaluate(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad_eval):
         grid = ctx.grid
-        g = arrays.empty(tuple(grad_eval.shape), grid.dtype, grad_eval.device)
-        g.copy_(grad_eval)  # the cotangent in the library's (column-major) layout
+        g = grad_eval
+        if g.dtype != grid.dtype or not g.is_cuda or not arrays.is_colmajor(g):
+            # the cotangent in the library's (column-major) layout
+            g = arrays.empty(tuple(grad_eval.shape), grid.dtype, grad_eval.device)
+            g.copy_(grad_eval)
         cp_bar = arrays.empty(ctx.cp_shape, grid.dtype, grad_eval.device)
         evaluate_adjoint_(grid, derivative_order=ctx.order, control_points=cp_bar, eval=g)
         return cp_bar, None, None

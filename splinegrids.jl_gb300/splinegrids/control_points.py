@@ -154,14 +154,10 @@ def get_n_control_points(obj) -> int:
 
 # ---------------------------------------------------------------------- device ops
 def _refmat_structs(As, device, dtype):
-    arr = (_lib.RefMat * max(1, len(As)))()
-    keep = []
-    for r, A in enumerate(As):
-        rp, cs, nz = A.device_arrays(device, dtype)
-        keep += [rp, cs, nz]
-        arr[r].m, arr[r].n, arr[r].nnz = A.m, A.n, len(A.nzval)
-        arr[r].row_pointer, arr[r].column_start, arr[r].nzval = (rp.data_ptr(), cs.data_ptr(),
-                                                                  nz.data_ptr())
+    keep = [A.device_arrays(device, dtype) for A in As]
+    arr = (_lib.RefMat * max(1, len(As)))(*[
+        (A.m, A.n, len(A.nzval), rp.data_ptr(), cs.data_ptr(), nz.data_ptr())
+        for A, (rp, cs, nz) in zip(As, keep)])
     return arr, keep
 
 

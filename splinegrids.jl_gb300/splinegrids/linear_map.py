@@ -29,16 +29,43 @@ from .control_points import (LocallyRefinedControlPoints,
 from .spline_grid import (SplineGrid, evaluate_, evaluate_adjoint_, validate_partial_derivatives)
 
 
+def _copy_levels(control_points, x: torch.Tensor, out: bool) -> None:
+    """Between x (flat, [n_control_points, Nout] column-major) and the levels' values, which
+    are its consecutive rows; one column of one level is one copy, all issued by one
+    library call."""
+    ncp, nout = control_points.n_control_points(), control_points.nout
+    vals = [lr.refinement_values for lr in control_points.local_refinements]
+    if nout * len(vals) > 64 or any(v.dtype != x.dtype or not v.is_cuda or not arrays.is_colmajor(v)
+                                    for v in vals):
+        xm = arrays.reshape(x, (ncp, nout))
+        r = 0
+        for v in vals:
+            rows = xm[r:r + v.shape[0]]
+            (rows if out else v).copy_(v if out else rows)
+            r += v.shape[0]
+        return
+    es, x0 = x.element_size(), x.data_ptr()
+    xs, vs, nb = [], [], []
+    r = 0
+    for v in vals:
+        n, v0 = v.shape[0], v.data_ptr()
+        if n:
+            for o in range(nout):
+                xs.append(x0 + es * (r + ncp * o))
+                vs.append(v0 + es * n * o)
+                nb.append(es * n)
+        r += n
+    k = len(nb)
+    if k:
+        dst, src = (xs, vs) if out else (vs, xs)
+        _lib.check(_lib.load().sg_copy_list(k, (C.c_void_p * k)(*dst), (C.c_void_p * k)(*src),
+                                            (C.c_int64 * k)(*nb), _lib.stream_handle()))
+
+
 def _copy_in(control_points, x: torch.Tensor) -> None:
     """copyto!(control_points, reshape(x, n_control_points, Nout)), without allocating."""
     if isinstance(control_points, LocallyRefinedControlPoints):
-        ncp, nout = control_points.n_control_points(), control_points.nout
-        xm = arrays.reshape(x, (ncp, nout))
-        r = 0
-        for lr in control_points.local_refinements:
-            n = lr.n_refined
-            lr.refinement_values.copy_(xm[r:r + n])
-            r += n
+        _copy_levels(control_points, x, False)
     else:
         arrays.vec(obtain(control_points)).copy_(x)
 
@@ -46,13 +73,7 @@ def _copy_in(control_points, x: torch.Tensor) -> None:
 def _copy_out(x: torch.Tensor, control_points) -> None:
     """copyto!(reshape(x, n_control_points, Nout), control_points), without allocating."""
     if isinstance(control_points, LocallyRefinedControlPoints):
-        ncp, nout = control_points.n_control_points(), control_points.nout
-        xm = arrays.reshape(x, (ncp, nout))
-        r = 0
-        for lr in control_points.local_refinements:
-            n = lr.n_refined
-            xm[r:r + n].copy_(lr.refinement_values)
-            r += n
+        _copy_levels(control_points, x, True)
     else:
         x.copy_(arrays.vec(obtain(control_points)))
 

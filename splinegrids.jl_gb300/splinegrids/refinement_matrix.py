@@ -153,7 +153,7 @@ class RefinementMatrix:
 
     def device_arrays(self, device, dtype: torch.dtype):
         """(row_pointer, column_start, nzval) as CUDA tensors, cached per (device, dtype)."""
-        key = (str(device), dtype)
+        key = (device if isinstance(device, str) else str(device), dtype)
         if key not in self._dev:
             self._dev[key] = (torch.as_tensor(self.row_pointer).to(device),
                               torch.as_tensor(self.column_start).to(device),

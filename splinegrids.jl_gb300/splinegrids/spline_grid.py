@@ -174,9 +174,10 @@ class SplineGrid:
             if tv != torch.float32:
                 raise TypeError("bfloat16 control points need a Float32 grid")
             code = _lib.SG_BF16_F32
-        if code not in self._plans:
-            self._plans[code] = _Plan(self, code)
-        return self._plans[code]
+        p = self._plans.get(code)
+        if p is None:
+            p = self._plans[code] = _Plan(self, code)
+        return p
 
     def refresh_plans(self) -> None:
         """Re-read sample indices after set_sample_indices_ changed them."""
@@ -230,6 +231,8 @@ def validate_spline_grid(spline_dimensions, control_points, weights, eval) -> No
 
 def validate_partial_derivatives(grid_or_dims, derivative_order) -> None:
     """validate_partial_derivatives (src/validation.jl:52-88)."""
+    if not any(derivative_order):
+        return  # values alone: available in every dimension
     if isinstance(grid_or_dims, SplineGrid):
         if grid_or_dims.is_nurbs():
             if any(o != 0 for o in derivative_order):
@@ -256,14 +259,16 @@ def evaluate_(grid: SplineGrid, derivative_order=None, control_points=None, eval
     the control points, divided by the weighted denominator for NURBS."""
     order = tuple(derivative_order) if derivative_order is not None else (0,) * grid.nin
     validate_partial_derivatives(grid, order)
-    cp = obtain(grid.control_points if control_points is None else control_points)
+    own = obtain(grid.control_points)
+    cp = own if control_points is None else obtain(control_points)
     ev = grid.eval if eval is None else eval
-    assert tuple(cp.shape) == tuple(obtain(grid.control_points).shape)
-    assert tuple(ev.shape) == tuple(grid.eval.shape)
-    if cp.dtype not in (grid.dtype, torch.bfloat16) or ev.dtype != grid.dtype:
+    dt, cdt = grid.dtype, cp.dtype
+    assert cp.shape == own.shape
+    assert ev.shape == grid.eval.shape
+    if cdt not in (dt, torch.bfloat16) or ev.dtype != dt:
         raise TypeError(f"control points {cp.dtype} / eval {ev.dtype} do not match the grid's "
                         f"{grid.dtype}")
-    plan = grid.plan(cp.dtype)
+    plan = grid.plan(cdt)
     w = arrays.ptr(grid.weights, "weights") if grid.weights is not None else None
     _lib.check(_lib.load().sg_evaluate(plan.handle, _lib.i32_array(order),
                                        arrays.ptr(cp, "control_points"), w,
@@ -322,14 +327,16 @@ def evaluate_adjoint_(grid: SplineGrid, derivative_order=None, control_points=No
     (src/adjoint.jl:42-83): control_points <- M' * eval.  Deterministic gather form."""
     assert not grid.is_nurbs(), "Adjoint evaluation not supported for NURBS."
     order = tuple(derivative_order) if derivative_order is not None else (0,) * grid.nin
-    validate_partial_derivatives(grid.spline_dimensions, order)
-    cp = obtain(grid.control_points if control_points is None else control_points)
+    validate_partial_derivatives(grid, order)
+    own = obtain(grid.control_points)
+    cp = own if control_points is None else obtain(control_points)
     ev = grid.eval if eval is None else eval
-    assert tuple(cp.shape) == tuple(obtain(grid.control_points).shape)
-    assert tuple(ev.shape) == tuple(grid.eval.shape)
-    if cp.dtype != grid.dtype or ev.dtype != grid.dtype:
+    dt = grid.dtype
+    assert cp.shape == own.shape
+    assert ev.shape == grid.eval.shape
+    if cp.dtype != dt or ev.dtype != dt:
         raise TypeError("adjoint arrays must have the grid's float type")
-    plan = grid.plan(grid.dtype)
+    plan = grid.plan(dt)
     _lib.check(_lib.load().sg_evaluate_adjoint(plan.handle, _lib.i32_array(order),
                                                arrays.ptr(ev, "eval"),
                                                arrays.ptr(cp, "control_points"),

@@ -12,17 +12,19 @@
 //
 // Layout of one iteration on the device (vectors stay in HBM, scalars in a device struct):
 //   F = A V                      (caller: the grid's forward evaluation)
-//   U = F/alpha - (alpha/beta) U ; partial sums of U^2       k_lsqr_axpby
-//   beta = ||U||, ||A|| estimate                              k_lsqr_scalar (phase U)
+//   U = F/alpha - (alpha/beta) U ; partial sums of U^2;
+//   beta = ||U||, ||A|| estimate                              k_lsqr_axpby (phase U)
 //   G = A' U                     (caller: the grid's adjoint)
-//   V = G/beta - (beta/alpha) V ; partial sums of V^2, W^2    k_lsqr_axpby
-//   alpha = ||V||, Givens rotation, estimates, stopping rules k_lsqr_scalar (phase V)
-//   X += t1 W ; W = V/alpha + t2 W                            k_lsqr_xw
+//   V = G/beta - (beta/alpha) V ; partial sums of V^2, W^2;
+//   alpha = ||V||, Givens rotation                            k_lsqr_axpby (phase V)
+//   X += t1 W ; W = V/alpha + t2 W ; beside it (block 0) the
+//   estimates and stopping rules                              k_lsqr_xw
+// The last block of a vector pass to finish sums the partials and does the scalar step.
 // U and V are kept unnormalised (u = U/beta, v = V/alpha), so no pass over a vector only
 // rescales it: the scale is folded into the next pass that reads it.  Every reduction is a
 // fixed-order two-level sum (per-block partials, then one block), so a solve is bitwise
 // reproducible.  The iteration can be captured once into a CUDA graph whose body runs in a
-// device-side `while` conditional node: the scalar kernel sets the loop condition after
+// device-side `while` conditional node: the x/w pass sets the loop condition after
 // every step (open while no stopping rule holds, closed when one does, and maxiter is one
 // of the rules), so a whole solve is one graph launch with no host round trip.
 #include <math.h>
@@ -33,7 +35,9 @@ namespace sg {
 namespace {
 
 constexpr int kLsqrThreads = 256;
-constexpr int kLsqrMaxBlocks = 8 * 152;  // grid of the vector passes: at most 8 blocks per SM
+// Grid of the vector passes: two blocks per SM at most.  (4.2 M values, Float32: 304 blocks
+// 10.3 us, 1216 blocks 12.3: every block ends with a Float64 reduction.)
+constexpr int kLsqrMaxBlocks = 2 * 152;
 
 struct LsqrState {
     // Golub-Kahan scalars of the current iteration
@@ -41,12 +45,14 @@ struct LsqrState {
     // QR recurrence (paper section 4.1) and the norm / condition estimates (section 5)
     double rhobar, phibar, anorm, acond, ddnorm, res2, xnorm, xxnorm, z, cs2, sn2;
     double bnorm, rnorm, arnorm;
-    // coefficients of the vector passes, written by the scalar kernel
+    // coefficients of the vector passes, written by the scalar step
     double cu_a, cu_b, cv_a, cv_b, t1, t2, inv_alpha;
     // parameters
     double damp, atol, btol, ctol, eps;
+    // between the two parts of a step (the scalar step and its estimates)
+    double theta, tau, gambar, rhs, zbar;
     long long itn, maxiter;
-    int istop, done;
+    int istop, done, estimate;
 };
 
 int n_blocks(int64_t n) {
@@ -71,41 +77,150 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
     return r;  // valid in thread 0
 }
 
-// U = b, and (n-space) X = 0, W = 0; partial sums of b^2.
+// Sum of squares.  Float64 values: Float64 FMAs.  Float32 values: the Float64 pipe (two
+// lanes per SM and clock, conversions included) would be the bound of the whole pass, so the
+// squares are summed without error in three Float32 words: r^2 = p + e exactly (FMA), and
+// each addition keeps its rounding error in the next word (TwoSum, Knuth, TAOCP 4.2.2).  The
+// three words carry about 70 bits, more than the Float64 sum they replace (53).  Groups of
+// values whose squares or errors could leave Float32's range go the Float64 way.
+// Measured on 4.2 M Float32 values (the pass U = a F + b U with its sum): 24.6 -> 10.3 us.
+template <typename T>
+struct SumSq {
+    double s = 0.0;
+    template <int N>
+    __device__ __forceinline__ void add(const T (&v)[N]) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) s += (double)v[k] * (double)v[k];
+    }
+    __device__ __forceinline__ double get() const { return s; }
+};
+template <>
+struct SumSq<float> {
+    double s = 0.0;
+    float w0 = 0.f, w1 = 0.f, w2 = 0.f;
+    static __device__ __forceinline__ float two_sum(float a, float b, float &err) {
+        const float r = __fadd_rn(a, b), bb = __fsub_rn(r, a);
+        err = __fadd_rn(__fsub_rn(a, __fsub_rn(r, bb)), __fsub_rn(b, bb));
+        return r;
+    }
+    template <int N>
+    __device__ __forceinline__ void add(const float (&v)[N]) {
+        // the errors of squares far below the group's largest may be lost: they are below
+        // 2^-65 of the sum
+        float m = 0.f;
+#pragma unroll
+        for (int k = 0; k < N; ++k) m = fmaxf(m, fabsf(v[k]));
+        if ((m >= 0x1p-40f && m <= 0x1p50f) || m == 0.f) {  // (a NaN stays one in p)
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const float p = __fmul_rn(v[k], v[k]), e = __fmaf_rn(v[k], v[k], -p);
+                float t, u, x;
+                w0 = two_sum(w0, p, t);
+                t = two_sum(t, e, u);
+                w1 = two_sum(w1, t, x);
+                w2 = __fadd_rn(w2, __fadd_rn(u, x));
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < N; ++k) s += (double)v[k] * (double)v[k];
+        }
+    }
+    __device__ __forceinline__ double get() const { return ((double)w2 + (double)w1) + (double)w0 + s; }
+};
+
+enum { kPhaseStart = 0, kPhaseU = 1, kPhaseV = 2 };
+
+// What the vector passes share: the state, the blocks' partial sums and the counter of
+// blocks that have finished.
+struct LsqrShared {
+    LsqrState *st;
+    double *part, *part2;  // [kLsqrMaxBlocks] each
+    unsigned *count;       // zero between passes
+    int *skip_xw;
+    cudaGraphConditionalHandle cond;
+    int has_cond;
+};
+
+template <typename T>
+__device__ void lsqr_scalar(const LsqrShared &sh, double s, double s2, int phase);
+
+// End of a vector pass: the block's sums go to part / part2; the last block to finish adds
+// all of them in a fixed order and does the pass' scalar step.
+template <typename T>
+__device__ __forceinline__ void lsqr_finish(const LsqrShared &L, double s, double s2, bool two, int phase) {
+    __shared__ double sh[kLsqrThreads / 32];
+    __shared__ int last;
+    s = block_sum(s, sh);
+    if (two) s2 = block_sum(s2, sh);
+    if (threadIdx.x == 0) {
+        L.part[blockIdx.x] = s;
+        if (two) L.part2[blockIdx.x] = s2;
+        __threadfence();
+        last = atomicAdd(L.count, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+        a += __ldcg(L.part + i);
+        if (two) b += __ldcg(L.part2 + i);
+    }
+    a = block_sum(a, sh);
+    if (two) b = block_sum(b, sh);
+    if (threadIdx.x == 0) *L.count = 0;
+    if (threadIdx.x < 32) {  // block_sum's result is thread 0's
+        a = __shfl_sync(0xffffffffu, a, 0);
+        b = __shfl_sync(0xffffffffu, b, 0);
+        lsqr_scalar<T>(L, a, b, phase);
+    }
+}
+
+// U = b, and (n-space) X = 0, W = 0; the sum of b^2 and the start of the recurrence.
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict__ b, T *__restrict__ U, int64_t m,
                                                 T *__restrict__ X, T *__restrict__ W, int64_t n,
-                                                double *__restrict__ part) {
-    __shared__ double sh[kLsqrThreads / 32];
+                                                LsqrShared L) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += stride) {
-        const T v = b[i];
-        U[i] = v;
-        s += (double)v * (double)v;
+    SumSq<T> s;
+    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (; i + 3 * stride < m; i += 4 * stride) {
+        T v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = b[i + k * stride];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) U[i + k * stride] = v[k];
+        s.add(v);
+    }
+    for (; i < m; i += stride) {
+        const T v[1] = {b[i]};
+        U[i] = v[0];
+        s.add(v);
     }
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         X[i] = T(0);
         W[i] = T(0);
     }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    lsqr_finish<T>(L, s.get(), 0.0, false, kPhaseStart);
 }
 
-// Y = a * Xin + b * Y with (a, b) = coef[0..1] read from the state; partial sums of the new
-// Y^2 into part[block], and (when W is given) of W^2 into part2[block].
+// Y = a * Xin + b * Y with (a, b) the state's coefficients of the phase; the sums of the new
+// Y^2 and (phase V) of W^2, then the phase's scalar step.
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_axpby(const T *__restrict__ Xin, T *__restrict__ Y, int64_t n,
-                                                const double *__restrict__ coef,
-                                                const int *__restrict__ done,
-                                                double *__restrict__ part,
-                                                const T *__restrict__ W, double *__restrict__ part2) {
-    __shared__ double sh[kLsqrThreads / 32];
-    if (*done) return;  // the solve has stopped: leave every vector as it is
-    const T a = (T)coef[0], bb = (T)coef[1];
+                                                const T *__restrict__ W, int phase, LsqrShared L) {
+    const LsqrState *st = L.st;
+    if (st->done) {  // the solve has stopped: leave every vector as it is
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            *L.skip_xw = 1;
+            if (L.has_cond) cudaGraphSetConditional(L.cond, 0);
+        }
+        return;
+    }
+    const T a = (T)(phase == kPhaseU ? st->cu_a : st->cv_a), bb = (T)(phase == kPhaseU ? st->cu_b : st->cv_b);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    double s = 0.0, s2 = 0.0;
+    SumSq<T> s, s2;
     int64_t i = i0;
     // four independent elements in flight per thread
     for (; i + 3 * stride < n; i += 4 * stride) {
@@ -114,80 +229,63 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_axpby(const T *__restrict
         for (int k = 0; k < 4; ++k) { x[k] = Xin[i + k * stride]; y[k] = Y[i + k * stride]; }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const T r = bb == T(0) ? a * x[k] : fma(a, x[k], bb * y[k]);
-            Y[i + k * stride] = r;
-            s += (double)r * (double)r;
+            y[k] = bb == T(0) ? a * x[k] : fma(a, x[k], bb * y[k]);
+            Y[i + k * stride] = y[k];
         }
+        s.add(y);
     }
     for (; i < n; i += stride) {
-        const T r = bb == T(0) ? a * Xin[i] : fma(a, Xin[i], bb * Y[i]);
-        Y[i] = r;
-        s += (double)r * (double)r;
+        const T r[1] = {bb == T(0) ? a * Xin[i] : fma(a, Xin[i], bb * Y[i])};
+        Y[i] = r[0];
+        s.add(r);
     }
     if (W) {
         for (int64_t j = i0; j < n; j += stride) {
-            const double w = (double)W[j];
-            s2 += w * w;
+            const T w[1] = {W[j]};
+            s2.add(w);
         }
     }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-    if (W) {
-        s2 = block_sum(s2, sh);
-        if (threadIdx.x == 0) part2[blockIdx.x] = s2;
-    }
+    lsqr_finish<T>(L, s.get(), s2.get(), W != nullptr, phase);
 }
-
-// X += t1 W ; W = inv_alpha V + t2 W.
-template <typename T>
-__global__ void __launch_bounds__(kLsqrThreads) k_lsqr_xw(const T *__restrict__ V, T *__restrict__ W, T *__restrict__ X,
-                                             int64_t n, const LsqrState *__restrict__ st,
-                                             const int *__restrict__ skip) {
-    if (*skip) return;
-    const T t1 = (T)st->t1, t2 = (T)st->t2, ia = (T)st->inv_alpha;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const T w = W[i];
-        X[i] = fma(t1, w, X[i]);
-        W[i] = fma(ia, V[i], t2 * w);
-    }
-}
-
-// Sum of part[0..nb) in a fixed order by one block.
-__device__ double sum_partials(const double *part, int nb, double *sh) {
-    double s = 0.0;
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) s += part[i];
-    return block_sum(s, sh);
-}
-
-enum { kPhaseStart = 0, kPhaseU = 1, kPhaseV = 2 };
 
 template <typename T>
 __device__ bool one_plus_is_one(double t) {
     return (T)1 + (T)t <= (T)1;
 }
 
-// One block.  Phase start: beta = ||b||.  Phase U: beta = ||U||.  Phase V: alpha = ||V||,
-// the QR step, estimates and stopping rules (first call: the initialisation).
-template <typename T>
-__global__ void __launch_bounds__(kLsqrThreads) k_lsqr_scalar(LsqrState *st, const double *__restrict__ part,
-                                                 const double *__restrict__ part2, int nb,
-                                                 int nb2, int phase, int *skip_xw,
-                                                 cudaGraphConditionalHandle cond, int has_cond) {
-    __shared__ double sh[kLsqrThreads / 32];
-    if (phase != kPhaseStart && st->done) {
-        if (threadIdx.x == 0) {
-            *skip_xw = 1;
-            if (has_cond) cudaGraphSetConditional(cond, 0);
-        }
-        return;
+// One Float64 division or square root is a chain of dozens of dependent operations on a
+// slow pipe, and a step has about thirty of them.  The warp does the independent ones of
+// a level together, one per lane, and every lane gets all results.
+struct Lanes {
+    int lane;
+    // r[i] = n_i / d_i
+    __device__ __forceinline__ void div(double n0, double d0, double n1, double d1, double n2, double d2, double n3,
+                                        double d3, double n4, double d4, double n5, double d5, double n6, double d6,
+                                        double (&r)[7]) const {
+        const double n = lane == 0 ? n0 : lane == 1 ? n1 : lane == 2 ? n2 : lane == 3 ? n3 : lane == 4 ? n4
+                                                                          : lane == 5 ? n5 : n6;
+        const double d = lane == 0 ? d0 : lane == 1 ? d1 : lane == 2 ? d2 : lane == 3 ? d3 : lane == 4 ? d4
+                                                                          : lane == 5 ? d5 : d6;
+        const double v = n / d;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) r[i] = __shfl_sync(0xffffffffu, v, i);
     }
-    const double s = sum_partials(part, nb, sh);
-    double s2 = 0.0;
-    if (phase == kPhaseV) s2 = sum_partials(part2, nb2, sh);
-    if (threadIdx.x != 0) return;
-    LsqrState S = *st;
-    *skip_xw = 1;
+    __device__ __forceinline__ void root(double a, double b, double c, double (&r)[4], double d = 1.0) const {
+        const double v = sqrt(lane == 0 ? a : lane == 1 ? b : lane == 2 ? c : d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, v, i);
+    }
+};
+
+// The scalar step of a phase, by one warp (every lane holds every value).  Phase start: beta =
+// ||b||.  Phase U: beta = ||U||.  Phase V: alpha = ||V||, the QR step, estimates and stopping
+// rules (first call: the initialisation).  s, s2: the pass' sums of squares.
+template <typename T>
+__device__ void lsqr_scalar(const LsqrShared &L, double s, double s2, int phase) {
+    LsqrState S = *L.st;
+    const Lanes W{(int)(threadIdx.x & 31)};
+    double q[7], r[4];
+    int skip = 1;
     if (phase == kPhaseStart) {
         // a new solve: the recurrence starts afresh, the parameters stay
         S.alpha = S.rhobar = S.phibar = S.anorm = S.acond = S.ddnorm = S.res2 = 0.0;
@@ -196,6 +294,7 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_scalar(LsqrState *st, con
         S.t1 = S.t2 = S.inv_alpha = S.cu_a = S.cu_b = 0.0;
         S.istop = 0;
         S.done = 0;
+        S.estimate = 0;
         S.beta = sqrt(s);
         S.bnorm = S.beta;
         S.cv_a = S.beta > 0.0 ? 1.0 / S.beta : 0.0;  // V = A'u = G / beta
@@ -206,8 +305,9 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_scalar(LsqrState *st, con
         // paper section 5.1: ||B_k||_F accumulates alpha_k^2 + beta_{k+1}^2 (+ damp^2)
         if (beta > 0.0) {
             S.anorm = sqrt(S.anorm * S.anorm + S.alpha * S.alpha + beta * beta + S.damp * S.damp);
-            S.cv_a = 1.0 / beta;                                 // A'u = G / beta
-            S.cv_b = S.alpha > 0.0 ? -beta / S.alpha : 0.0;      // - beta v = -(beta/alpha) V
+            W.div(1.0, beta, -beta, S.alpha, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, q);
+            S.cv_a = q[0];                            // A'u = G / beta
+            S.cv_b = S.alpha > 0.0 ? q[1] : 0.0;      // - beta v = -(beta/alpha) V
         } else {
             S.cv_a = 0.0;  // u is zero: v keeps its value (the paper's "if beta > 0")
             S.cv_b = 1.0;
@@ -216,88 +316,127 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_scalar(LsqrState *st, con
     } else if (S.itn == 0) {
         // initialisation (paper section 4.1, step 1): alpha_1 v_1 = A' u_1, w_1 = v_1
         const double alpha = sqrt(s);
+        W.div(1.0, alpha, -alpha, S.beta, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, q);
         S.alpha = alpha;
         S.rhobar = alpha;
         S.phibar = S.beta;
         S.rnorm = S.beta;
         S.arnorm = alpha * S.beta;
-        S.inv_alpha = alpha > 0.0 ? 1.0 / alpha : 0.0;
+        S.inv_alpha = alpha > 0.0 ? q[0] : 0.0;
         S.t1 = 0.0;
         S.t2 = 0.0;
         S.cu_a = S.inv_alpha;  // A v = F / alpha
-        S.cu_b = S.beta > 0.0 ? -alpha / S.beta : 0.0;
-        *skip_xw = 0;
+        S.cu_b = S.beta > 0.0 ? q[1] : 0.0;
+        skip = 0;
         if (S.arnorm == 0.0) {  // x = 0 solves the problem exactly
             S.istop = 0;
             S.done = 1;
         }
         S.itn = 1;
     } else {
-        // with beta == 0 the previous v was kept, so alpha is unchanged
-        const double alpha = S.beta > 0.0 ? sqrt(s) : S.alpha;
         const double beta = S.beta;
         // the damped system's extra rotation (paper section 4.3)
-        const double dampsq = S.damp * S.damp;
-        const double rhobar1 = sqrt(S.rhobar * S.rhobar + dampsq);
-        const double cs1 = S.rhobar / rhobar1, sn1 = S.damp / rhobar1;
+        const double rho1sq = S.rhobar * S.rhobar + S.damp * S.damp;
+        W.root(s, rho1sq, rho1sq + beta * beta, r);
+        // with beta == 0 the previous v was kept, so alpha is unchanged
+        const double alpha = beta > 0.0 ? r[0] : S.alpha;
+        const double rhobar1 = r[1], rho = r[2];
+        W.div(S.rhobar, rhobar1, S.damp, rhobar1, 1.0, alpha, -alpha, beta, rhobar1, rho, beta, rho, s2, rho * rho, q);
+        const double cs1 = q[0], sn1 = q[1];
+        S.inv_alpha = alpha > 0.0 ? q[2] : 0.0;
+        S.cu_a = S.inv_alpha;
+        S.cu_b = beta > 0.0 ? q[3] : 0.0;
         const double psi = sn1 * S.phibar;
         const double phibar0 = cs1 * S.phibar;
         // plane rotation eliminating beta (section 4.1, step 4)
-        const double rho = sqrt(rhobar1 * rhobar1 + beta * beta);
-        const double cs = rhobar1 / rho, sn = beta / rho;
+        const double cs = q[4], sn = q[5];
         const double theta = sn * alpha;
-        S.rhobar = -cs * alpha;
         const double phi = cs * phibar0;
+        S.rhobar = -cs * alpha;
         S.phibar = sn * phibar0;
-        const double tau = sn * phi;
-        // x and w update coefficients (step 5)
-        S.t1 = phi / rho;
-        S.t2 = -theta / rho;
-        S.inv_alpha = alpha > 0.0 ? 1.0 / alpha : 0.0;
+        S.tau = sn * phi;
         // estimates (section 5): ||D_k||_F from ||w_k||^2 / rho_k^2, ||x|| via the
         // rotation of the lower bidiagonal factor
-        S.ddnorm += s2 / (rho * rho);
-        const double delta = S.sn2 * rho;
-        const double gambar = -S.cs2 * rho;
-        const double rhs = phi - delta * S.z;
-        const double zbar = rhs / gambar;
-        S.xnorm = sqrt(S.xxnorm + zbar * zbar);
-        const double gamma = sqrt(gambar * gambar + theta * theta);
-        S.cs2 = gambar / gamma;
-        S.sn2 = theta / gamma;
-        S.z = rhs / gamma;
-        S.xxnorm += S.z * S.z;
-        S.acond = S.anorm * sqrt(S.ddnorm);
+        S.ddnorm += q[6];
         S.res2 += psi * psi;
-        S.rnorm = sqrt(S.phibar * S.phibar + S.res2);
-        S.arnorm = alpha * fabs(tau);
+        S.theta = theta;
+        S.gambar = -S.cs2 * rho;
+        S.rhs = phi - S.sn2 * rho * S.z;
+        // x and w update coefficients (step 5)
+        W.div(phi, rho, -theta, rho, S.rhs, S.gambar, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, q);
+        S.t1 = q[0];
+        S.t2 = q[1];
+        S.zbar = q[2];
         S.alpha = alpha;
-        S.cu_a = S.inv_alpha;
-        S.cu_b = beta > 0.0 ? -alpha / beta : 0.0;
-        *skip_xw = 0;
-        // stopping rules (section 6); the later assignment wins, as in the paper's order
-        const double test1 = S.rnorm / S.bnorm;
-        const double test2 = S.arnorm / (S.anorm * S.rnorm + S.eps);
-        const double test3 = 1.0 / (S.acond + S.eps);
-        const double t1s = test1 / (1.0 + S.anorm * S.xnorm / S.bnorm);
-        const double rtol = S.btol + S.atol * S.anorm * S.xnorm / S.bnorm;
-        int istop = 0;
-        if (S.itn >= S.maxiter) istop = 7;
-        if (one_plus_is_one<T>(test3)) istop = 6;
-        if (one_plus_is_one<T>(test2)) istop = 5;
-        if (one_plus_is_one<T>(t1s)) istop = 4;
-        if (test3 <= S.ctol) istop = 3;
-        if (test2 <= S.atol) istop = 2;
-        if (test1 <= rtol) istop = 1;
-        if (!(isfinite(alpha) && isfinite(beta) && isfinite(S.rnorm))) istop = -1;
-        S.istop = istop;
-        if (istop != 0) S.done = 1;
-        else S.itn += 1;
+        S.estimate = 1;  // the x/w pass does the rest beside its vectors
+        skip = 0;
     }
-    *st = S;
+    if (W.lane != 0) return;
+    *L.st = S;
+    *L.skip_xw = skip;
     // The loop handle starts each launch at 0 (no iteration): the initialisation opens
-    // the loop, the step that meets a stopping rule closes it.  Only phase V sets it.
-    if (has_cond && phase == kPhaseV) cudaGraphSetConditional(cond, S.done ? 0u : 1u);
+    // the loop, the step that meets a stopping rule closes it.
+    if (L.has_cond && phase == kPhaseV && !S.estimate) cudaGraphSetConditional(L.cond, S.done ? 0u : 1u);
+}
+
+// The rest of phase V, by one warp: the norm and condition estimates and the stopping rules.
+// Nothing in the x/w update waits for them.
+template <typename T>
+__device__ void lsqr_estimate(const LsqrShared &L) {
+    LsqrState S = *L.st;
+    const Lanes W{(int)(threadIdx.x & 31)};
+    double q[7], r[4];
+    W.root(S.gambar * S.gambar + S.theta * S.theta, S.phibar * S.phibar + S.res2, S.xxnorm + S.zbar * S.zbar, r,
+           S.ddnorm);
+    const double gamma = r[0];
+    S.rnorm = r[1];
+    S.xnorm = r[2];
+    S.acond = S.anorm * r[3];
+    S.arnorm = S.alpha * fabs(S.tau);
+    W.div(S.gambar, gamma, S.theta, gamma, S.rhs, gamma, S.rnorm, S.bnorm, S.arnorm, S.anorm * S.rnorm + S.eps, 1.0,
+          S.acond + S.eps, S.anorm * S.xnorm, S.bnorm, q);
+    S.cs2 = q[0];
+    S.sn2 = q[1];
+    S.z = q[2];
+    S.xxnorm += S.z * S.z;
+    // stopping rules (section 6); the later assignment wins, as in the paper's order
+    const double test1 = q[3], test2 = q[4], test3 = q[5];
+    W.div(test1, 1.0 + q[6], S.atol * S.anorm * S.xnorm, S.bnorm, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, 1.0, q);
+    const double t1s = q[0], rtol = S.btol + q[1];
+    int istop = 0;
+    if (S.itn >= S.maxiter) istop = 7;
+    if (one_plus_is_one<T>(test3)) istop = 6;
+    if (one_plus_is_one<T>(test2)) istop = 5;
+    if (one_plus_is_one<T>(t1s)) istop = 4;
+    if (test3 <= S.ctol) istop = 3;
+    if (test2 <= S.atol) istop = 2;
+    if (test1 <= rtol) istop = 1;
+    if (!(isfinite(S.alpha) && isfinite(S.beta) && isfinite(S.rnorm))) istop = -1;
+    S.istop = istop;
+    if (istop != 0) S.done = 1;
+    else S.itn += 1;
+    S.estimate = 0;
+    if (W.lane != 0) return;
+    *L.st = S;
+    if (L.has_cond) cudaGraphSetConditional(L.cond, S.done ? 0u : 1u);
+}
+
+// X += t1 W ; W = inv_alpha V + t2 W; block 0 first completes the scalar step.
+template <typename T>
+__global__ void __launch_bounds__(kLsqrThreads) k_lsqr_xw(const T *__restrict__ V, T *__restrict__ W, T *__restrict__ X,
+                                             int64_t n, LsqrShared L) {
+    if (*L.skip_xw) return;
+    const T t1 = (T)L.st->t1, t2 = (T)L.st->t2, ia = (T)L.st->inv_alpha;
+    const int64_t stride = (int64_t)(gridDim.x - 1) * blockDim.x;
+    if (blockIdx.x == 0) {  // this block's own work
+        if (threadIdx.x < 32 && L.st->estimate) lsqr_estimate<T>(L);
+        return;
+    }
+    for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const T w = W[i];
+        X[i] = fma(t1, w, X[i]);
+        W[i] = fma(ia, V[i], t2 * w);
+    }
 }
 
 }  // namespace
@@ -311,7 +450,7 @@ struct sg_lsqr {
     void *U = nullptr, *V = nullptr, *W = nullptr, *X = nullptr, *F = nullptr, *G = nullptr;
     LsqrState *st = nullptr;  // device
     double *part = nullptr;   // 2 * kLsqrMaxBlocks partial sums
-    int *skip = nullptr;      // device flag: skip the x/w pass of this iteration
+    int *skip = nullptr;      // device flag: skip the x/w pass of this iteration; [1]: finished blocks
     cudaGraphConditionalHandle cond = 0;
     int has_cond = 0;
     cudaStream_t body = nullptr;
@@ -322,32 +461,21 @@ struct sg_lsqr {
 
 namespace {
 
-int lsqr_launch_axpby(sg_lsqr *h, const void *Xin, void *Y, int64_t len, int which,
-                      const void *Wn, cudaStream_t s) {
-    const double *coef = which == 0 ? &h->st->cu_a : &h->st->cv_a;
-    const int *done = &h->st->done;
-    const int nb = n_blocks(len);
-    if (h->dtype == SG_F64)
-        k_lsqr_axpby<double><<<nb, kLsqrThreads, 0, s>>>(
-            (const double *)Xin, (double *)Y, len, coef, done, h->part, (const double *)Wn,
-            h->part + kLsqrMaxBlocks);
-    else
-        k_lsqr_axpby<float><<<nb, kLsqrThreads, 0, s>>>(
-            (const float *)Xin, (float *)Y, len, coef, done, h->part, (const float *)Wn,
-            h->part + kLsqrMaxBlocks);
-    return cuda_check(cudaGetLastError(), "k_lsqr_axpby launch");
+LsqrShared lsqr_shared(const sg_lsqr *h) {
+    return LsqrShared{h->st, h->part, h->part + kLsqrMaxBlocks, (unsigned *)(h->skip + 1), h->skip, h->cond,
+                      h->has_cond};
 }
 
-int lsqr_launch_scalar(sg_lsqr *h, int nb, int nb2, int phase, cudaStream_t s) {
+int lsqr_launch_axpby(sg_lsqr *h, const void *Xin, void *Y, int64_t len, int phase, const void *Wn,
+                      cudaStream_t s) {
+    const int nb = n_blocks(len);
     if (h->dtype == SG_F64)
-        k_lsqr_scalar<double><<<1, kLsqrThreads, 0, s>>>(h->st, h->part, h->part + kLsqrMaxBlocks,
-                                                        nb, nb2, phase, h->skip, h->cond,
-                                                        h->has_cond);
+        k_lsqr_axpby<double><<<nb, kLsqrThreads, 0, s>>>((const double *)Xin, (double *)Y, len, (const double *)Wn,
+                                                        phase, lsqr_shared(h));
     else
-        k_lsqr_scalar<float><<<1, kLsqrThreads, 0, s>>>(h->st, h->part, h->part + kLsqrMaxBlocks,
-                                                       nb, nb2, phase, h->skip, h->cond,
-                                                       h->has_cond);
-    return cuda_check(cudaGetLastError(), "k_lsqr_scalar launch");
+        k_lsqr_axpby<float><<<nb, kLsqrThreads, 0, s>>>((const float *)Xin, (float *)Y, len, (const float *)Wn,
+                                                       phase, lsqr_shared(h));
+    return cuda_check(cudaGetLastError(), "k_lsqr_axpby launch");
 }
 
 bool vec_ok(const void *p) { return p && ((uintptr_t)p % 8) == 0; }
@@ -374,7 +502,8 @@ extern "C" int sg_lsqr_create(int32_t dtype, int64_t m, int64_t n, void *U, void
     h->U = U; h->V = V; h->W = W; h->X = X; h->F = F; h->G = G;
     int rc = dev_alloc((void **)&h->st, sizeof(LsqrState), "lsqr: state");
     if (!rc) rc = dev_alloc((void **)&h->part, 2 * kLsqrMaxBlocks * sizeof(double), "lsqr: partials");
-    if (!rc) rc = dev_alloc((void **)&h->skip, sizeof(int), "lsqr: flag");
+    if (!rc) rc = dev_alloc((void **)&h->skip, 2 * sizeof(int), "lsqr: flag");
+    if (!rc) rc = cuda_check(cudaMemset(h->skip, 0, 2 * sizeof(int)), "lsqr: flag");
     if (!rc) {
         LsqrState S = {};
         S.damp = damp;
@@ -411,39 +540,31 @@ extern "C" int sg_lsqr_start(sg_lsqr *h, const void *b, sg_stream_t stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const int nb = n_blocks(h->m > h->n ? h->m : h->n);
     if (h->dtype == SG_F64)
-        k_lsqr_start<double><<<nb, kLsqrThreads, 0, s>>>((const double *)b, (double *)h->U, h->m,
-                                                        (double *)h->X, (double *)h->W, h->n,
-                                                        h->part);
+        k_lsqr_start<double><<<nb, kLsqrThreads, 0, s>>>((const double *)b, (double *)h->U, h->m, (double *)h->X,
+                                                        (double *)h->W, h->n, lsqr_shared(h));
     else
-        k_lsqr_start<float><<<nb, kLsqrThreads, 0, s>>>((const float *)b, (float *)h->U, h->m,
-                                                       (float *)h->X, (float *)h->W, h->n,
-                                                       h->part);
-    int rc = cuda_check(cudaGetLastError(), "k_lsqr_start launch");
-    if (rc) return rc;
-    return lsqr_launch_scalar(h, nb, 0, kPhaseStart, s);
+        k_lsqr_start<float><<<nb, kLsqrThreads, 0, s>>>((const float *)b, (float *)h->U, h->m, (float *)h->X,
+                                                       (float *)h->W, h->n, lsqr_shared(h));
+    return cuda_check(cudaGetLastError(), "k_lsqr_start launch");
 }
 
 extern "C" int sg_lsqr_after_forward(sg_lsqr *h, sg_stream_t stream) {
     if (!h) return set_error(SG_ERR_INVALID_ARGUMENT, "sg_lsqr_after_forward: NULL handle");
-    cudaStream_t s = (cudaStream_t)stream;
-    int rc = lsqr_launch_axpby(h, h->F, h->U, h->m, 0, nullptr, s);
-    if (!rc) rc = lsqr_launch_scalar(h, n_blocks(h->m), 0, kPhaseU, s);
-    return rc;
+    return lsqr_launch_axpby(h, h->F, h->U, h->m, kPhaseU, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int sg_lsqr_after_adjoint(sg_lsqr *h, sg_stream_t stream) {
     if (!h) return set_error(SG_ERR_INVALID_ARGUMENT, "sg_lsqr_after_adjoint: NULL handle");
     cudaStream_t s = (cudaStream_t)stream;
-    int rc = lsqr_launch_axpby(h, h->G, h->V, h->n, 1, h->W, s);
-    if (!rc) rc = lsqr_launch_scalar(h, n_blocks(h->n), n_blocks(h->n), kPhaseV, s);
+    int rc = lsqr_launch_axpby(h, h->G, h->V, h->n, kPhaseV, h->W, s);
     if (rc) return rc;
-    const int nb = n_blocks(h->n);
+    const int nb = n_blocks(h->n) + 1;
     if (h->dtype == SG_F64)
         k_lsqr_xw<double><<<nb, kLsqrThreads, 0, s>>>((const double *)h->V, (double *)h->W,
-                                                     (double *)h->X, h->n, h->st, h->skip);
+                                                     (double *)h->X, h->n, lsqr_shared(h));
     else
         k_lsqr_xw<float><<<nb, kLsqrThreads, 0, s>>>((const float *)h->V, (float *)h->W,
-                                                    (float *)h->X, h->n, h->st, h->skip);
+                                                    (float *)h->X, h->n, lsqr_shared(h));
     return cuda_check(cudaGetLastError(), "k_lsqr_xw launch");
 }
 

@@ -23,10 +23,11 @@ import weakref
 import torch
 
 from . import _lib, arrays
-from .control_points import (LocallyRefinedControlPoints,
+from .control_points import (DefaultControlPoints, LocallyRefinedControlPoints,
                              evaluate_adjoint_control_points_, evaluate_control_points_,
                              get_n_control_points, obtain)
-from .spline_grid import (SplineGrid, evaluate_, evaluate_adjoint_, validate_partial_derivatives)
+from .spline_grid import (SplineGrid, _Plan, evaluate_, evaluate_adjoint_,
+                          validate_partial_derivatives)
 
 
 def _copy_levels(control_points, x: torch.Tensor, out: bool) -> None:
@@ -189,27 +190,64 @@ class LSQRSolver:
                                       btol, conlim, maxiter, C.byref(h)))
         self.handle = h
         self._fin = weakref.finalize(self, lib.sg_lsqr_destroy, h)
+        # plain control points: the operator reads V and writes G themselves instead of
+        # copying them through the grid's control points on every application; these hold
+        # the last A' u after a solve, as when every application goes through them
+        cps = A.grid.control_points
+        self._direct = (isinstance(cps, DefaultControlPoints) and obtain(cps).dtype == A.dtype)
+        self._adj_plan = None
         # create every plan and device table the operator uses before any capture
         A.mul_(self.F, self.V)
         A.rmul_(self.G, self.U)
+        if self._direct:
+            plan = A.grid.plan(A.dtype)
+            if graph and A.grid.nin == 2 and plan.paths() == ("fused", "separable"):
+                # a captured adjoint takes the fused path, because a graph may be replayed
+                # on any stream while the plan's intermediate is in use; the solver's graph
+                # has this plan, and its intermediate, for itself
+                self._adj_plan = _Plan(A.grid, arrays.dtype_code(A.dtype))
+                self._adj_plan.set_strategy("separable")
+            self._V, self._G = (arrays.reshape(v, tuple(cps.shape)) for v in (self.V, self.G))
+            self._F, self._U = (arrays.reshape(v, tuple(A.grid.eval.shape)) for v in (self.F, self.U))
         self.graph = False
         if graph:
             self._capture()
             self.graph = True
 
     # --------------------------------------------------------------- steps
+    def _forward(self) -> None:
+        if self._direct:
+            evaluate_(self.A.grid, self.A.derivative_order, control_points=self._V, eval=self._F)
+        else:
+            self.A.mul_(self.F, self.V)
+
+    def _adjoint(self) -> None:
+        if not self._direct:
+            self.A.rmul_(self.G, self.U)
+        elif self._adj_plan is not None:
+            _lib.check(_lib.load().sg_evaluate_adjoint(
+                self._adj_plan.handle, _lib.i32_array(self.A.derivative_order), self.U.data_ptr(),
+                self.G.data_ptr(), _lib.stream_handle()))
+        else:
+            evaluate_adjoint_(self.A.grid, self.A.derivative_order, control_points=self._G,
+                              eval=self._U)
+
     def _prologue(self, s: int) -> None:
         lib = _lib.load()
         _lib.check(lib.sg_lsqr_start(self.handle, self.B.data_ptr(), s))
-        self.A.rmul_(self.G, self.U)
+        self._adjoint()
         _lib.check(lib.sg_lsqr_after_adjoint(self.handle, s))
 
     def _iteration(self, s: int) -> None:
         lib = _lib.load()
-        self.A.mul_(self.F, self.V)
+        self._forward()
         _lib.check(lib.sg_lsqr_after_forward(self.handle, s))
-        self.A.rmul_(self.G, self.U)
+        self._adjoint()
         _lib.check(lib.sg_lsqr_after_adjoint(self.handle, s))
+
+    def _epilogue(self) -> None:
+        if self._direct:
+            arrays.vec(obtain(self.A.grid.control_points)).copy_(self.G)
 
     def _capture(self) -> None:
         lib = _lib.load()
@@ -226,6 +264,7 @@ class LSQRSolver:
                 bs = torch.cuda.ExternalStream(body.value, device=self.A.device)
                 with torch.cuda.stream(bs):
                     self._iteration(_lib.stream_handle())
+                self._epilogue()
             finally:
                 _lib.check(lib.sg_lsqr_capture_end(self.handle, s))
         torch.cuda.current_stream(self.A.device).wait_stream(cs)
@@ -256,6 +295,7 @@ class LSQRSolver:
             self._prologue(s)
             while not self.info()["done"]:
                 self._iteration(s)
+            self._epilogue()
         out = x if x is not None else torch.empty_like(self.X)
         out.copy_(self.X)
         return out

@@ -93,22 +93,22 @@ struct sg_grid_plan {
     // Nin = 2: the fused single-launch path (sg_fused2d.cuh) when the grid fits it
     int32_t strategy = SG_STRATEGY_AUTO;
     bool f2_fwd_ok = false, f2_adj_ok = false;
-    // AUTO: the separable adjoint all the same (large, chunked axis 0).  Its intermediate is
-    // a buffer of its own, in use by one stream at a time: a call on another stream while
-    // the last user's work is in flight, and a call under capture, take the fused path,
-    // which needs none.
+    // AUTO: the separable adjoint all the same (large, chunked axis 0).  The scratch of such a
+    // plan is in use by one stream at a time (ScratchLease): an AUTO call on another stream
+    // while the last user's work is in flight, and one under capture, take the fused
+    // path, which needs none.
     bool f2_adj_skip = false;
-    void *auto_scratch = nullptr;
-    cudaEvent_t auto_done = nullptr;          // after the last use
-    unsigned long long auto_stream = 0;       // its stream's id
-    bool auto_used = false;
-    std::mutex auto_mutex;
+    cudaEvent_t scratch_done = nullptr;       // after the scratch's last use
+    unsigned long long scratch_stream = 0;    // its stream's id
+    bool scratch_used = false;
+    std::mutex scratch_mutex;
     sg::F2Tiling f2_fwd, f2_adj;
     int64_t f2_adj_target = 0;      // cotangent values per adjoint tile (0: the wave model)
     std::vector<int32_t> lb0_host;  // axis-0 support table (host copy, for re-tiling)
     std::vector<int32_t> lb1_host;  // axis-1 support table (host copy, forward tiles)
     bool sorted_all = true, sorted1 = true;
     int32_t f2_fwd_kind = 0;        // fused forward: 0 warp tasks, 2 tiles (sorted axis 1)
+    int32_t f2_fwd_stage = 0;       // tiles: F2Grid::stage
     // optional per-pass timing: events[2*i], events[2*i+1] bracket pass i
     bool timing = false;
     cudaEvent_t events[2 * SG_MAX_NIN] = {};
@@ -194,6 +194,7 @@ static void plan_fused_tilings(sg_grid_plan *p) {
                                d.nout, f2_tile_cols(dt), 0, f2_slots(dt, 2), p->f2_fwd)) {
         p->f2_fwd_ok = true;
         p->f2_fwd_kind = 2;
+        p->f2_fwd_stage = !p->perm[0] && p->f2_fwd.count() > f2_slots(dt, 2);
     } else {
         p->f2_fwd_ok = f2_forward_tiling(d.n_samples[0], d.n_samples[1], d.nout, 0, f2_slots(dt, 0),
                                          p->f2_fwd);
@@ -209,8 +210,14 @@ static void plan_fused_tilings(sg_grid_plan *p) {
     // two passes are faster: their axis-1 units have a halo along one axis only, and the
     // intermediate (n1 / ns1 of the cotangent) stays in L2.  (4096, 4096) x 3: Float32 52 us
     // against 66, Float64 460 against 527; (2048, 2048): 12 against 23.
-    p->f2_adj_skip = d.n_samples[0] >= 2 * np &&
+    p->f2_adj_skip = p->f2_adj_ok && d.n_samples[0] >= 2 * np &&
                      d.n_samples[0] * d.n_samples[1] * d.nout >= kSeparableAdjValues;
+    if (p->f2_adj_skip && !p->scratch_done &&
+        cudaEventCreateWithFlags(&p->scratch_done, cudaEventDisableTiming) != cudaSuccess) {
+        (void)cudaGetLastError();
+        p->scratch_done = nullptr;
+        p->f2_adj_skip = false;
+    }
 }
 
 static int plan_scan_indices(sg_grid_plan *p, cudaStream_t s) {
@@ -332,10 +339,6 @@ extern "C" int sg_grid_plan_create(const sg_grid_desc *desc, sg_stream_t stream,
         for (int b = 0; b < nbuf && !rc; ++b)
             rc = dev_alloc(&p->scratch[b], (size_t)p->scratch_elems * es, "plan: scratch allocation");
     }
-    if (!rc && p->f2_adj_skip) {
-        rc = dev_alloc(&p->auto_scratch, (size_t)p->scratch_elems * elem_size(p->desc.dtype), "plan: adjoint intermediate");
-        if (!rc) rc = cuda_check(cudaEventCreateWithFlags(&p->auto_done, cudaEventDisableTiming), "plan: event");
-    }
     if (!rc) rc = dev_alloc((void **)&p->status, sizeof(int), "plan: status");
     if (!rc) rc = cuda_check(cudaMemsetAsync(p->status, 0, sizeof(int), s), "plan: status");
     if (rc) {
@@ -397,8 +400,7 @@ extern "C" void sg_grid_plan_destroy(sg_grid_plan *p) {
         if (p->events[i]) cudaEventDestroy(p->events[i]);
     for (int b = 0; b < 2; ++b)
         dev_free(p->scratch[b]);
-    dev_free(p->auto_scratch);
-    if (p->auto_done) cudaEventDestroy(p->auto_done);
+    if (p->scratch_done) cudaEventDestroy(p->scratch_done);
     for (int k = 0; k < SG_MAX_NIN; ++k) {
         dev_free(p->perm[k]);
         dev_free(p->lb[k]);
@@ -410,7 +412,7 @@ extern "C" void sg_grid_plan_destroy(sg_grid_plan *p) {
 extern "C" int64_t sg_grid_plan_workspace_bytes(const sg_grid_plan *p) {
     if (!p) return 0;
     const int nbuf = p->desc.nin >= 3 ? 2 : (p->desc.nin == 2 ? 1 : 0);
-    return (nbuf + (p->auto_scratch ? 1 : 0)) * p->scratch_elems * (p->desc.dtype == SG_F64 ? 8 : 4);
+    return nbuf * p->scratch_elems * (p->desc.dtype == SG_F64 ? 8 : 4);
 }
 
 // derivative_order checks of src/validation.jl:52-88 with the reference's messages.
@@ -478,6 +480,7 @@ static F2Grid f2_grid(const sg_grid_plan *p, const int32_t *ord, const void *X, 
     g.d0 = d.degree[0];
     g.d1 = d.degree[1];
     g.nch = d.nout;
+    g.stage = p->f2_fwd_stage;
     return g;
 }
 
@@ -486,8 +489,57 @@ static bool use_fused(const sg_grid_plan *p, bool ok) {
 }
 static bool use_fused_adjoint(const sg_grid_plan *p) {
     return use_fused(p, p->f2_adj_ok) &&
-           (p->strategy == SG_STRATEGY_FUSED || !p->f2_adj_skip || !p->auto_scratch);
+           (p->strategy == SG_STRATEGY_FUSED || !p->f2_adj_skip);
 }
+
+// The scratch of a plan with f2_adj_skip for the calls issued while the lease lives (other
+// plans have no such rule: the lease is theirs at once).  may_fail: ok stays false when
+// another stream's work still uses it, or when the stream is capturing (a graph can be replayed
+// at any time); otherwise the stream waits for that work.
+struct ScratchLease {
+    sg_grid_plan *p;
+    cudaStream_t s;
+    std::unique_lock<std::mutex> lock;
+    unsigned long long id = 0;
+    bool ok = false, record = false;
+    int rc = SG_OK;
+    ScratchLease(sg_grid_plan *p_, cudaStream_t s_, bool may_fail) : p(p_), s(s_) {
+        if (!p->scratch_done) {
+            ok = true;
+            return;
+        }
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        rc = cuda_check(cudaStreamIsCapturing(s, &cap), "plan: capture status");
+        if (rc) return;
+        if (cap != cudaStreamCaptureStatusNone) {
+            ok = !may_fail;
+            return;
+        }
+        rc = cuda_check(cudaStreamGetId(s, &id), "plan: stream id");
+        if (rc) return;
+        lock = std::unique_lock<std::mutex>(p->scratch_mutex);
+        if (p->scratch_used && id != p->scratch_stream) {
+            if (may_fail) {
+                const cudaError_t e = cudaEventQuery(p->scratch_done);
+                if (e == cudaErrorNotReady) {
+                    (void)cudaGetLastError();  // not an error
+                    return;
+                }
+                rc = cuda_check(e, "plan: scratch");
+            } else {
+                rc = cuda_check(cudaStreamWaitEvent(s, p->scratch_done, 0), "plan: scratch");
+            }
+            if (rc) return;
+        }
+        ok = record = true;
+    }
+    int end() {  // after the last launch that uses the scratch
+        if (!record) return SG_OK;
+        p->scratch_used = true;
+        p->scratch_stream = id;
+        return cuda_check(cudaEventRecord(p->scratch_done, s), "plan: scratch");
+    }
+};
 
 // Forward pass k (contract axis k) of one derivative order: X -> Y.  Only order[k] is
 // read; the last pass writes eval (NURBS: and divides).
@@ -563,14 +615,16 @@ extern "C" int sg_evaluate(sg_grid_plan *p, const int32_t *derivative_order,
         timer.end();
         return rc;
     }
+    ScratchLease lease(p, s, false);
+    if (lease.rc) return lease.rc;
     const void *X = control_points;
-    for (int k = 0; k < d.nin; ++k) {
+    for (int k = 0; k < d.nin && !rc; ++k) {
         void *Y = (k == d.nin - 1) ? eval : p->scratch[k % 2];
         rc = forward_pass(p, k, derivative_order, X, Y, weights, s, timer);
-        if (rc) return rc;
         X = Y;
     }
-    return SG_OK;
+    const int rc2 = lease.end();
+    return rc ? rc : rc2;
 }
 
 // Depth-first walk of the prefix tree of the requested orders: the intermediate after
@@ -637,8 +691,11 @@ extern "C" int sg_evaluate_multi(sg_grid_plan *p, int32_t n_orders, const int32_
                                             orders + (size_t)b * nin, orders + (size_t)b * nin + nin);
     });
     PassTimer timer(p, s);
-    return forward_tree(p, orders, ix.data(), 0, n_orders, 0, control_points, weights, evals, s,
-                        timer);
+    ScratchLease lease(p, s, false);
+    if (lease.rc) return lease.rc;
+    rc = forward_tree(p, orders, ix.data(), 0, n_orders, 0, control_points, weights, evals, s, timer);
+    const int rc2 = lease.end();
+    return rc ? rc : rc2;
 }
 
 // The passes of evaluate_adjoint!, last axis first, through scratch[0] and scratch[1].
@@ -695,45 +752,20 @@ extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_or
     if (!eval_bar) return set_error(SG_ERR_INVALID_ARGUMENT, "eval_bar is NULL");
 
     PassTimer timer(p, s);
-    bool fused = use_fused_adjoint(p);
-    if (!fused && use_fused(p, p->f2_adj_ok)) {  // AUTO, separable: when its buffer is free
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        unsigned long long id = 0;
-        rc = cuda_check(cudaStreamIsCapturing(s, &cap), "adjoint: capture status");
-        if (!rc && cap == cudaStreamCaptureStatusNone) {
-            rc = cuda_check(cudaStreamGetId(s, &id), "adjoint: stream id");
-            std::lock_guard<std::mutex> lock(p->auto_mutex);
-            bool free_now = true;
-            if (!rc && p->auto_used && id != p->auto_stream) {
-                const cudaError_t e = cudaEventQuery(p->auto_done);
-                if (e == cudaErrorNotReady) {
-                    (void)cudaGetLastError();
-                    free_now = false;
-                } else {
-                    rc = cuda_check(e, "adjoint: intermediate");
-                }
-            }
-            if (!rc && free_now) {
-                void *const bufs[2] = {p->auto_scratch, nullptr};
-                rc = separable_adjoint(p, derivative_order, eval_bar, control_points_bar, bufs, s, timer);
-                const int rc2 = cuda_check(cudaEventRecord(p->auto_done, s), "adjoint: intermediate");
-                p->auto_used = true;
-                p->auto_stream = id;
-                return rc ? rc : rc2;
-            }
+    if (!use_fused_adjoint(p)) {
+        ScratchLease lease(p, s, use_fused(p, p->f2_adj_ok));  // AUTO can do without
+        if (lease.rc) return lease.rc;
+        if (lease.ok) {
+            rc = separable_adjoint(p, derivative_order, eval_bar, control_points_bar, p->scratch, s, timer);
+            const int rc2 = lease.end();
+            return rc ? rc : rc2;
         }
-        if (rc) return rc;
-        fused = true;
     }
-    if (fused) {  // Nin = 2: both axes in one launch
-        timer.begin();
-        rc = f2_launch_grid(d.dtype == SG_F64 ? SG_F64 : SG_F32,
-                            f2_grid(p, derivative_order, eval_bar, control_points_bar), p->f2_adj, 1,
-                            p->status, s);
-        timer.end();
-        return rc;
-    }
-    return separable_adjoint(p, derivative_order, eval_bar, control_points_bar, p->scratch, s, timer);
+    timer.begin();  // Nin = 2: both axes in one launch
+    rc = f2_launch_grid(d.dtype == SG_F64 ? SG_F64 : SG_F32,
+                        f2_grid(p, derivative_order, eval_bar, control_points_bar), p->f2_adj, 1, p->status, s);
+    timer.end();
+    return rc;
 }
 
 // Measured choice of the adjoint stream's chunk size per axis k >= 1: each candidate

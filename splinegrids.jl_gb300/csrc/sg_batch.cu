@@ -358,6 +358,8 @@ static int batch_scratch(sg_batch_plan *p, int g) {
     return rc;
 }
 
+static void batch_retile(sg_batch_plan *p);
+
 extern "C" int sg_batch_plan_create(int32_t n_grids, const sg_grid_desc *grids,
                                     const int32_t *derivative_orders, sg_stream_t stream,
                                     sg_batch_plan **out) {
@@ -521,6 +523,7 @@ extern "C" int sg_batch_plan_create(int32_t n_grids, const sg_grid_desc *grids,
         batch_free(p);
         return rc;
     }
+    batch_retile(p);
     *out = p;
     return SG_OK;
 }
@@ -658,16 +661,40 @@ static void build_passes(sg_batch_plan *p, const void *const *cps, void *const *
 extern "C" int sg_batch_run(sg_batch_plan *p, int32_t what, sg_stream_t stream);
 extern "C" int sg_batch_check(sg_batch_plan *p, sg_stream_t stream);
 
+// Cotangent values per fused adjoint tile when none are asked for: axis 1 whole (0: no
+// cotangent row is read twice) when that makes three tiles and more per two resident
+// CTAs.  Otherwise about three tiles per CTA, which read their neighbours' boundary rows
+// again; tiles below 2^15 values are mostly set-up.  (304 CTAs.  32 grids x 16 sets, 597
+// whole tiles: whole 308 us, cut 350.  24 grids x 16 sets of at most 512 samples, 186 whole
+// tiles: whole 132 us, cut 97.  8 grids x 4 sets, 43 tiles: 212 and 51.)
+static int64_t batch_adjoint_target(const sg_batch_plan *p) {
+    if (p->f2_adj_target > 0) return p->f2_adj_target;
+    const int np = (int)f2_pairs_per_tile(p->dtype);
+    int64_t total = 0, whole = 0;
+    for (int g = 0; g < p->n_grids; ++g) {
+        if (!p->f2_ok[g]) continue;
+        const sg_grid_desc &d = p->desc[g];
+        F2Tiling t;
+        if (f2_adjoint_tiling(p->lb0_host[g].data(), d.n_basis[0], d.degree[0], d.n_samples[0], d.n_basis[1],
+                              d.degree[1], d.n_samples[1], d.nout, np, f2_align_elems(p->dtype), 0, 0, t))
+            whole += t.count();
+        total += d.n_samples[0] * d.n_samples[1] * d.nout;
+    }
+    const int64_t slots = f2_slots(p->dtype, 1);
+    return 2 * whole >= 3 * slots ? 0 : std::max<int64_t>(1 << 15, total / (3 * slots));
+}
+
 // Tilings of the fused grids for the plan's unit sizes.
 static void batch_retile(sg_batch_plan *p) {
     const int np = (int)f2_pairs_per_tile(p->dtype);
+    const int64_t adj_target = batch_adjoint_target(p);
     for (int g = 0; g < p->n_grids; ++g) {
         if (!p->f2_ok[g]) continue;
         const sg_grid_desc &d = p->desc[g];
         f2_forward_tile_tiling(p->lb1_host[g].data(), d.n_basis[1], d.degree[1], d.n_samples[0], d.n_samples[1],
                                d.nout, f2_tile_cols(p->dtype), p->f2_fwd_target, 0, p->f2_fwd[g]);
         f2_adjoint_tiling(p->lb0_host[g].data(), d.n_basis[0], d.degree[0], d.n_samples[0], d.n_basis[1],
-                          d.degree[1], d.n_samples[1], d.nout, np, f2_align_elems(p->dtype), p->f2_adj_target, 0,
+                          d.degree[1], d.n_samples[1], d.nout, np, f2_align_elems(p->dtype), adj_target, 0,
                           p->f2_adj[g]);
     }
 }
@@ -680,6 +707,9 @@ static void build_fused(sg_batch_plan *p, const void *const *cps, void *const *e
     const size_t es = p->dtype == SG_F64 ? 8 : 4;
     descs.assign(2 * (size_t)p->n_grids, F2Grid());
     std::vector<std::pair<int64_t, F2Tile>> lists[2];
+    int64_t n_fwd = 0;
+    for (int g = 0; g < p->n_grids; ++g) n_fwd += grid_fused(p, g) ? p->f2_fwd[g].count() : 0;
+    const bool stage = n_fwd > f2_slots(p->dtype, 2);  // see F2Grid::stage
     for (int g = 0; g < p->n_grids; ++g) {
         if (!grid_fused(p, g)) continue;
         const sg_grid_desc &d = p->desc[g];
@@ -707,6 +737,7 @@ static void build_fused(sg_batch_plan *p, const void *const *cps, void *const *e
                 F2Tile t = p->f2_fwd[g].tile(i, 2, d.nout, d.n_samples[0], d.n_samples[1]);
                 t.grid = 2 * g;
                 f2_tile_columns(p->lb1_host[g].data(), d.n_basis[1], d.degree[1], t.b_lo, t.b_len, t.cb, t.ncol);
+                if (stage) f2_tile_columns(p->lb0_host[g].data(), d.n_basis[0], d.degree[0], t.a_lo, t.a_len, t.pa, t.na);
                 lists[0].push_back({(int64_t)t.a_len * t.G * t.b_len, t});
             }
         }

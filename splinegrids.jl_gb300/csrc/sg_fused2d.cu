@@ -28,33 +28,23 @@ k_f2_fwd_grid(F2Grid g, F2Tiling tiling) {
 
 // One grid, forward over sorted axis-1 samples: blockIdx.x is the tile.
 template <typename T, typename TX>
-__global__ void __launch_bounds__(kF2TileWarps * 32)
+__global__ void __launch_bounds__(kF2TileWarps * 32, sizeof(T) == 4 ? 5 : 4)
 k_f2_fwdt_grid(F2Grid g, F2Tiling tiling) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ F2Grid s_g;
-    __shared__ F2Tile s_t;
-    if (threadIdx.x == 0) {
-        s_g = g;
-        s_t = tiling.tile((int64_t)blockIdx.x, 2, g.nch, g.ns0, g.ns1);
-    }
-    __syncthreads();
-    f2_run_forward_tile<T, TX>(s_g, s_t, smem);
+    const F2Tile t = tiling.tile((int64_t)blockIdx.x, 2, g.nch, g.ns0, g.ns1);
+    f2_run_forward_tile<T, TX>(g, t, smem);
 }
 
-// Batch forward tiles: block x runs tile x of the list.
+// Batch forward tiles: block x runs tile x of the list.  Every thread reads the tile and the
+// grid's descriptor itself (the same addresses for all: one request a warp), which costs
+// two loads in a row and no barrier.
 template <typename T>
-__global__ void __launch_bounds__(kF2TileWarps * 32)
+__global__ void __launch_bounds__(kF2TileWarps * 32, sizeof(T) == 4 ? 5 : 4)
 k_f2_fwdt_batch(const F2Grid *__restrict__ grids, const F2Tile *__restrict__ tiles) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ F2Grid s_g;
-    __shared__ F2Tile s_t;
-    static_assert(sizeof(F2Grid) % 4 == 0 && sizeof(F2Grid) / 4 <= kF2TileWarps * 32, "descriptor copy");
-    if (threadIdx.x == 0) s_t = tiles[blockIdx.x];
-    __syncthreads();
-    if (threadIdx.x < sizeof(F2Grid) / 4)
-        reinterpret_cast<int32_t *>(&s_g)[threadIdx.x] = reinterpret_cast<const int32_t *>(grids + s_t.grid)[threadIdx.x];
-    __syncthreads();
-    f2_run_forward_tile<T, T>(s_g, s_t, smem);
+    const F2Tile t = tiles[blockIdx.x];
+    const F2Grid g = grids[t.grid];
+    f2_run_forward_tile<T, T>(g, t, smem);
 }
 
 // One grid, adjoint: blockIdx.x is the tile.

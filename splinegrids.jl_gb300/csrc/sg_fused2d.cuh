@@ -97,7 +97,11 @@ struct F2Grid {
     const void *X;               // forward: control points [n0, n1, nch]; adjoint: eval_bar
     void *Y;                     // forward: eval [ns0, ns1, nch]; adjoint: gradient
     int64_t ns0, ns1, n0, n1;
-    int32_t d0, d1, nch, pad;
+    int32_t d0, d1, nch;
+    // forward tiles: stage the tile's control points (axis-0 samples sorted, and more tiles
+    // than fit the GPU at once, so that loads wait behind other tiles' stores; a single
+    // wave loses 0.4 us to the extra barrier)
+    int32_t stage;
 };
 
 // One unit.  Forward: samples [a_lo, a_lo+a_len) of axis 0 x rows [b_lo, b_lo+b_len)
@@ -109,6 +113,7 @@ struct F2Tile {
     int32_t a_lo, a_len;
     int32_t b_lo, b_len;
     int32_t cb, ncol;    // forward tile: first axis-1 column and column count (0: from the samples)
+    int32_t pa, na;      // forward tile: first axis-0 control point of its samples' supports, count (0: from the samples)
 };
 
 // Uniform blocking of one grid in one direction.  Adjoint unit i is (group, a block,
@@ -123,7 +128,7 @@ struct F2Tiling {
     __host__ __device__ int64_t count() const { return (int64_t)ngrp * nba * nbb; }
     __host__ __device__ F2Tile tile(int64_t i, int kind, int nch, int64_t na, int64_t nb) const {
         F2Tile t;
-        t.cb = t.ncol = 0;
+        t.cb = t.ncol = t.pa = t.na = 0;
         int64_t ia, ib;
         if (kind != 1) {  // forward (warp tasks: 0, tiles: 2)
             ia = i % nba;
@@ -704,11 +709,13 @@ constexpr int kF2TileWarps = 8;    // warps (phase-2 row strides) per forward ti
 constexpr int kF2TileRows = 512;   // rows of axis 1 per forward tile at most
 template <typename T>
 __host__ __device__ constexpr int kF2TileCols() { return sizeof(T) == 4 ? 64 : 32; }
+constexpr int kF2TileBlock = 512;  // control points of a tile that are staged (values)
 template <typename T>
 __host__ __device__ constexpr int64_t f2_tile_smem() {
     return (int64_t)kF2TileCols<T>() * kF2TileS0 * sizeof(T)  // Y tile
            + (int64_t)kF2TileRows * 4 * sizeof(T)             // the rows' axis-1 basis values
-           + (int64_t)kF2TileRows * 4;                        // the rows' Y offsets
+           + (int64_t)kF2TileRows * 4                         // the rows' Y offsets
+           + (int64_t)kF2TileBlock * sizeof(T);               // the tile's control points
 }
 
 // Phase 1 of a forward tile for axis-0 degree D0 - 1: the Y tile's columns [cb, ce) of
@@ -767,7 +774,40 @@ __device__ __forceinline__ void f2_forward_tile(const F2Grid &g, const F2Tile &t
     const int ce = tl.ncol > 0 ? tl.cb + tl.ncol
                                : (int)support_start(g.idx1[tl.b_lo + tl.b_len - 1], D1 - 1, n1) + D1;
     if (ce - cb > kF2TileCols<T>() || ce <= cb || tl.b_len > kF2TileRows) return;  // (ruled out by the host)
-    {  // phase 1: the rows' headers, then the Y tile
+    // Phase 1.  The launch writes eval as fast as memory takes it, so a load waits behind the
+    // stores of the SM's other tiles, and what a tile costs is the number of loads that
+    // wait for one another: its control points (the block of its samples' supports and
+    // its columns, a few hundred values when axis 0 is sorted), its axis-0 basis rows and the
+    // rows' headers are all fetched at once, and Y is formed from the staged block.  Larger
+    // blocks and unsorted samples read the control points per sample instead.  Measured, per
+    // sample against staged: (4096, 4096) x 3 35.7 and 32.1 us; 32 grids x 16 sets 292 and 280.
+    const int pa = tl.na > 0 ? tl.pa : (g.stage ? (int)support_start(g.idx0[tl.a_lo], g.d0, (int)g.n0) : 0);
+    const int na = tl.na > 0 ? tl.na
+                 : g.stage ? (int)support_start(g.idx0[tl.a_lo + tl.a_len - 1], g.d0, (int)g.n0) + g.d0 + 1 - pa : 0;
+    const bool staged = na > 0 && na * (ce - cb) <= kF2TileBlock;
+    T *Ps = reinterpret_cast<T *>(hY + kF2TileRows);  // [columns][na]
+    {
+        const int n0 = (int)g.n0, d0 = g.d0;
+        const int sl = tid & (S - 1);
+        const int s0 = tl.a_lo + (sl < tl.a_len ? sl : 0);
+        const int pos = CT ? sl : (sl & 31) * 4 + (sl >> 5);
+        T bw[4];
+        int b0 = 0;
+        if (staged) {
+            const TX *__restrict__ P = (const TX *)g.X + ((uint32_t)pa + (uint32_t)n0 * ((uint32_t)n1 * (uint32_t)c + (uint32_t)cb));
+            const int total = na * (ce - cb);
+            for (int e = tid; e < total; e += NT) {
+                const int col = e / na;
+                const TX *src = P + (uint32_t)n0 * (uint32_t)col + (uint32_t)(e - col * na);
+                if constexpr (std::is_same<T, TX>::value) cp_async<(int)sizeof(T)>(Ps + e, src);
+                else Ps[e] = (T)to_f(*src);
+            }
+            cp_async_commit();
+            const T *__restrict__ B0 = (const T *)g.B0;
+            b0 = (int)support_start(g.idx0[s0], d0, n0) - pa;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) bw[i] = i <= d0 ? B0[s0 + ns0 * i] : T(0);
+        }
         const T *__restrict__ B1 = (const T *)g.B1;
         for (int j = tid; j < tl.b_len; j += NT) {
             const int r = tl.b_lo + j;
@@ -775,16 +815,35 @@ __device__ __forceinline__ void f2_forward_tile(const F2Grid &g, const F2Tile &t
 #pragma unroll
             for (int k = 0; k < 4; ++k) hB1[j * 4 + k] = k < D1 ? B1[r + ns1 * k] : T(0);
         }
-        const int sl = tid & (S - 1);
-        if (sl < tl.a_len) {
-            const int pos = CT ? sl : (sl & 31) * 4 + (sl >> 5);
-            const int col0 = cb + tid / S;
-            constexpr int CS = NT / S;
-            switch (g.d0) {
-                case 0: f2_tile_phase1<T, TX, 1>(g, tl, Ys, sl, pos, cb, ce, col0, CS); break;
-                case 1: f2_tile_phase1<T, TX, 2>(g, tl, Ys, sl, pos, cb, ce, col0, CS); break;
-                case 2: f2_tile_phase1<T, TX, 3>(g, tl, Ys, sl, pos, cb, ce, col0, CS); break;
-                default: f2_tile_phase1<T, TX, 4>(g, tl, Ys, sl, pos, cb, ce, col0, CS); break;
+        const int col0 = tid / S;
+        constexpr int CS = NT / S;
+        if (staged) {
+            cp_async_wait<0>();
+            __syncthreads();
+            const T *pc = Ps + col0 * na + b0;
+            T *yc = Ys + col0 * S + pos;
+            if (sl < tl.a_len) {
+#define SG_F2_P1(D0)                                                            \
+    for (int col = col0; col < ce - cb; col += CS, pc += CS * na, yc += CS * S) { \
+        T a = T(0);                                                             \
+        _Pragma("unroll") for (int i = 0; i < D0; ++i) a = ::fma(bw[i], pc[i], a); \
+        *yc = a;                                                                \
+    }                                                                           \
+    break;
+                switch (d0) {
+                    case 0: SG_F2_P1(1)
+                    case 1: SG_F2_P1(2)
+                    case 2: SG_F2_P1(3)
+                    default: SG_F2_P1(4)
+                }
+#undef SG_F2_P1
+            }
+        } else if (sl < tl.a_len) {
+            switch (d0) {
+                case 0: f2_tile_phase1<T, TX, 1>(g, tl, Ys, sl, pos, cb, ce, cb + col0, CS); break;
+                case 1: f2_tile_phase1<T, TX, 2>(g, tl, Ys, sl, pos, cb, ce, cb + col0, CS); break;
+                case 2: f2_tile_phase1<T, TX, 3>(g, tl, Ys, sl, pos, cb, ce, cb + col0, CS); break;
+                default: f2_tile_phase1<T, TX, 4>(g, tl, Ys, sl, pos, cb, ce, cb + col0, CS); break;
             }
         }
     }

@@ -20,7 +20,7 @@ bool f2_forward_tiling(int64_t ns0, int64_t ns1, int nch, int64_t target, int sl
 bool f2_forward_tile_tiling(const int32_t *lb1, int64_t n1, int d1, int64_t ns0, int64_t ns1, int nch,
                             int cols, int64_t target, int slots, F2Tiling &t);
 // First axis-1 column and column count of the forward tile over rows [b_lo, b_lo + b_len)
-// of a sorted axis (lb1: its support table).
+// of a sorted axis (lb1: its support table); the same for control points of axis 0.
 void f2_tile_columns(const int32_t *lb1, int64_t n1, int d1, int64_t b_lo, int64_t b_len, int32_t &cb,
                      int32_t &ncol);
 // Columns of a forward tile's intermediate for the value type.

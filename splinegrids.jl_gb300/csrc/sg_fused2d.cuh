@@ -46,6 +46,7 @@ constexpr int kF2NS = 3;           // adjoint: stages in the ring
 constexpr int kF2PhaseBPerStage = 1;  // adjoint: pending phase-B items a thread takes per stage
 constexpr int kF2BarBytes = ((2 * kF2NS * 8 + 15) / 16) * 16;  // full + empty mbarriers
 constexpr int kF2MaxG = 32;        // adjoint: channels per tile at most (one bulk copy each)
+constexpr int kF2Cps = 512;        // adjoint: axis-0 control points of a tile whose supports are staged
 
 // Adjoint tiles: (sample, channel) pairs per tile; four pairs per consumer thread for
 // Float32 (two register pairs), two for Float64.
@@ -74,6 +75,9 @@ struct F2Pair;
 template <>
 struct F2Pair<float> {
     using V = float2;
+    using B = float2;  // a basis value as the FMA takes it
+    static __device__ __forceinline__ B basis(float b) { return make_float2(b, b); }
+    static __device__ __forceinline__ V dup(B b) { return b; }
     static __device__ __forceinline__ V zero() { return make_float2(0.f, 0.f); }
     static __device__ __forceinline__ V make(float a, float b) { return make_float2(a, b); }
     static __device__ __forceinline__ V fma(V b, V x, V c) { return __ffma2_rn(b, x, c); }
@@ -81,6 +85,9 @@ struct F2Pair<float> {
 template <>
 struct F2Pair<double> {
     using V = double2;
+    using B = double;
+    static __device__ __forceinline__ B basis(double b) { return b; }
+    static __device__ __forceinline__ V dup(B b) { return make_double2(b, b); }
     static __device__ __forceinline__ V zero() { return make_double2(0.0, 0.0); }
     static __device__ __forceinline__ V make(double a, double b) { return make_double2(a, b); }
     static __device__ __forceinline__ V fma(V b, V x, V c) {
@@ -156,8 +163,8 @@ struct F2Tiling {
 
 // adjoint shared memory, in carving order
 template <typename T>
-__host__ __device__ constexpr int64_t f2_adj_hdr_bytes() {  // per stage: basis rows, starts, segment bases
-    return align16((int64_t)kF2Rows * 4 * 2 * sizeof(T)) + align16(kF2Rows * 4) + align16(kF2MaxG * 4);
+__host__ __device__ constexpr int64_t f2_adj_hdr_bytes() {  // per stage: basis rows (Float32: as pairs), starts
+    return (int64_t)kF2Rows * 4 * 8 + align16(kF2Rows * 4);
 }
 template <typename T>
 __host__ __device__ constexpr int64_t f2_adj_smem() {
@@ -166,7 +173,8 @@ __host__ __device__ constexpr int64_t f2_adj_smem() {
            + kF2NS * f2_adj_hdr_bytes<T>()                             // stage headers
            + kF2NS * align16((int64_t)f2_stage_elems<T>() * sizeof(T))  // cotangent ring
            + align16((int64_t)kF2Ring * f2_zstride<T>() * sizeof(T))   // Z ring
-           + (int64_t)f2_pairs<T>() * 4 * sizeof(T);                  // axis-0 weight list
+           + (int64_t)f2_pairs<T>() * 4 * sizeof(T)                   // axis-0 weight list
+           + (int64_t)(kF2Cps + 1) * 8;                               // its control points
 }
 
 // ---------------------------------------------------------------------------------
@@ -347,6 +355,7 @@ struct F2AdjSmem {
     T *ring;             // [kF2NS][f2_stage_elems]
     T *Zs;               // [kF2Ring][zstride]
     T *W0;               // [4 NP]: the axis-0 weights B0[s, c0 - b0(s)], c0-major, s increasing
+    int2 *C0;            // [kF2Cps + 1]: first sample (of the tile's) and weight of each control point
     __device__ explicit F2AdjSmem(unsigned char *smem) {
         full = reinterpret_cast<uint64_t *>(smem);
         empty = full + kF2NS;
@@ -356,16 +365,14 @@ struct F2AdjSmem {
         Zs = ring + kF2NS * (align16((int64_t)f2_stage_elems<T>() * sizeof(T)) / (int64_t)sizeof(T));
         W0 = reinterpret_cast<T *>(reinterpret_cast<unsigned char *>(Zs) +
                                    align16((int64_t)kF2Ring * f2_zstride<T>() * sizeof(T)));
+        C0 = reinterpret_cast<int2 *>(W0 + 4 * f2_pairs<T>());
     }
-    template <typename V>
-    __device__ V *hB(int slot) { return reinterpret_cast<V *>(hdr + slot * f2_adj_hdr_bytes<T>()); }
+    // a stage's header: row j's axis-1 basis values at hB + 4 j (Float32: each twice), starts hb
+    __device__ typename F2Pair<T>::B *hB(int slot) {
+        return reinterpret_cast<typename F2Pair<T>::B *>(hdr + slot * f2_adj_hdr_bytes<T>());
+    }
     __device__ int32_t *hb(int slot) {
-        return reinterpret_cast<int32_t *>(hdr + slot * f2_adj_hdr_bytes<T>() +
-                                           align16((int64_t)kF2Rows * 4 * 2 * sizeof(T)));
-    }
-    __device__ int32_t *hseg(int slot) {
-        return reinterpret_cast<int32_t *>(hdr + slot * f2_adj_hdr_bytes<T>() +
-                                           align16((int64_t)kF2Rows * 4 * 2 * sizeof(T)) + align16(kF2Rows * 4));
+        return reinterpret_cast<int32_t *>(hdr + slot * f2_adj_hdr_bytes<T>() + (int64_t)kF2Rows * 4 * 8);
     }
 };
 
@@ -399,6 +406,7 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
                                              uint32_t &gstage, int *status) {
     using PT = F2Pair<T>;
     using V = typename PT::V;
+    using BV = typename PT::B;
     constexpr int NC = 32 * kF2Consumers;
     constexpr int J = f2_j<T>();
     constexpr int JP = J / 2;
@@ -411,6 +419,7 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
     constexpr int64_t STAGE = align16((int64_t)f2_stage_elems<T>() * ES) / ES;
     constexpr int d1 = D1 - 1;
     static_assert(J % 2 == 0, "pairs per thread come in couples");
+    static_assert(SR == 4 && H == 4, "stages of four rows, halves of four columns");
     F2AdjSmem<T> sm(smem);
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
@@ -488,7 +497,6 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
                     mbar_expect_tx(&sm.full[slot], (unsigned)(re16 - ra0));
                     if (re16 > ra0) bulk_g2s(d, (const void *)ra0, (unsigned)(re16 - ra0), &sm.full[slot]);
                 }
-                if (lane == 0) sm.hseg(slot)[0] = (int)((a - a0) / ES);
             } else if (lane < G) {  // the copies first: they are the long pole; one per lane
                 const int c = lane;     // (channel c's rows are consecutive in memory)
                 const uintptr_t a = (uintptr_t)(X + (uint32_t)ns0 * ((uint32_t)r0 + (uint32_t)ns1 *
@@ -508,16 +516,11 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
                 const int j = lane - SR * (q % QB);
                 if (j >= 0 && j < nr) {
                     sm.hb(slot)[j] = h_b;
-                    Pack<T, 4> hv;  // the row's basis values, one 16-byte (Float64: 32-byte) entry
+                    Pack<BV, 4> hv;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) hv.v[i] = i < D1 ? h_v[i < D1 ? i : 0] : T(0);
-                    stp<T, 4>(sm.template hB<T>(slot) + j * 4, hv);
+                    for (int i = 0; i < 4; ++i) hv.v[i] = PT::basis(i < D1 ? h_v[i < D1 ? i : 0] : T(0));
+                    *reinterpret_cast<Pack<BV, 4> *>(sm.hB(slot) + j * 4) = hv;
                 }
-            }
-            if (!chunk && lane < G) {  // channel `lane`: its segment's base (element of sample 0)
-                const uintptr_t a = (uintptr_t)(X + (uint32_t)ns0 * ((uint32_t)r0 + (uint32_t)ns1 *
-                                                                     (uint32_t)(tl.c_lo + lane)));
-                sm.hseg(slot)[lane] = lane * seg + (int)((a & 15) / ES);
             }
             __syncwarp();
             // publishes the header with the data (a test hook can withhold the CTA's first
@@ -559,14 +562,21 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
             }
         }
     }
+    const bool c0_staged = K0 <= kF2Cps;
+    if (c0_staged)
+        for (int c = tid; c <= K0; c += NC) sm.C0[c] = make_int2(lb0[C0a + c] - s0lo, off0[C0a + c] - ob);
+    // Where the thread's pairs lie in a stage.  A stage's rows start 4 ns0 values after the
+    // previous stage's, a multiple of 16 bytes, so the lead of the aligned copies is the same
+    // in every stage of the tile.
     const int npairs = w0 * G;
-    int pofs[J];  // sample (relative to the tile's first) + channel segment of each pair
-    int pcl[J];
+    int xo[J];
 #pragma unroll
     for (int j = 0; j < J; ++j) {
         const int p = tid + NC * j;
-        pcl[j] = p < npairs ? p / w0 : 0;
-        pofs[j] = p < npairs ? p % w0 : 0;
+        const int cl = p < npairs ? p / w0 : 0, so = p < npairs ? p - cl * w0 : 0;
+        const uintptr_t a = (uintptr_t)(X + (uint32_t)ns0 * ((uint32_t)s1lo + (uint32_t)ns1 * (uint32_t)(tl.c_lo + cl)) +
+                                        (chunk ? s0lo : 0));
+        xo[j] = cl * seg + (int)((a & 15) / ES) + so;
     }
     // Phase B of a finished half (ring columns pb_col0 .. + pb_nc - 1) is pending from the
     // half's barrier until the next one: each consumer thread takes its items a few at
@@ -575,27 +585,38 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
     // the columns).  Work item: (column pair, c0, channel), the pair fastest; a pair's
     // two outputs share every weight load and run as one packed FMA chain (one output
     // when pb_nc is odd and the pair is the last).
-    int pb_col0 = 0, pb_nc = 0, pb_np2 = 1, pb_o = 0, pb_n = 0;
+    int pb_col0 = 0, pb_nc = 0, pb_sh = 0, pb_o = 0, pb_n = 0;
+    // r / K0 for r < K0 G: exact by a 32-bit reciprocal while K0 and K0 G are small
+    const uint32_t k0_inv = (uint32_t)((0x100000000ull + K0 - 1) / (uint32_t)K0);
     auto b_item = [&](int o) {
-        const int slot0 = (pb_col0 - C1a) % R;
-        const int hp = o % pb_np2;
-        const int r2 = o / pb_np2;
-        const int c0 = C0a + r2 % K0;
-        const int cl = r2 / K0;
-        const int sb = lb0[c0];
-        const int m = lb0[c0 + 1 + d0] - sb;
+        const int hp = o & pb_sh, r2 = o >> pb_sh;
+        const int cl = G == 1 ? 0 : (c0_staged ? (int)__umulhi((uint32_t)r2, k0_inv) : r2 / K0);
+        const int ci = r2 - cl * K0, c0 = C0a + ci;
+        int sb, wb, m;
+        if (c0_staged) {
+            const int2 e = sm.C0[ci], f = sm.C0[ci + 1];
+            sb = e.x;
+            wb = e.y;
+            m = f.y - e.y;
+        } else {
+            sb = lb0[c0] - s0lo;
+            wb = off0[c0] - ob;
+            m = off0[c0 + 1] - off0[c0];
+        }
         const int h = 2 * hp;
-        const T *zc = sm.Zs + (slot0 + h) * ZS + w0 * cl + (sb - s0lo);
-        const T *w = sm.W0 + (off0[c0] - ob);
+        const T *zc = sm.Zs + ((pb_col0 - C1a) % R + h) * ZS + w0 * cl + sb;
+        const T *w = sm.W0 + wb;
         T *yo = (T *)g.Y + ((uint32_t)c0 + (uint32_t)n0 * ((uint32_t)(pb_col0 + h) + (uint32_t)n1 *
                                                             (uint32_t)(tl.c_lo + cl)));
         if (h + 1 < pb_nc) {
             V a = PT::zero();
+#pragma unroll 4
             for (int k = 0; k < m; ++k) a = PT::fma(PT::make(w[k], w[k]), PT::make(zc[k], zc[k + ZS]), a);
             yo[0] = a.x;  // increasing s, from zero, for both columns
             yo[n0] = a.y;
         } else {
             T a = T(0);
+#pragma unroll 4
             for (int k = 0; k < m; ++k) a = ::fma(w[k], zc[k], a);
             yo[0] = a;
         }
@@ -613,8 +634,9 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
     // control point `cur` is complete: into the ring (when in the block), then phase B
     // once a half of the ring is full or the block ends
     auto flush = [&]() {
-        if (cur >= C1a) {
-            T *z = sm.Zs + ((cur - C1a) % R) * ZS + tid;
+        const int done = cur - C1a;
+        if (done >= 0) {
+            T *z = sm.Zs + (done % R) * ZS + tid;
 #pragma unroll
             for (int jp = 0; jp < JP; ++jp) {
                 z[NC * (2 * jp)] = acc[0][jp].x;
@@ -627,13 +649,13 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
             for (int jp = 0; jp < JP; ++jp) acc[k][jp] = acc[k + 1][jp];
 #pragma unroll
         for (int jp = 0; jp < JP; ++jp) acc[D1 - 1][jp] = PT::zero();
-        if (cur >= C1a && ((cur - C1a) % H == H - 1 || cur == cend - 1)) {
+        if (done >= 0 && (done % H == H - 1 || cur == cend - 1)) {
             b_some(1 << 30);  // the previous half: the rest of this thread's items
             f2_consumer_sync();
-            pb_col0 = cur - (cur - C1a) % H;
-            pb_nc = cur - pb_col0 + 1;
-            pb_np2 = (pb_nc + 1) >> 1;
-            pb_n = K0 * pb_np2 * G;
+            pb_nc = done % H + 1;
+            pb_col0 = cur - pb_nc + 1;
+            pb_sh = pb_nc > 2 ? 1 : 0;
+            pb_n = (K0 * G) << pb_sh;
             pb_o = tid;
         }
         ++cur;
@@ -653,27 +675,30 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
             }
             continue;
         }
-        const int r0 = s1lo + q * SR;
-        const int nr = (s1hi - r0) < SR ? (s1hi - r0) : SR;
+        const int left = s1hi - (s1lo + q * SR);
+        const int nr = left < SR ? left : SR;
         const T *base = sm.ring + (int64_t)slot * STAGE;
-        const int32_t *hseg = sm.hseg(slot);
+        const BV *hB = sm.hB(slot);
         const T *xp[J];
 #pragma unroll
-        for (int j = 0; j < J; ++j) xp[j] = base + hseg[pcl[j]] + pofs[j];
-        const T *hB = sm.template hB<T>(slot);
+        for (int j = 0; j < J; ++j) xp[j] = base + xo[j];
         const int32_t *hb = sm.hb(slot);
+        // Not unrolled: a batch runs tiles of all degrees side by side, each its own code, and
+        // larger loops miss the instruction cache (four rows at once: 368 us against 301, 32 grids
+        // x 16 sets; slots fitted to the tile's pairs, three times the code, 410).
+#pragma unroll 1
         for (int u = 0; u < nr; ++u) {
             const int b = hb[u];
             while (cur < b) flush();
-            V x[JP];
+            V xv[JP];
 #pragma unroll
-            for (int jp = 0; jp < JP; ++jp) x[jp] = PT::make(xp[2 * jp][u * rs], xp[2 * jp + 1][u * rs]);
-            const Pack<T, 4> hv = ldp<T, 4>(hB + u * 4);  // one load for the row's basis values
+            for (int jp = 0; jp < JP; ++jp) xv[jp] = PT::make(xp[2 * jp][u * rs], xp[2 * jp + 1][u * rs]);
+            const Pack<BV, 4> hv = *reinterpret_cast<const Pack<BV, 4> *>(hB + u * 4);
 #pragma unroll
             for (int k = 0; k < D1; ++k) {
-                const V bv = PT::make(hv.v[k], hv.v[k]);
+                const V bv = PT::dup(hv.v[k]);
 #pragma unroll
-                for (int jp = 0; jp < JP; ++jp) acc[k][jp] = PT::fma(bv, x[jp], acc[k][jp]);
+                for (int jp = 0; jp < JP; ++jp) acc[k][jp] = PT::fma(bv, xv[jp], acc[k][jp]);
             }
         }
         __syncwarp();

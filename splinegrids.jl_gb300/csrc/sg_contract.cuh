@@ -245,31 +245,38 @@ fwd_axis0_tile(const Tile &tl, const int32_t *__restrict__ idx, const T *__restr
             __stcs(Y + j + ns * (int64_t)o, (T)((double)num / (double)den));
         }
         return;
-    } else {
-        const int64_t Qy = (MODE == kHomog) ? Qr * (int64_t)(nch + 1) : Qr * (int64_t)nch;
-#pragma unroll 4
-        for (int64_t q = tl.by; q < Qy; q += tl.gy) {
-            T acc = T(0);
-            if constexpr (MODE == kPlain) {
-                const TX *xp = X + b + n * q;
+    } else if constexpr (MODE == kHomog) {
+        // column r of the weights (by, by + gy, ...) with channels bz, bz + gz, ... of it:
+        // channel 0 is the weight itself, channel o >= 1 is w * P[..., o-1]
+        for (int64_t r = tl.by; r < Qr; r += tl.gy) {
+            const T *wp = w + b + n * r;
+            T wv[DA];
 #pragma unroll
-                for (int i = 0; i < DA; ++i)
-                    if (i <= dd) acc += bw[i] * ld_as<T>(xp + i);
-            } else {  // kHomog
-                const int64_t r = q % Qr;
-                const int64_t o = q / Qr;  // 0: weight channel, o >= 1: w * P[..., o-1]
-                const T *wp = w + b + n * r;
+            for (int i = 0; i < DA; ++i) wv[i] = (i <= dd) ? bw[i] * wp[i] : T(0);
+            for (int64_t o = tl.bz; o <= nch; o += tl.gz) {
+                T acc = T(0);
                 if (o == 0) {
 #pragma unroll
                     for (int i = 0; i < DA; ++i)
-                        if (i <= dd) acc += bw[i] * wp[i];
+                        if (i <= dd) acc = ::fma(bw[i], wp[i], acc);
                 } else {
                     const TX *xp = X + b + n * (r + Qr * (o - 1));
 #pragma unroll
                     for (int i = 0; i < DA; ++i)
-                        if (i <= dd) acc += (bw[i] * wp[i]) * ld_as<T>(xp + i);
+                        if (i <= dd) acc = ::fma(wv[i], ld_as<T>(xp + i), acc);
                 }
+                Y[j + ns * (r + Qr * o)] = acc;
             }
+        }
+    } else {
+        const int64_t Qy = Qr * (int64_t)nch;
+#pragma unroll 4
+        for (int64_t q = tl.by; q < Qy; q += tl.gy) {
+            T acc = T(0);
+            const TX *xp = X + b + n * q;
+#pragma unroll
+            for (int i = 0; i < DA; ++i)
+                if (i <= dd) acc += bw[i] * ld_as<T>(xp + i);
             Y[j + ns * q] = acc;
         }
     }
@@ -283,8 +290,6 @@ fwd_axis0_tile(const Tile &tl, const int32_t *__restrict__ idx, const T *__restr
 // rows of the current knot span and reloads it only when the span changes (every
 // n_samples/n_basis samples), so X is read ~once per span while each output costs d+1
 // FMAs.  FINAL passes write eval with streaming stores.
-//   kRational (NURBS, last axis): Q is the NC channel axis of the homogeneous layout;
-//   the thread keeps NC windows and divides channels 1..nch by channel 0 in Float64.
 // ns: sample count of the axis (stride of B and Y); jcount: samples addressed by this
 // call, counted from the (possibly shifted) idx/B/Y bases.
 // ---------------------------------------------------------------------------------
@@ -293,12 +298,11 @@ __host__ __device__ constexpr int64_t fwd_axis_smem_bytes() {
     return align16(kChunk * 8) + align16(kChunk * DegreeTraits<D>::DP * (int64_t)sizeof(T));
 }
 
-template <int D, typename T, int VEC, int MODE, int NC, bool FINAL, bool CG, bool ST>
+template <int D, typename T, int VEC, bool FINAL, bool CG, bool ST>
 __device__ __forceinline__ void
 fwd_axis_tile(const Tile &tl, unsigned char *smem, const int32_t *__restrict__ idx,
               const T *__restrict__ B, int64_t ns, int64_t jcount, int d,
-              const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int nch,
-              T *__restrict__ Y) {
+              const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, T *__restrict__ Y) {
     using DT = DegreeTraits<D>;
     constexpr int DA = DT::DA;
     constexpr int DP = DT::DP;
@@ -323,79 +327,32 @@ fwd_axis_tile(const Tile &tl, unsigned char *smem, const int32_t *__restrict__ i
     if (nv == 0) return;
     const int jn = (int)((jcount - j0) < kChunk ? (jcount - j0) : kChunk);
 
-    if constexpr (MODE == kPlain) {
-        for (int64_t q = tl.bz; q < Q; q += tl.gz) {
-            const T *xq = X + m0 + M * n * q;
-            T *yq = Y + m0 + M * (j0 + ns * q);
-            Pack<T, VEC> win[DA];
-            int64_t bprev = -1;
-            for (int t = 0; t < jn; ++t) {
-                const int64_t b = s_b[t];
-                if (b != bprev) {
-#pragma unroll
-                    for (int i = 0; i < DA; ++i)
-                        if (i <= dd) win[i] = ldm<CG, ST, T, VEC>(xq + M * (b + i), ls, nv);
-                    bprev = b;
-                }
-                Pack<T, VEC> acc;
-#pragma unroll
-                for (int v = 0; v < VEC; ++v) acc.v[v] = T(0);
-                T bv[DA];
-                basis_row<T, DA, DP>(s_B + t * DP, bv);
-#pragma unroll
-                for (int i = 0; i < DA; ++i) {
-                    if (i <= dd) {
-#pragma unroll
-                        for (int v = 0; v < VEC; ++v) acc.v[v] += bv[i] * win[i].v[v];
-                    }
-                }
-                stm<FINAL, ST, T, VEC>(yq + M * t, acc, ls, nv);
-            }
-        }
-    } else {  // kRational: channels 0..nch in-thread (nch + 1 <= NC)
-        if (tl.bz != 0) return;
-        Pack<T, VEC> win[NC][DA];
+    for (int64_t q = tl.bz; q < Q; q += tl.gz) {
+        const T *xq = X + m0 + M * n * q;
+        T *yq = Y + m0 + M * (j0 + ns * q);
+        Pack<T, VEC> win[DA];
         int64_t bprev = -1;
         for (int t = 0; t < jn; ++t) {
             const int64_t b = s_b[t];
             if (b != bprev) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c)
-                    if (c <= nch) {
-                        const T *xc = X + m0 + M * n * c;
-#pragma unroll
-                        for (int i = 0; i < DA; ++i)
-                            if (i <= dd) win[c][i] = ldm<CG, ST, T, VEC>(xc + M * (b + i), ls, nv);
-                    }
+                for (int i = 0; i < DA; ++i)
+                    if (i <= dd) win[i] = ldm<CG, ST, T, VEC>(xq + M * (b + i), ls, nv);
                 bprev = b;
             }
-            Pack<T, VEC> acc[NC];
+            Pack<T, VEC> acc;
 #pragma unroll
-            for (int c = 0; c < NC; ++c)
-#pragma unroll
-                for (int v = 0; v < VEC; ++v) acc[c].v[v] = T(0);
+            for (int v = 0; v < VEC; ++v) acc.v[v] = T(0);
             T bv[DA];
             basis_row<T, DA, DP>(s_B + t * DP, bv);
 #pragma unroll
             for (int i = 0; i < DA; ++i) {
                 if (i <= dd) {
 #pragma unroll
-                    for (int c = 0; c < NC; ++c)
-                        if (c <= nch)
-#pragma unroll
-                            for (int v = 0; v < VEC; ++v) acc[c].v[v] += bv[i] * win[c][i].v[v];
+                    for (int v = 0; v < VEC; ++v) acc.v[v] += bv[i] * win[i].v[v];
                 }
             }
-#pragma unroll
-            for (int c = 1; c < NC; ++c) {
-                if (c <= nch) {
-                    Pack<T, VEC> r;
-#pragma unroll
-                    for (int v = 0; v < VEC; ++v)
-                        r.v[v] = (T)((double)acc[c].v[v] / (double)acc[0].v[v]);
-                    stm<true, ST, T, VEC>(Y + m0 + M * ((j0 + t) + ns * (int64_t)(c - 1)), r, ls, nv);
-                }
-            }
+            stm<FINAL, ST, T, VEC>(yq + M * t, acc, ls, nv);
         }
     }
 }
@@ -685,14 +642,13 @@ k_fwd_axis0(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns
     fwd_axis0_tile<D, TX, T, MODE>(grid_tile(), idx, B, ns, d, X, w, n, Qr, nch, Y);
 }
 
-template <int D, typename T, int VEC, int MODE, int NC, bool FINAL, bool ST>
+template <int D, typename T, int VEC, bool FINAL, bool ST>
 __global__ void __launch_bounds__(kThreads)
 k_fwd_axis(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns,
            int64_t jcount, int d, const T *__restrict__ X, int64_t M, int64_t n, int64_t Q,
-           int nch, T *__restrict__ Y) {
+           T *__restrict__ Y) {
     __shared__ __align__(16) unsigned char smem[fwd_axis_smem_bytes<D, T>()];
-    fwd_axis_tile<D, T, VEC, MODE, NC, FINAL, false, ST>(grid_tile(), smem, idx, B, ns, jcount, d,
-                                                         X, M, n, Q, nch, Y);
+    fwd_axis_tile<D, T, VEC, FINAL, false, ST>(grid_tile(), smem, idx, B, ns, jcount, d, X, M, n, Q, Y);
 }
 
 template <int D, typename T, int VEC, bool ST>

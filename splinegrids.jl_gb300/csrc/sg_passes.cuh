@@ -70,12 +70,16 @@ inline int vec_width(const AxisPass &p) {
 template <typename T, typename TX, int D, int MODE>
 inline void launch_fwd_axis0_t(const AxisPass &p, cudaStream_t s) {
     const unsigned gx = (unsigned)((p.ns + kThreads - 1) / kThreads);
-    int64_t Qy = (MODE == kHomog) ? p.Q * (p.nch + 1) : (MODE == kRational ? 1 : p.Q * p.nch);
+    int64_t Qy = (MODE == kHomog) ? p.Q : (MODE == kRational ? 1 : p.Q * p.nch);
     // each thread walks Qy/gridDim.y columns with its basis values in registers; size
     // grid.y for ~32 CTAs per SM (a few columns per thread: more loads in flight per SM)
     // rather than one output per thread
-    const int64_t want_y = (kTargetCtas * 4 + gx - 1) / gx;
+    const int64_t want_y = (kTargetCtas * (MODE == kHomog ? 2 : 4) + gx - 1) / gx;
     dim3 grid(gx, gdim(Qy < want_y ? Qy : want_y, kMaxGridYZ));
+    if (MODE == kHomog) {  // channels in turn by one thread unless that leaves too few blocks
+        const int64_t z = want_y / grid.y;
+        grid.z = gdim(z < p.nch + 1 ? z : p.nch + 1, kMaxGridYZ);
+    }
     k_fwd_axis0<D, TX, T, MODE><<<grid, kThreads, 0, s>>>(
         p.idx, (const T *)p.B, p.ns, p.d, (const TX *)p.X, (const T *)p.w, p.n, p.Q, p.nch,
         (T *)p.Y);
@@ -133,7 +137,7 @@ inline void launch_fwd_axis0_m(const AxisPass &p, cudaStream_t s) {
 
 
 // ------------------------------------------------------------------ forward axis k
-template <typename T, int D, int VEC, int MODE, int NC, bool FINAL, bool ST>
+template <typename T, int D, int VEC, bool FINAL, bool ST>
 inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
     const int64_t per_cta = (int64_t)kThreads * VEC;
     const unsigned gx = (unsigned)((p.M + per_cta - 1) / per_cta);
@@ -144,10 +148,10 @@ inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
         const int64_t cn = (chunks - c0 < kMaxGridYZ) ? chunks - c0 : kMaxGridYZ;
         const int64_t jb = c0 * kChunk;
         const int64_t jcount = (p.ns - jb < cn * kChunk) ? p.ns - jb : cn * kChunk;
-        dim3 grid(gx, (unsigned)cn, MODE == kRational ? 1u : gdim(p.Q, kMaxGridYZ));
-        k_fwd_axis<D, T, VEC, MODE, NC, FINAL, ST><<<grid, kThreads, 0, s>>>(
+        dim3 grid(gx, (unsigned)cn, gdim(p.Q, kMaxGridYZ));
+        k_fwd_axis<D, T, VEC, FINAL, ST><<<grid, kThreads, 0, s>>>(
             p.idx + jb, (const T *)p.B + jb, p.ns, jcount, p.d, (const T *)p.X, p.M, p.n, p.Q,
-            p.nch, (T *)p.Y + p.M * jb);
+            (T *)p.Y + p.M * jb);
     }
 }
 
@@ -155,28 +159,41 @@ inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
 // to kThreadFwdValues outputs, where the tasks leave most of the GPU idle ((50, 50, 25) x 4,
 // Float64, all three axes: 6.7 us against 24.5; at 6 M outputs the threads take 35 against 19)
 constexpr int64_t kThreadFwdValues = 1 << 19;
-template <typename T, int D, bool ST, bool FINAL>
+// Samples of a warp task: kFwdRowsMax, halved down to kFwdRowsMin while that leaves fewer than
+// 16 tasks an SM (Float64, whose rows take longer: 27).  A task runs its samples one after
+// the other, so few long tasks leave most of the chip idle; short ones load their windows
+// more often.  With 32 samples a task and with this rule, all passes: (64, 64) NURBS, (1024,
+// 1024) x 3 samples 20.9 and 8.9 us; (100, 100, 100) x 3 17.7 and 10.6; (200, 160, 120) Float64 54.7
+// and 44.6; with twice the tasks wanted (200, 300) NURBS, (2000, 3000) takes 15.5 for 12.5.
+constexpr int kFwdRowsMax = 32, kFwdRowsMin = 4;
+template <typename T>
+constexpr int64_t fwd_tasks() { return (int64_t)kNumSMs * (sizeof(T) == 4 ? 16 : 27); }
+template <typename T, int D, bool ST, bool FINAL, int NC = 0>
 inline void launch_fwd_warp(const AxisPass &p, cudaStream_t s) {
     const int64_t gxw = (p.M + warp_width<T>() - 1) / warp_width<T>();
-    const int64_t tasks = gxw * ((p.ns + kFwdGridRows - 1) / kFwdGridRows) * p.Q;
+    const int64_t Q = NC > 0 ? 1 : p.Q;  // rational: a task holds all channels
+    int rows = kFwdRowsMax;
+    while (rows > kFwdRowsMin && gxw * ((p.ns + rows - 1) / rows) * Q < fwd_tasks<T>()) rows /= 2;
+    const int64_t tasks = gxw * ((p.ns + rows - 1) / rows) * Q;
     const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
     if (blocks == 0) return;
-    const int64_t total = p.M * p.ns * p.Q;
-    if (total <= kThreadFwdValues) {
+    const int64_t total = p.M * p.ns * Q;
+    if (NC == 0 && total <= kThreadFwdValues) {
         k_fwd_thread<D, T><<<(unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s>>>(
             p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
             (T *)p.Y);
         return;
     }
-    k_fwd_warp<D, T, ST, FINAL><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.Q, gxw, (T *)p.Y);
+    k_fwd_warp<D, T, ST, FINAL, NC><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
+        p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, Q, NC > 0 ? (int)p.nch : 0, gxw,
+        (p.ns + rows - 1) / rows, rows, (T *)p.Y);
 }
 
 template <typename T, int D, int VEC, bool ST>
 inline void launch_fwd_axis_v(const AxisPass &p, cudaStream_t s) {
     if (p.mode == kRational) {
-        if (p.nch + 1 <= 2) launch_fwd_axis_t<T, D, VEC, kRational, 2, true, ST>(p, s);
-        else launch_fwd_axis_t<T, D, VEC, kRational, 4, true, ST>(p, s);
+        if (p.nch + 1 <= 2) launch_fwd_warp<T, D, ST, true, 2>(p, s);
+        else launch_fwd_warp<T, D, ST, true, 4>(p, s);
     } else if (p.final_pass) {
         launch_fwd_warp<T, D, ST, true>(p, s);
     } else {
@@ -222,8 +239,8 @@ inline void launch_fwd_axis(const AxisPass &p, cudaStream_t s) {
         case 4: launch_fwd_axis_plain<T, 5>(p, s); break;
         case 5: launch_fwd_axis_plain<T, 6>(p, s); break;
         default:  // any degree: runtime-degree kernel, scalar accesses
-            if (p.final_pass) launch_fwd_axis_t<T, 0, 1, kPlain, 1, true, false>(p, s);
-            else launch_fwd_axis_t<T, 0, 1, kPlain, 1, false, false>(p, s);
+            if (p.final_pass) launch_fwd_axis_t<T, 0, 1, true, false>(p, s);
+            else launch_fwd_axis_t<T, 0, 1, false, false>(p, s);
     }
 }
 

@@ -26,7 +26,6 @@ namespace sg {
 constexpr int kWarpRows = 32;     // rows staged per batch (one per lane)
 constexpr int kAdjGroup = 4;      // adjoint: rows loaded ahead per group (two groups in flight)
 constexpr int kFwdTaskRows = 128;  // forward: samples per warp task at most (batched tasks)
-constexpr int kFwdGridRows = 32;  // forward: samples per warp task of the per-grid kernel
 
 template <typename T>
 __host__ __device__ constexpr int warp_width() { return 32 * (16 / (int)sizeof(T)); }
@@ -38,7 +37,7 @@ __host__ __device__ constexpr int warp_adj_smem() {
 }
 template <int D, typename T>
 __host__ __device__ constexpr int warp_fwd_smem() {
-    return (int)align16(kFwdTaskRows * DegreeTraits<D>::DP * (int64_t)sizeof(T)) + kFwdTaskRows * 4;
+    return (int)align16(kFwdTaskRows * DegreeTraits<D>::DP * (int64_t)sizeof(T)) + kFwdTaskRows * 8;
 }
 
 // m-lanes of one warp task
@@ -203,14 +202,20 @@ adj_axis_warp(int64_t mw, int64_t chunk, int64_t q, int lane, unsigned char *wsm
 }
 
 // ---------------------------------------------------------------------------------
-// Forward pass over axis k >= 1 (kPlain):  Y[m, j, q] = sum_i B[j, i] X[m, b(j)+i, q].
+// Forward pass over axis k >= 1:  Y[m, j, q] = sum_i B[j, i] X[m, b(j)+i, q].
 // Task = (mw, jchunk, q) with jchunk = samples [j0, j0 + rows), rows <= kFwdTaskRows.  The warp keeps
 // the d+1 input rows of the current knot span in a rotating register window (phase p:
 // win[(p + i) % DA] holds row b + i) plus the row after it, fetched one run ahead; a
 // run of samples with one support start is evaluated with packed FMAs and no window
 // checks, and the window rotates by one row per advance of the support start (sorted
-// samples) or reloads on any other change.  FINAL passes write eval with streaming
-// stores.
+// samples) or reloads on any other change.  Where a run ends is staged with its support
+// start (counted over the warp's 32 staged rows; a run that goes on is met again as one
+// with the same start).  FINAL passes write eval with streaming stores.
+// NC > 0 (NURBS, last axis): the q axis holds the channels of the homogeneous layout; a
+// task keeps the windows of all nch + 1 <= NC of them and divides channels 1..nch by
+// channel 0, rounded as a Float64 division of the two would be.  Its windows are loaded
+// again at each new span (a row fetched ahead took 94 registers instead of 62).  It is bound
+// by the issue of its instructions, four fifths of them the divisions (97 a row of 128 values).
 // ---------------------------------------------------------------------------------
 template <int P, int DA, int VEC, typename T>
 __device__ __forceinline__ Pack<T, VEC> rot_dot_pack(const Pack<T, VEC> (&win)[DA], const T (&bv)[DA]) {
@@ -238,72 +243,107 @@ __device__ __forceinline__ Pack<T, VEC> rot_dot_pack(const Pack<T, VEC> (&win)[D
     return y;
 }
 
-template <int D, typename T, bool ST, bool FINAL>
+template <typename T, int VEC>
+__device__ __forceinline__ Pack<T, VEC> quotient(const Pack<T, VEC> &a, const Pack<T, VEC> &b) {
+    Pack<T, VEC> r;
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) r.v[v] = (T)((double)a.v[v] / (double)b.v[v]);
+    return r;
+}
+
+template <int D, typename T, bool ST, bool FINAL, int NC = 0>
 __device__ __forceinline__ void
 fwd_axis_warp(int64_t mw, int64_t jchunk, int rows, int64_t q, int lane, unsigned char *wsmem,
               const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns, int d,
-              const T *__restrict__ X, int64_t M, int64_t n, T *__restrict__ Y) {
+              const T *__restrict__ X, int64_t M, int64_t n, T *__restrict__ Y, int nch = 0) {
     using DT = DegreeTraits<D>;
     static_assert(D >= 1 && D <= 6, "forward warp tasks take degrees 0..5");
     constexpr int DA = DT::DA;
     constexpr int DP = DT::DP;
     constexpr int VEC = 16 / (int)sizeof(T);
+    constexpr int NW = NC > 0 ? NC : 1;  // windows
     const int dd = DT::deg(d);
     T *s_B = reinterpret_cast<T *>(wsmem);  // [kFwdTaskRows][DP]
-    int32_t *s_b = reinterpret_cast<int32_t *>(wsmem + align16(kFwdTaskRows * DP * (int64_t)sizeof(T)));
+    // support start of a row and the end of its run
+    int2 *s_b = reinterpret_cast<int2 *>(wsmem + align16(kFwdTaskRows * DP * (int64_t)sizeof(T)));
 
     const int64_t j0 = jchunk * rows;
     const int jn = (int)((ns - j0) < rows ? (ns - j0) : rows);
     __syncwarp();
-    for (int r = lane; r < jn; r += 32) {
+    for (int r0 = 0; r0 < jn; r0 += 32) {
+        const int r = r0 + lane;
         const int64_t j = j0 + r;
-        s_b[r] = (int32_t)support_start(idx[j], dd, n);
+        int b = -3;  // ends the last run
+        if (r < jn) {
+            b = (int)support_start(idx[j], dd, n);
 #pragma unroll
-        for (int i = 0; i < DP; ++i) s_B[r * DP + i] = (i <= dd) ? B[j + ns * i] : T(0);
+            for (int i = 0; i < DP; ++i) s_B[r * DP + i] = (i <= dd) ? B[j + ns * i] : T(0);
+        }
+        const int before = __shfl_up_sync(0xffffffffu, b, 1);
+        const unsigned heads = __ballot_sync(0xffffffffu, lane > 0 && b != before);
+        const unsigned after = (heads >> lane) >> 1;
+        if (r < jn) s_b[r] = make_int2(b, after ? r + __ffs((int)after) : r0 + 32);
     }
     __syncwarp();
     const WarpLanes<ST, VEC> ln(mw, lane, M);
     if (ln.nv == 0) return;
     const T *xq = X + ln.m0 + M * n * q;
     T *yq = Y + ln.m0 + M * (j0 + ns * q);
-    Pack<T, VEC> win[DA], nxt;
+    Pack<T, VEC> win[NW][DA], nxt;
     int p = 0, bprev = -2;
     int t = 0;
     while (t < jn) {
-        const int b = s_b[t];
-        int e = t + 1;
-        while (e < jn && s_b[e] == b) ++e;
-        if (b == bprev + 1) {  // rotate: the prefetched row after the window joins it
+        const int2 be = s_b[t];
+        const int b = be.x, e = be.y < jn ? be.y : jn;
+        if (NC == 0 && b == bprev + 1) {  // rotate: the prefetched row after the window joins it
             switch (p) {
-                case 0: win[0] = nxt; break;
-                case 1: win[1 % DA] = nxt; break;
-                case 2: win[2 % DA] = nxt; break;
-                case 4: if constexpr (DA > 4) win[4 % DA] = nxt; break;
-                case 5: if constexpr (DA > 5) win[5 % DA] = nxt; break;
-                default: win[3 % DA] = nxt; break;
+                case 0: win[0][0] = nxt; break;
+                case 1: win[0][1 % DA] = nxt; break;
+                case 2: win[0][2 % DA] = nxt; break;
+                case 4: if constexpr (DA > 4) win[0][4 % DA] = nxt; break;
+                case 5: if constexpr (DA > 5) win[0][5 % DA] = nxt; break;
+                default: win[0][3 % DA] = nxt; break;
             }
             p = (p + 1 == DA) ? 0 : p + 1;
         } else if (b != bprev) {
 #pragma unroll
-            for (int i = 0; i < DA; ++i) win[i] = ldw<ST, T, VEC>(xq + M * (b + i), ln.nv);
+            for (int c = 0; c < NW; ++c)
+                if (c <= nch)
+#pragma unroll
+                    for (int i = 0; i < DA; ++i)
+                        win[c][i] = ldw<ST, T, VEC>(xq + M * (b + i + n * c), ln.nv);
             p = 0;
         }
+        if (NC == 0 && b != bprev && b + dd + 1 < n) nxt = ldw<ST, T, VEC>(xq + M * (b + dd + 1), ln.nv);
         bprev = b;
-        if (b + dd + 1 < n) nxt = ldw<ST, T, VEC>(xq + M * (b + dd + 1), ln.nv);
-        switch (p) {
-#define SG_FWD_RUN(P)                                                          \
-    for (; t < e; ++t) {                                                       \
-        T bv[DA];                                                              \
-        basis_row<T, DA, DP>(s_B + t * DP, bv);                                \
-        stw<FINAL, ST, T, VEC>(yq + M * t, rot_dot_pack<(P) % DA>(win, bv), ln.nv); \
+        if constexpr (NC > 0) {
+#pragma unroll 1
+            for (; t < e; ++t) {
+                T bv[DA];
+                basis_row<T, DA, DP>(s_B + t * DP, bv);
+                const Pack<T, VEC> den = rot_dot_pack<0>(win[0], bv);
+#pragma unroll
+                for (int c = 1; c < NW; ++c)
+                    if (c <= nch)
+                        stw<FINAL, ST, T, VEC>(yq + M * (t + ns * (c - 1)),
+                                               quotient(rot_dot_pack<0>(win[c], bv), den), ln.nv);
+            }
+        } else {
+            switch (p) {
+#define SG_FWD_RUN(P)                                                                  \
+    for (; t < e; ++t) {                                                               \
+        T bv[DA];                                                                      \
+        basis_row<T, DA, DP>(s_B + t * DP, bv);                                        \
+        stw<FINAL, ST, T, VEC>(yq + M * t, rot_dot_pack<(P) % DA>(win[0], bv), ln.nv); \
     }
-            case 0: SG_FWD_RUN(0) break;
-            case 1: SG_FWD_RUN(1) break;
-            case 2: SG_FWD_RUN(2) break;
-            case 4: if constexpr (DA > 4) { SG_FWD_RUN(4) } break;
-            case 5: if constexpr (DA > 5) { SG_FWD_RUN(5) } break;
-            default: SG_FWD_RUN(3) break;
+                case 0: SG_FWD_RUN(0) break;
+                case 1: SG_FWD_RUN(1) break;
+                case 2: SG_FWD_RUN(2) break;
+                case 4: if constexpr (DA > 4) { SG_FWD_RUN(4) } break;
+                case 5: if constexpr (DA > 5) { SG_FWD_RUN(5) } break;
+                default: SG_FWD_RUN(3) break;
 #undef SG_FWD_RUN
+            }
         }
     }
 }
@@ -570,19 +610,28 @@ k_fwd0_warp(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns
     fwd0_warp<D, T>(cg * 32, s0, s1, lane, smem + w * warp_fwd0_smem<D, T>(), idx, B, ns, d, X, n, Q, Y);
 }
 
-template <int D, typename T, bool ST, bool FINAL>
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+// (Float32 rational tasks of two channels are held to 64 registers: 32 warps an SM.)
+template <int D, typename T, bool ST, bool FINAL, int NC>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock, (NC == 2 && sizeof(T) == 4) ? 8 : 1)
 k_fwd_warp(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns, int d,
-           const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int64_t gxw,
-           T *__restrict__ Y) {
+           const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int nch, int64_t gxw, int64_t jchunks,
+           int rows, T *__restrict__ Y) {
     __shared__ __align__(16) unsigned char smem[kWarpsPerBlock * warp_fwd_smem<D, T>()];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w;
-    const int64_t jchunks = (ns + kFwdGridRows - 1) / kFwdGridRows;
     if (task >= gxw * jchunks * Q) return;
-    const int64_t mw = task % gxw, r = task / gxw;
-    fwd_axis_warp<D, T, ST, FINAL>(mw, r % jchunks, kFwdGridRows, r / jchunks, lane, smem + w * warp_fwd_smem<D, T>(),
-                                   idx, B, ns, d, X, M, n, Y);
+    int64_t mw, chunk, q, r;
+    if (gxw * jchunks * Q <= UINT32_MAX) {  // 32-bit divisions, a quarter of the set-up's instructions fewer
+        r = (uint32_t)task / (uint32_t)gxw;
+        q = (uint32_t)r / (uint32_t)jchunks;
+    } else {
+        r = task / gxw;
+        q = r / jchunks;
+    }
+    mw = task - r * gxw;
+    chunk = r - q * jchunks;
+    fwd_axis_warp<D, T, ST, FINAL, NC>(mw, chunk, rows, q, lane, smem + w * warp_fwd_smem<D, T>(),
+                                       idx, B, ns, d, X, M, n, Y, nch);
 }
 
 }  // namespace sg

@@ -99,4 +99,45 @@ __device__ __forceinline__ int64_t support_start(int32_t idx, int d, int64_t n) 
     return clamp64((int64_t)idx - d - 1, 0, n - 1 - d);
 }
 
+// ---------------------------------------------------------------------------------
+// Launches in a row.  launch() lets the GPU set a kernel up while the kernel before it in the
+// stream ends (programmatic stream serialization); the kernel's first statement, grid_start,
+// waits until that kernel has completed and its writes are visible.  It saves 1 to 2 us a
+// launch: forward and adjoint of (10, 10, 5) control points, (50, 50, 25) x 4 samples, Float64, six
+// passes, 43 us without and 28 with it; (64, 64), (1024, 1024), two launches, 19.5 and 14.8.
+// Kernels never signal their completion early: blocks of the next pass that take places
+// while this one's last blocks run sit unevenly over the SMs (adjoint of (120, 100), (1040,
+// 731) x 3, Float64: 71 us with the signal at the start, 43 without).  The batch kernels, one
+// launch each way, gain nothing and are launched plainly.
+//
+// No load may move before the wait, not even one the compiler takes to be of memory that
+// nobody writes (const __restrict__ parameters): a kernel adds the returned zero, which only the
+// wait's asm produces, to the block number that all its addresses follow from, or passes its
+// input pointers through.  The number costs less: Float64 adjoint of (256, 256), (4096, 4096) x
+// 3 and its forward 879 us with the pointers, 857 with the number.
+// ---------------------------------------------------------------------------------
+template <typename... P>
+__device__ __forceinline__ uint32_t grid_start(P &...inputs) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint32_t zero;
+    asm volatile("mov.u32 %0, 0;" : "=r"(zero)::"memory");
+    ((inputs += zero), ...);
+    return zero;
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace sg

@@ -639,7 +639,9 @@ __global__ void __launch_bounds__(kThreads)
 k_fwd_axis0(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns, int d,
             const TX *__restrict__ X, const T *__restrict__ w, int64_t n, int64_t Qr, int nch,
             T *__restrict__ Y) {
-    fwd_axis0_tile<D, TX, T, MODE>(grid_tile(), idx, B, ns, d, X, w, n, Qr, nch, Y);
+    Tile tl = grid_tile();
+    tl.bx += grid_start();
+    fwd_axis0_tile<D, TX, T, MODE>(tl, idx, B, ns, d, X, w, n, Qr, nch, Y);
 }
 
 template <int D, typename T, int VEC, bool FINAL, bool ST>
@@ -647,6 +649,7 @@ __global__ void __launch_bounds__(kThreads)
 k_fwd_axis(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns,
            int64_t jcount, int d, const T *__restrict__ X, int64_t M, int64_t n, int64_t Q,
            T *__restrict__ Y) {
+    grid_start(idx, B, X);
     __shared__ __align__(16) unsigned char smem[fwd_axis_smem_bytes<D, T>()];
     fwd_axis_tile<D, T, VEC, FINAL, false, ST>(grid_tile(), smem, idx, B, ns, jcount, d, X, M, n, Q, Y);
 }
@@ -657,6 +660,7 @@ k_adj_axis(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
            const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
            const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int CC,
            T *__restrict__ Y) {
+    grid_start(idx, perm, lb, B, X);
     extern __shared__ __align__(16) unsigned char s_dyn[];
     adj_axis_tile<D, T, VEC, false, ST>(grid_tile(), s_dyn, idx, perm, lb, B, ns, d, X, M, n, Q,
                                         CC, Y);
@@ -667,6 +671,7 @@ __global__ void __launch_bounds__(kAdj0Threads)
 k_adj_axis0(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
             const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
             const T *__restrict__ X, int64_t n, int64_t Q, int QT, T *__restrict__ Y) {
+    grid_start(idx, perm, lb, B, X);
     extern __shared__ __align__(16) unsigned char s_dyn[];
     adj_axis0_tile<D, T, false>(grid_tile(), s_dyn, idx, perm, lb, B, ns, d, X, n, Q, QT, Y);
 }
@@ -678,6 +683,7 @@ __global__ void __launch_bounds__(kThreads)
 k_fwd_axis_rational_generic(const int32_t *__restrict__ idx, const T *__restrict__ B,
                             int64_t ns, int d, const T *__restrict__ X, int64_t M, int64_t n,
                             int nch, T *__restrict__ Y) {
+    grid_start(idx, B, X);
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
     for (int64_t j = blockIdx.y; j < ns; j += gridDim.y) {

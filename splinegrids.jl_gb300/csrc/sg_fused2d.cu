@@ -15,6 +15,7 @@ static int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 template <typename T, typename TX>
 __global__ void __launch_bounds__(kF2Lanes * kF2FwdWarps, 3)
 k_f2_fwd_grid(F2Grid g, F2Tiling tiling) {
+    grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ F2Grid s_g;
     if (threadIdx.x == 0) s_g = g;
@@ -30,6 +31,7 @@ k_f2_fwd_grid(F2Grid g, F2Tiling tiling) {
 template <typename T, typename TX>
 __global__ void __launch_bounds__(kF2TileWarps * 32, sizeof(T) == 4 ? 5 : 4)
 k_f2_fwdt_grid(F2Grid g, F2Tiling tiling) {
+    grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
     const F2Tile t = tiling.tile((int64_t)blockIdx.x, 2, g.nch, g.ns0, g.ns1);
     f2_run_forward_tile<T, TX>(g, t, smem);
@@ -51,6 +53,7 @@ k_f2_fwdt_batch(const F2Grid *__restrict__ grids, const F2Tile *__restrict__ til
 template <typename T>
 __global__ void __launch_bounds__(kF2AdjThreads, 2)
 k_f2_adj_grid(F2Grid g, F2Tiling tiling, int *status) {
+    grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ F2Grid s_g;
     __shared__ F2Tile s_t;
@@ -292,14 +295,14 @@ static int launch_grid_t(const F2Grid &g, const F2Tiling &t, int kind, int *stat
     }
     if (kind == 2) {
         if (n > 0x7fffffffLL) return set_error(SG_ERR_UNSUPPORTED, "fused 2D: too many tiles");
-        k_f2_fwdt_grid<T, TX><<<(unsigned)n, kF2TileWarps * 32, (size_t)f2_tile_smem<T>(), s>>>(g, t);
+        launch(k_f2_fwdt_grid<T, TX>, (unsigned)n, kF2TileWarps * 32, (size_t)f2_tile_smem<T>(), s, g, t);
     } else if (kind == 0) {
         const int64_t blocks = cdiv(n, kF2FwdWarps);
         if (blocks > 0x7fffffffLL) return set_error(SG_ERR_UNSUPPORTED, "fused 2D: too many units");
-        k_f2_fwd_grid<T, TX><<<(unsigned)blocks, kF2Lanes * kF2FwdWarps, (size_t)f2_fwd_smem<T>(), s>>>(g, t);
+        launch(k_f2_fwd_grid<T, TX>, (unsigned)blocks, kF2Lanes * kF2FwdWarps, (size_t)f2_fwd_smem<T>(), s, g, t);
     } else if constexpr (std::is_same<T, TX>::value) {
         if (n > 0x7fffffffLL) return set_error(SG_ERR_UNSUPPORTED, "fused 2D: too many tiles");
-        k_f2_adj_grid<T><<<(unsigned)n, kF2AdjThreads, (size_t)f2_adj_smem<T>(), s>>>(g, t, status);
+        launch(k_f2_adj_grid<T>, (unsigned)n, kF2AdjThreads, (size_t)f2_adj_smem<T>(), s, g, t, status);
     }
     return cuda_check(cudaGetLastError(), "fused 2D launch");
 }

@@ -181,6 +181,7 @@ template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict__ b, T *__restrict__ U, int64_t m,
                                                 T *__restrict__ X, T *__restrict__ W, int64_t n,
                                                 LsqrShared L) {
+    grid_start(b);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     SumSq<T> s;
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -209,6 +210,7 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_axpby(const T *__restrict__ Xin, T *__restrict__ Y, int64_t n,
                                                 const T *__restrict__ W, int phase, LsqrShared L) {
+    grid_start(Xin, W);
     const LsqrState *st = L.st;
     if (st->done) {  // the solve has stopped: leave every vector as it is
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -425,6 +427,7 @@ __device__ void lsqr_estimate(const LsqrShared &L) {
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_xw(const T *__restrict__ V, T *__restrict__ W, T *__restrict__ X,
                                              int64_t n, LsqrShared L) {
+    grid_start(V);
     if (*L.skip_xw) return;
     const T t1 = (T)L.st->t1, t2 = (T)L.st->t2, ia = (T)L.st->inv_alpha;
     const int64_t stride = (int64_t)(gridDim.x - 1) * blockDim.x;
@@ -470,11 +473,11 @@ int lsqr_launch_axpby(sg_lsqr *h, const void *Xin, void *Y, int64_t len, int pha
                       cudaStream_t s) {
     const int nb = n_blocks(len);
     if (h->dtype == SG_F64)
-        k_lsqr_axpby<double><<<nb, kLsqrThreads, 0, s>>>((const double *)Xin, (double *)Y, len, (const double *)Wn,
-                                                        phase, lsqr_shared(h));
+        launch(k_lsqr_axpby<double>, nb, kLsqrThreads, 0, s, (const double *)Xin, (double *)Y, len,
+               (const double *)Wn, phase, lsqr_shared(h));
     else
-        k_lsqr_axpby<float><<<nb, kLsqrThreads, 0, s>>>((const float *)Xin, (float *)Y, len, (const float *)Wn,
-                                                       phase, lsqr_shared(h));
+        launch(k_lsqr_axpby<float>, nb, kLsqrThreads, 0, s, (const float *)Xin, (float *)Y, len,
+               (const float *)Wn, phase, lsqr_shared(h));
     return cuda_check(cudaGetLastError(), "k_lsqr_axpby launch");
 }
 
@@ -540,11 +543,11 @@ extern "C" int sg_lsqr_start(sg_lsqr *h, const void *b, sg_stream_t stream) {
     cudaStream_t s = (cudaStream_t)stream;
     const int nb = n_blocks(h->m > h->n ? h->m : h->n);
     if (h->dtype == SG_F64)
-        k_lsqr_start<double><<<nb, kLsqrThreads, 0, s>>>((const double *)b, (double *)h->U, h->m, (double *)h->X,
-                                                        (double *)h->W, h->n, lsqr_shared(h));
+        launch(k_lsqr_start<double>, nb, kLsqrThreads, 0, s, (const double *)b, (double *)h->U, h->m,
+               (double *)h->X, (double *)h->W, h->n, lsqr_shared(h));
     else
-        k_lsqr_start<float><<<nb, kLsqrThreads, 0, s>>>((const float *)b, (float *)h->U, h->m, (float *)h->X,
-                                                       (float *)h->W, h->n, lsqr_shared(h));
+        launch(k_lsqr_start<float>, nb, kLsqrThreads, 0, s, (const float *)b, (float *)h->U, h->m,
+               (float *)h->X, (float *)h->W, h->n, lsqr_shared(h));
     return cuda_check(cudaGetLastError(), "k_lsqr_start launch");
 }
 
@@ -560,11 +563,11 @@ extern "C" int sg_lsqr_after_adjoint(sg_lsqr *h, sg_stream_t stream) {
     if (rc) return rc;
     const int nb = n_blocks(h->n) + 1;
     if (h->dtype == SG_F64)
-        k_lsqr_xw<double><<<nb, kLsqrThreads, 0, s>>>((const double *)h->V, (double *)h->W,
-                                                     (double *)h->X, h->n, lsqr_shared(h));
+        launch(k_lsqr_xw<double>, nb, kLsqrThreads, 0, s, (const double *)h->V, (double *)h->W,
+               (double *)h->X, h->n, lsqr_shared(h));
     else
-        k_lsqr_xw<float><<<nb, kLsqrThreads, 0, s>>>((const float *)h->V, (float *)h->W,
-                                                    (float *)h->X, h->n, lsqr_shared(h));
+        launch(k_lsqr_xw<float>, nb, kLsqrThreads, 0, s, (const float *)h->V, (float *)h->W, (float *)h->X,
+               h->n, lsqr_shared(h));
     return cuda_check(cudaGetLastError(), "k_lsqr_xw launch");
 }
 

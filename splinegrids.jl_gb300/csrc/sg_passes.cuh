@@ -80,8 +80,8 @@ inline void launch_fwd_axis0_t(const AxisPass &p, cudaStream_t s) {
         const int64_t z = want_y / grid.y;
         grid.z = gdim(z < p.nch + 1 ? z : p.nch + 1, kMaxGridYZ);
     }
-    k_fwd_axis0<D, TX, T, MODE><<<grid, kThreads, 0, s>>>(
-        p.idx, (const T *)p.B, p.ns, p.d, (const TX *)p.X, (const T *)p.w, p.n, p.Q, p.nch,
+    launch(k_fwd_axis0<D, TX, T, MODE>, grid, kThreads, 0, s,
+           p.idx, (const T *)p.B, p.ns, p.d, (const TX *)p.X, (const T *)p.w, p.n, p.Q, p.nch,
         (T *)p.Y);
 }
 
@@ -112,8 +112,8 @@ inline void launch_fwd0_warp(const AxisPass &p, cudaStream_t s) {
     SC = SC < 32 ? 32 : SC;
     const int64_t tasks = groups * ((p.ns + SC - 1) / SC);
     const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    k_fwd0_warp<D, T><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.n, Qy, SC, (T *)p.Y);
+    launch(k_fwd0_warp<D, T>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s,
+           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.n, Qy, SC, (T *)p.Y);
 }
 
 template <typename T, typename TX>
@@ -149,8 +149,8 @@ inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
         const int64_t jb = c0 * kChunk;
         const int64_t jcount = (p.ns - jb < cn * kChunk) ? p.ns - jb : cn * kChunk;
         dim3 grid(gx, (unsigned)cn, gdim(p.Q, kMaxGridYZ));
-        k_fwd_axis<D, T, VEC, FINAL, ST><<<grid, kThreads, 0, s>>>(
-            p.idx + jb, (const T *)p.B + jb, p.ns, jcount, p.d, (const T *)p.X, p.M, p.n, p.Q,
+        launch(k_fwd_axis<D, T, VEC, FINAL, ST>, grid, kThreads, 0, s,
+           p.idx + jb, (const T *)p.B + jb, p.ns, jcount, p.d, (const T *)p.X, p.M, p.n, p.Q,
             (T *)p.Y + p.M * jb);
     }
 }
@@ -179,13 +179,13 @@ inline void launch_fwd_warp(const AxisPass &p, cudaStream_t s) {
     if (blocks == 0) return;
     const int64_t total = p.M * p.ns * Q;
     if (NC == 0 && total <= kThreadFwdValues) {
-        k_fwd_thread<D, T><<<(unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s>>>(
-            p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
+        launch(k_fwd_thread<D, T>, (unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s,
+           p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
             (T *)p.Y);
         return;
     }
-    k_fwd_warp<D, T, ST, FINAL, NC><<<(unsigned)blocks, 32 * kWarpsPerBlock, 0, s>>>(
-        p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, Q, NC > 0 ? (int)p.nch : 0, gxw,
+    launch(k_fwd_warp<D, T, ST, FINAL, NC>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s,
+           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, Q, NC > 0 ? (int)p.nch : 0, gxw,
         (p.ns + rows - 1) / rows, rows, (T *)p.Y);
 }
 
@@ -227,8 +227,8 @@ template <typename T>
 inline void launch_fwd_axis(const AxisPass &p, cudaStream_t s) {
     if (p.mode == kRational && (p.nch + 1 > 4 || p.d > 3)) {
         dim3 grid((unsigned)((p.M + kThreads - 1) / kThreads), gdim(p.ns, kMaxGridYZ));
-        k_fwd_axis_rational_generic<T><<<grid, kThreads, 0, s>>>(
-            p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.nch, (T *)p.Y);
+        launch(k_fwd_axis_rational_generic<T>, grid, kThreads, 0, s,
+           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.nch, (T *)p.Y);
         return;
     }
     switch (p.d) {
@@ -265,7 +265,8 @@ inline void launch_adj_axis_t(const AxisPass &p, cudaStream_t s) {
                              smem);
         attr_set = true;
     }
-    k_adj_axis<D, T, VEC, ST><<<grid, kThreads, smem, s>>>(p.idx, p.perm, p.lb, (const T *)p.B, p.ns,
+    launch(k_adj_axis<D, T, VEC, ST>, grid, kThreads, smem, s,
+           p.idx, p.perm, p.lb, (const T *)p.B, p.ns,
                                                      p.d, (const T *)p.X, p.M, p.n, p.Q, (int)CC,
                                                      (T *)p.Y);
 }
@@ -275,8 +276,8 @@ template <typename T, int D>
 inline void launch_adj_thread(const AxisPass &p, cudaStream_t s) {
     const int64_t total = p.M * p.n * p.Q;
     if (total == 0) return;
-    k_adj_thread<D, T><<<(unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s>>>(
-        p.perm, p.lb, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
+    launch(k_adj_thread<D, T>, (unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s,
+           p.perm, p.lb, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
         (T *)p.Y);
 }
 
@@ -320,8 +321,8 @@ inline void launch_adj_ring(const AxisPass &p, cudaStream_t s) {
     if (per_chunk == 0) return;
     const int64_t CC = adj_chunk(p, per_chunk, kRingLat, kRingPer);
     const int64_t chunks = (p.n + CC - 1) / CC;
-    k_adj_ring<D, T><<<(unsigned)(per_chunk * chunks), 32, (ring_smem<D, T>()), s>>>(
-        p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, (T *)p.Y);
+    launch(k_adj_ring<D, T>, (unsigned)(per_chunk * chunks), 32, (ring_smem<D, T>()), s,
+           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, (T *)p.Y);
 }
 template <typename T, int D>
 inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
@@ -331,8 +332,8 @@ inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
     const int64_t CC = sizeof(T) == 4 ? adj_chunk(p, per_chunk, kColsLat, kColsPer)
                                       : adj_chunk(p, per_chunk, 64 * D + kColsLat, 64 * D);
     const int64_t chunks = (p.n + CC - 1) / CC, units = per_chunk * chunks;
-    k_adj_cols<D, T, 8><<<(unsigned)((units + kColsWarps - 1) / kColsWarps), 32 * kColsWarps, 0, s>>>(
-        p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
+    launch(k_adj_cols<D, T, 8>, (unsigned)((units + kColsWarps - 1) / kColsWarps), 32 * kColsWarps, 0, s,
+           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
 }
 
 template <typename T, int D>
@@ -383,7 +384,8 @@ inline void launch_adj_axis0_t(const AxisPass &p, cudaStream_t s) {
                              (int)adj_axis0_smem_bytes<D, T>(32));
         attr_set = true;
     }
-    k_adj_axis0<D, T><<<grid, kAdj0Threads, smem, s>>>(p.idx, p.perm, p.lb, (const T *)p.B,
+    launch(k_adj_axis0<D, T>, grid, kAdj0Threads, smem, s,
+           p.idx, p.perm, p.lb, (const T *)p.B,
                                                        p.ns, p.d, (const T *)p.X, p.n, p.Q, QT,
                                                        (T *)p.Y);
 }
@@ -401,7 +403,8 @@ inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
         return;
     }
     const int smem = a0_smem<D, T>();
-    k_adj0_tile<D, T><<<(unsigned)tiles, 32 * kA0Warps, smem, s>>>(p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X,
+    launch(k_adj0_tile<D, T>, (unsigned)tiles, 32 * kA0Warps, smem, s,
+           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X,
                                                                    p.n, p.Q, groups, (T *)p.Y);
 }
 
@@ -430,12 +433,14 @@ inline int launch_adj_line_q(const AxisPass &p, cudaStream_t s) {
     cfg.gridDim = dim3((unsigned)(units * S));
     cfg.blockDim = dim3(kLineThreads);
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)S;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch()
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cuda_check(cudaLaunchKernelEx(&cfg, k_adj_line<D, T, QT>, p.perm, p.lb, (const T *)p.B, p.ns,
                                          (const T *)p.X, p.n, p.Q, S, (T *)p.Y),
                       "adjoint launch");

@@ -77,6 +77,7 @@ __device__ __noinline__ T mult_entry(const MultArgs &a, const T *__restrict__ B,
 // entry of Y.
 template <typename T>
 __global__ void k_mult(MultArgs a, const T *__restrict__ B, T *__restrict__ Y, int64_t NY) {
+    grid_start(B);
     for (int64_t lin = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; lin < NY;
          lin += (int64_t)gridDim.x * blockDim.x)
         Y[lin] = mult_entry(a, B, lin);
@@ -155,6 +156,7 @@ __device__ __noinline__ T mult_adjoint_entry(const MultArgs &a, const T *__restr
 template <typename T>
 __global__ void k_mult_adjoint(MultArgs a, const T *__restrict__ Y, T *__restrict__ B,
                                int64_t NB) {
+    grid_start(Y);
     for (int64_t lin = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; lin < NB;
          lin += (int64_t)gridDim.x * blockDim.x)
         B[lin] = mult_adjoint_entry(a, Y, lin);
@@ -248,7 +250,7 @@ __device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)
 template <typename T, int ND>
 __global__ void __launch_bounds__(kMultThreads)
 k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, int64_t NY, bool small) {
-    const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x;
+    const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NY) return;
     int64_t I[ND], c0[ND], st[ND], z0[ND];
     int n[ND];
@@ -292,7 +294,7 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
 template <typename T, int ND>
 __global__ void __launch_bounds__(kMultThreads)
 k_mult_adjoint_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ Y, T *__restrict__ B, int64_t NB, bool small) {
-    const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x;
+    const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NB) return;
     int64_t J[ND], lo[ND], hi[ND], st[ND];
     int n[ND];
@@ -396,6 +398,7 @@ __device__ __forceinline__ bool ref_linear(const RefIdx &r, const int32_t *ridx,
 template <typename T>
 __global__ void k_local_refinement(RefIdx r, int nout, int64_t n_ref, const int32_t *ridx,
                                    const T *vals, T *cp, int64_t ncp) {
+    grid_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n_ref) return;
     int64_t lin;
@@ -407,6 +410,7 @@ __global__ void k_local_refinement(RefIdx r, int nout, int64_t n_ref, const int3
 template <typename T>
 __global__ void k_local_refinement_adjoint(RefIdx r, int nout, int64_t n_ref,
                                            const int32_t *ridx, T *vals, T *cp, int64_t ncp) {
+    grid_start();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n_ref) return;
     int64_t lin;
@@ -489,8 +493,10 @@ static void launch_mult_nd(const MultArgs &a, const void *X, void *Y, int64_t N,
     }
     const unsigned blocks = (unsigned)((N + kMultThreads - 1) / kMultThreads);
     const bool small = N <= 0xffffffffLL;
-    if (ADJ) k_mult_adjoint_nd<T, ND><<<blocks, kMultThreads, 0, s>>>(p, a, (const T *)X, (T *)Y, N, small);
-    else k_mult_nd<T, ND><<<blocks, kMultThreads, 0, s>>>(p, a, (const T *)X, (T *)Y, N, small);
+    if (ADJ) launch(k_mult_adjoint_nd<T, ND>, blocks, kMultThreads, 0, s,
+           p, a, (const T *)X, (T *)Y, N, small);
+    else launch(k_mult_nd<T, ND>, blocks, kMultThreads, 0, s,
+           p, a, (const T *)X, (T *)Y, N, small);
 }
 
 template <typename T, bool ADJ>
@@ -499,8 +505,10 @@ static void launch_mult(const MultArgs &a, const void *X, void *Y, int64_t N, cu
     if (a.ndims == 2 && one_launch) launch_mult_nd<T, 2, ADJ>(a, X, Y, N, s);
     else if (a.ndims == 3 && one_launch) launch_mult_nd<T, 3, ADJ>(a, X, Y, N, s);
     else if (a.ndims == 4 && one_launch) launch_mult_nd<T, 4, ADJ>(a, X, Y, N, s);
-    else if (ADJ) k_mult_adjoint<T><<<grid_for(N, 256), 256, 0, s>>>(a, (const T *)X, (T *)Y, N);
-    else k_mult<T><<<grid_for(N, 256), 256, 0, s>>>(a, (const T *)X, (T *)Y, N);
+    else if (ADJ) launch(k_mult_adjoint<T>, grid_for(N, 256), 256, 0, s,
+           a, (const T *)X, (T *)Y, N);
+    else launch(k_mult<T>, grid_for(N, 256), 256, 0, s,
+           a, (const T *)X, (T *)Y, N);
 }
 
 extern "C" int sg_mult(int32_t dtype, int32_t ndims, const int64_t *size_Y,
@@ -570,11 +578,13 @@ extern "C" int sg_local_refinement(int32_t dtype, int32_t nin, int32_t nout,
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned g = (unsigned)((n_refined + 255) / 256);
     if (dtype == SG_F32)
-        k_local_refinement<float><<<g, 256, 0, s>>>(r, nout, n_refined, refinement_indices,
+        launch(k_local_refinement<float>, g, 256, 0, s,
+           r, nout, n_refined, refinement_indices,
                                                     (const float *)refinement_values,
                                                     (float *)control_points, ncp);
     else
-        k_local_refinement<double><<<g, 256, 0, s>>>(r, nout, n_refined, refinement_indices,
+        launch(k_local_refinement<double>, g, 256, 0, s,
+           r, nout, n_refined, refinement_indices,
                                                      (const double *)refinement_values,
                                                      (double *)control_points, ncp);
     return cuda_check(cudaGetLastError(), "k_local_refinement launch");
@@ -594,11 +604,13 @@ extern "C" int sg_local_refinement_adjoint(int32_t dtype, int32_t nin, int32_t n
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned g = (unsigned)((n_refined + 255) / 256);
     if (dtype == SG_F32)
-        k_local_refinement_adjoint<float><<<g, 256, 0, s>>>(r, nout, n_refined, refinement_indices,
+        launch(k_local_refinement_adjoint<float>, g, 256, 0, s,
+           r, nout, n_refined, refinement_indices,
                                                             (float *)refinement_values,
                                                             (float *)control_points, ncp);
     else
-        k_local_refinement_adjoint<double><<<g, 256, 0, s>>>(r, nout, n_refined, refinement_indices,
+        launch(k_local_refinement_adjoint<double>, g, 256, 0, s,
+           r, nout, n_refined, refinement_indices,
                                                              (double *)refinement_values,
                                                              (double *)control_points, ncp);
     return cuda_check(cudaGetLastError(), "k_local_refinement_adjoint launch");

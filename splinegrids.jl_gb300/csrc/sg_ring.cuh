@@ -100,7 +100,7 @@ k_adj_ring(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
     const int lane = threadIdx.x;
     unsigned char *const ring = smem + lane * 16, *const ring_end = ring + kRingRows * RB;
     V *s_B = reinterpret_cast<V *>(smem + kRingRows * RB);
-    const int64_t unit = blockIdx.x;
+    const int64_t unit = blockIdx.x + grid_start();
     const int64_t mw = unit % gxw, rest = unit / gxw;
     const int64_t chunk = rest % chunks, q = rest / chunks;
     const int c0 = (int)(chunk * CC);
@@ -249,7 +249,7 @@ k_adj_cols(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
     static_assert(32 % U == 0, "groups divide the staged batch");
     __shared__ __align__(16) T sh[kColsWarps][32 * RV];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t unit = (int64_t)blockIdx.x * kColsWarps + w;
+    const int64_t unit = (int64_t)blockIdx.x * kColsWarps + w + grid_start();
     if (unit >= units) return;
     T *s_B = sh[w];
     const int64_t mw = unit % gxw, rest = unit / gxw;
@@ -385,8 +385,9 @@ k_adj0_tile(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, co
     T *xs = reinterpret_cast<T *>(smem);  // [32][SEG + 1]
     T *bs = reinterpret_cast<T *>(smem + align16(32 * (SEG + 1) * (int64_t)sizeof(T)));  // [D][SEG]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t q0 = (blockIdx.x % groups) * 32;
-    const int c0 = (int)(blockIdx.x / groups) * kA0Cp;
+    const uint32_t tile = blockIdx.x + grid_start();
+    const int64_t q0 = (tile % groups) * 32;
+    const int c0 = (int)(tile / groups) * kA0Cp;
     const int c1 = c0 + kA0Cp < n ? c0 + kA0Cp : (int)n;
     const int s_lo = lb[c0], s_hi = lb[c1 + d];
     T acc[PER];
@@ -461,8 +462,9 @@ k_adj_line(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
     __shared__ T part[kLineThreads / 32][QT];
     __shared__ T total[QT];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int64_t unit = blockIdx.x / S;
-    const int rank = (int)(blockIdx.x % S);
+    const uint32_t block = blockIdx.x + grid_start();
+    const int64_t unit = block / S;
+    const int rank = (int)(block % S);
     const int64_t c = unit % n, q0 = (unit / n) * QT;
     const int64_t lo = lb[c], len = lb[c + D] - lo;
     const int64_t per = (len + S - 1) / S;
@@ -525,7 +527,7 @@ __global__ void __launch_bounds__(kThreadBlock)
 k_adj_thread(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, const T *__restrict__ B, uint32_t ns,
              const T *__restrict__ X, uint32_t M, uint32_t n, uint32_t total, T *__restrict__ Y) {
     constexpr int d = D - 1;
-    const uint32_t lin = blockIdx.x * kThreadBlock + threadIdx.x;
+    const uint32_t lin = blockIdx.x * kThreadBlock + threadIdx.x + grid_start();
     if (lin >= total) return;
     const uint32_t r = lin / M, m = lin - r * M;
     const uint32_t q = r / n, c = r - q * n;
@@ -560,7 +562,7 @@ template <int D, typename T>
 __global__ void __launch_bounds__(kThreadBlock)
 k_fwd_thread(const int32_t *__restrict__ idx, const T *__restrict__ B, uint32_t ns, const T *__restrict__ X, uint32_t M,
              uint32_t n, uint32_t total, T *__restrict__ Y) {
-    const uint32_t lin = blockIdx.x * kThreadBlock + threadIdx.x;
+    const uint32_t lin = blockIdx.x * kThreadBlock + threadIdx.x + grid_start();
     if (lin >= total) return;
     const uint32_t r = lin / M, m = lin - r * M;
     const uint32_t q = r / ns, j = r - q * ns;

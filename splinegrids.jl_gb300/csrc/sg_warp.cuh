@@ -602,7 +602,7 @@ k_fwd0_warp(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns
             const T *__restrict__ X, int64_t n, int64_t Q, int64_t SC, T *__restrict__ Y) {
     __shared__ __align__(16) unsigned char smem[kWarpsPerBlock * warp_fwd0_smem<D, T>()];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w;
+    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w + grid_start();
     const int64_t groups = (Q + 31) / 32, chunks = (ns + SC - 1) / SC;
     if (task >= groups * chunks) return;
     const int64_t cg = task % groups, s0 = (task / groups) * SC;
@@ -618,7 +618,7 @@ k_fwd_warp(const int32_t *__restrict__ idx, const T *__restrict__ B, int64_t ns,
            int rows, T *__restrict__ Y) {
     __shared__ __align__(16) unsigned char smem[kWarpsPerBlock * warp_fwd_smem<D, T>()];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w;
+    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w + grid_start();
     if (task >= gxw * jchunks * Q) return;
     int64_t mw, chunk, q, r;
     if (gxw * jchunks * Q <= UINT32_MAX) {  // 32-bit divisions, a quarter of the set-up's instructions fewer

@@ -167,14 +167,16 @@ __global__ void k_mult_adjoint(MultArgs a, const T *__restrict__ Y, T *__restric
 // volumes with their Nout dimension), every index array unrolled.  The kernels above are
 // bound by latency: their nine-entry index arrays live in local memory, and an odometer
 // re-reads row pointers, column starts and band values for every term, so a thread is one
-// chain of dependent loads.  Here a thread finds each dimension's band once, keeps the
-// factors of the two fastest dimensions in registers (kMultCap each) and its terms are
-// independent loads; entries with a wider band take the general function.  Terms and
-// factors keep their order, so only the contraction of the last product with the sum can
-// change a bit.  Measured on (16, 16, 8) -> (114, 114, 50), degree 2, three bisections,
-// Float32: mult! 71 -> 35 us, mult_adjoint! 204 -> 40 us (three launches each).
+// chain of dependent loads.  Here a thread finds each dimension's band once, and the sum is
+// the unrolled one for the widest band of its warp (2 to 5 terms a dimension, factors in
+// registers, independent loads) or plain loops for wider ones: bound by the terms'
+// instructions, so one sum for all widths up to 5, 25 predicated terms a plane, took 2 to 4
+// times as long.  Terms and factors keep their order, so only the contraction of the last
+// product with the sum can change a bit.  Measured, us, general kernels / one sum for all /
+// now: (58, 58, 26) -> (114, 114, 50), bands of 2, Float32: mult! 46 / 22 / 11.7, mult_adjoint! 79
+// / 17 / 12.6; bands of 3: 122 / - / 14.7, 231 / 286 / 39.6; (257, 257) x 3 -> (512, 512) x 3, bands of
+// 3, Float64: 54 / 75 / 39.6, 72 / 114 / 67.5.
 // ---------------------------------------------------------------------------------
-constexpr int kMultCap = 5;        // a bisected column is covered by degree + 2 rows (degree <= 3: 5)
 constexpr int kMultThreads = 128;
 
 template <int ND>
@@ -215,36 +217,92 @@ __device__ __forceinline__ void nd_decode(const int64_t (&size)[ND], int64_t lin
     }
 }
 
-// The sum over dimensions ND-1 .. 0 (0 fastest) of X at lo[d] + k_d < n[d], stride st[d],
-// times the factors; f(d, k): factor of dimension d >= 2 at term k; w0, w1: the factors
-// of dimensions 0 and 1.
-template <typename T, int ND, typename F>
-__device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)[ND], const int (&n)[ND],
-                                    const int64_t (&st)[ND], const T (&w0)[kMultCap], const T (&w1)[kMultCap], F f) {
-    int64_t base = 0;
+// The sum of x at k_d < n[d], stride st[d] (0 fastest), times the factors f(d, k) of dimension d at
+// term k, over the first NR dimensions.  n[d] <= C: the factors sit in registers, the loads of a
+// k2 are independent.
+template <int C, int NR, typename T, int ND, typename F>
+__device__ __forceinline__ T nd_sum_c(const T *__restrict__ x, const int (&n)[ND], const int64_t (&st)[ND], F f) {
+    constexpr int C1 = NR > 1 ? C : 1;
+    T w[NR][C];
 #pragma unroll
-    for (int d = 0; d < ND; ++d) base += lo[d] * st[d];
+    for (int d = 0; d < NR; ++d)
+#pragma unroll
+        for (int k = 0; k < C; ++k) w[d][k] = k < n[d] ? f(d, k) : T(1);
     T acc = T(0);
-    const int n2 = ND > 2 ? n[ND > 2 ? 2 : 0] : 1, n3 = ND > 3 ? n[ND > 3 ? 3 : 0] : 1;
+#pragma unroll(C == 2 ? 2 : 1)
+    for (int k2 = 0; k2 < (NR > 2 ? C : 1); ++k2) {
+        T w2 = T(1);
+        if constexpr (NR > 2) {
+            if (k2 >= n[2]) break;
+#pragma unroll
+            for (int k = 0; k < C; ++k) w2 = k == k2 ? w[2][k] : w2;
+        }
+        T v[C1][C];
+#pragma unroll
+        for (int k1 = 0; k1 < C1; ++k1)
+#pragma unroll
+            for (int k0 = 0; k0 < C; ++k0)
+                if ((NR < 2 || k1 < n[1]) && k0 < n[0]) v[k1][k0] = x[k0 + (NR > 1 ? k1 * st[1] : 0)];
+#pragma unroll
+        for (int k1 = 0; k1 < C1; ++k1)
+#pragma unroll
+            for (int k0 = 0; k0 < C; ++k0)
+                if ((NR < 2 || k1 < n[1]) && k0 < n[0]) {
+                    T t = v[k1][k0] * w[0][k0];
+                    if constexpr (NR > 1) t = t * w[1][k1];
+                    if constexpr (NR > 2) t = t * w2;
+                    acc += t;
+                }
+        if constexpr (NR > 2) x += st[2];
+    }
+    return acc;
+}
+
+// Bands of any width, all ND dimensions.
+template <typename T, int ND, typename F>
+__device__ __forceinline__ T nd_sum_any(const T *__restrict__ X, const int (&n)[ND], const int64_t (&st)[ND], F f) {
+    T acc = T(0);
+    const int n1 = n[1], n2 = ND > 2 ? n[ND > 2 ? 2 : 0] : 1, n3 = ND > 3 ? n[ND > 3 ? 3 : 0] : 1;
     for (int k3 = 0; k3 < n3; ++k3) {
         const T w3 = ND > 3 ? f(3, k3) : T(1);
         for (int k2 = 0; k2 < n2; ++k2) {
             const T w2 = ND > 2 ? f(2, k2) : T(1);
-            const T *x = X + base + (ND > 2 ? k2 * st[ND > 2 ? 2 : 0] : 0) + (ND > 3 ? k3 * st[ND > 3 ? 3 : 0] : 0);
-            T v[kMultCap][kMultCap];
-#pragma unroll
-            for (int k1 = 0; k1 < kMultCap; ++k1)
-#pragma unroll
-                for (int k0 = 0; k0 < kMultCap; ++k0)
-                    v[k1][k0] = (k1 < n[1] && k0 < n[0]) ? x[k0 + k1 * st[1]] : T(0);
-#pragma unroll
-            for (int k1 = 0; k1 < kMultCap; ++k1)
-#pragma unroll
-                for (int k0 = 0; k0 < kMultCap; ++k0)
-                    if (k1 < n[1] && k0 < n[0]) acc += v[k1][k0] * w0[k0] * w1[k1] * w2 * w3;
+            for (int k1 = 0; k1 < n1; ++k1) {
+                const T w1 = f(1, k1);
+                const T *x = X + k1 * st[1] + (ND > 2 ? k2 * st[ND > 2 ? 2 : 0] : 0) + (ND > 3 ? k3 * st[ND > 3 ? 3 : 0] : 0);
+#pragma unroll 4
+                for (int k0 = 0; k0 < n[0]; ++k0) acc += x[k0] * f(0, k0) * w1 * w2 * w3;
+            }
         }
     }
     return acc;
+}
+
+// The narrowest of the sums that holds every band of the warp's threads (the vote keeps the
+// warp in one of them): a term that a thread does not have costs it as much as one it has.
+// A row of a bisected dimension has degree / 2 + 1 columns at most, a column degree + 2 rows.
+// last: the last dimension is refined (Nout is not: no factors of one are multiplied).
+template <int NR, typename T, int ND, typename F>
+__device__ __forceinline__ T nd_sum_n(const T *__restrict__ x, const int (&n)[ND], const int64_t (&st)[ND], F f) {
+    int widest = n[0];
+#pragma unroll
+    for (int d = 1; d < NR; ++d) widest = n[d] > widest ? n[d] : widest;
+    const int cap = (int)__reduce_max_sync(__activemask(), (unsigned)widest);
+    if (cap <= 2) return nd_sum_c<2, NR>(x, n, st, f);
+    if (cap <= 3) return nd_sum_c<3, NR>(x, n, st, f);
+    if (cap <= 4) return nd_sum_c<4, NR>(x, n, st, f);
+    if (cap <= 5) return nd_sum_c<5, NR>(x, n, st, f);
+    return nd_sum_any(x, n, st, f);
+}
+template <typename T, int ND, typename F>
+__device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)[ND], const int (&n)[ND],
+                                    const int64_t (&st)[ND], bool last, F f) {
+    const T *x = X;
+#pragma unroll
+    for (int d = 0; d < ND; ++d) x += lo[d] * st[d];
+    if (!last) return nd_sum_n<ND - 1>(x, n, st, f);
+    if constexpr (ND < 4) return nd_sum_n<ND>(x, n, st, f);
+    else return nd_sum_any(x, n, st, f);
 }
 
 template <typename T, int ND>
@@ -267,7 +325,7 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
         if (p.rp[d]) {
             int64_t nc;
             nd_row(p, d, I[d], c0[d], nc, z0[d]);
-            fits = fits && (d > 1 || nc <= kMultCap) && (nc <= 0 || (c0[d] >= 0 && c0[d] + nc <= p.sB[d]));
+            fits = fits && (nc <= 0 || (c0[d] >= 0 && c0[d] + nc <= p.sB[d]));
             n[d] = nc < 0 ? 0 : (int)nc;
         }
     }
@@ -275,32 +333,25 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
         Y[lin] = mult_entry(a, B, lin);
         return;
     }
-    T w0[kMultCap], w1[kMultCap];
-#pragma unroll
-    for (int k = 0; k < kMultCap; ++k) {
-        w0[k] = p.rp[0] && k < n[0] ? ((const T *)p.nz[0])[z0[0] + k] : T(1);
-        w1[k] = p.rp[1] && k < n[1] ? ((const T *)p.nz[1])[z0[1] + k] : T(1);
-    }
     auto f = [&](int d, int k) {
-        if constexpr (ND > 3) {
-            if (d == 3) return p.rp[3] ? ((const T *)p.nz[3])[z0[3] + k] : T(1);
-        }
-        if constexpr (ND > 2) return p.rp[2] ? ((const T *)p.nz[2])[z0[2] + k] : T(1);
-        return T(1);
+        T r = T(1);
+#pragma unroll
+        for (int e = 0; e < ND; ++e)
+            if (e == d && p.rp[e]) r = ((const T *)p.nz[e])[z0[e] + k];
+        return r;
     };
-    Y[lin] = nd_sum<T, ND>(B, c0, n, st, w0, w1, f);
+    Y[lin] = nd_sum(B, c0, n, st, p.rp[ND - 1] != nullptr, f);
 }
 
 template <typename T, int ND>
 __global__ void __launch_bounds__(kMultThreads)
-k_mult_adjoint_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ Y, T *__restrict__ B, int64_t NB, bool small) {
+k_mult_adjoint_nd(MultNd<ND> p, const T *__restrict__ Y, T *__restrict__ B, int64_t NB, bool small) {
     const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NB) return;
     int64_t J[ND], lo[ND], hi[ND], st[ND];
     int n[ND];
     nd_decode<ND>(p.sB, lin, small, J);
     int64_t acc = 1;
-    bool fits = true;
 #pragma unroll
     for (int d = 0; d < ND; ++d) {
         st[d] = acc;
@@ -342,33 +393,21 @@ k_mult_adjoint_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ Y, T *__restri
             lo[d] = l1[d];
             hi[d] = l0[d];
             const int64_t c = hi[d] > lo[d] ? hi[d] - lo[d] : 0;
-            fits = fits && (d > 1 || c <= kMultCap);
             n[d] = (int)c;
         }
     }
-    if (!fits) {
-        B[lin] = mult_adjoint_entry(a, Y, lin);
-        return;
-    }
-    auto factor = [&](int d, int k) {  // A_d[lo + k, J]
-        int64_t c0, nc, z0;
-        nd_row(p, d, lo[d] + k, c0, nc, z0);
-        return ((const T *)p.nz[d])[z0 + (J[d] - c0)];
-    };
-    T w0[kMultCap], w1[kMultCap];
+    auto f = [&](int d, int k) {  // A_d[lo + k, J]
+        T r = T(1);
 #pragma unroll
-    for (int k = 0; k < kMultCap; ++k) {
-        w0[k] = p.rp[0] && k < n[0] ? factor(0, k) : T(1);
-        w1[k] = p.rp[1] && k < n[1] ? factor(1, k) : T(1);
-    }
-    auto f = [&](int d, int k) {
-        if constexpr (ND > 3) {
-            if (d == 3) return p.rp[3] ? factor(3, k) : T(1);
-        }
-        if constexpr (ND > 2) return p.rp[2] ? factor(2, k) : T(1);
-        return T(1);
+        for (int e = 0; e < ND; ++e)
+            if (e == d && p.rp[e]) {
+                int64_t c0, nc, z0;
+                nd_row(p, e, lo[e] + k, c0, nc, z0);
+                r = ((const T *)p.nz[e])[z0 + (J[e] - c0)];
+            }
+        return r;
     };
-    B[lin] = nd_sum<T, ND>(Y, lo, n, st, w0, w1, f);
+    B[lin] = nd_sum(Y, lo, n, st, p.rp[ND - 1] != nullptr, f);
 }
 
 struct RefIdx {
@@ -494,7 +533,7 @@ static void launch_mult_nd(const MultArgs &a, const void *X, void *Y, int64_t N,
     const unsigned blocks = (unsigned)((N + kMultThreads - 1) / kMultThreads);
     const bool small = N <= 0xffffffffLL;
     if (ADJ) launch(k_mult_adjoint_nd<T, ND>, blocks, kMultThreads, 0, s,
-           p, a, (const T *)X, (T *)Y, N, small);
+           p, (const T *)X, (T *)Y, N, small);
     else launch(k_mult_nd<T, ND>, blocks, kMultThreads, 0, s,
            p, a, (const T *)X, (T *)Y, N, small);
 }

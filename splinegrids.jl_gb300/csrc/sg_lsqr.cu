@@ -29,14 +29,17 @@
 // of the rules), so a whole solve is one graph launch with no host round trip.
 #include <math.h>
 
+#include <type_traits>
+
 #include "sg_common.cuh"
 
 namespace sg {
 namespace {
 
 constexpr int kLsqrThreads = 256;
-// Grid of the vector passes: two blocks per SM at most.  (4.2 M values, Float32: 304 blocks
-// 10.3 us, 1216 blocks 12.3: every block ends with a Float64 reduction.)
+// Grid of the vector passes: two blocks per SM at most.  (Every block ends with a Float64
+// reduction: 12 iterations of a (2048, 2048) Float32 fit take 653 us with 304 blocks, 712 with
+// 608, 774 with 912.)
 constexpr int kLsqrMaxBlocks = 2 * 152;
 
 struct LsqrState {
@@ -176,6 +179,30 @@ __device__ __forceinline__ void lsqr_finish(const LsqrShared &L, double s, doubl
     }
 }
 
+// Calls step(V, G, i, gap) for the thread's share of n values: G groups of V consecutive ones at
+// i, i + gap, ...  16-byte groups where every pointer allows it (two in flight for each
+// operand), else four single values: the passes wait for memory, so bytes in flight count
+// (12 iterations of a (2048, 2048) Float32 fit: 687 us with single values, 649 with groups).
+template <int V> using Count = std::integral_constant<int, V>;
+template <typename T, typename F>
+__device__ __forceinline__ void lsqr_each(int64_t n, bool packed, int64_t i0, int64_t stride, F step) {
+    constexpr int V = 16 / (int)sizeof(T);
+    int64_t i = i0;
+    if (packed) {
+        const int64_t np = n / V;
+        for (; i + stride < np; i += 2 * stride) step(Count<V>{}, Count<2>{}, i * V, stride * V);
+        if (i < np) step(Count<V>{}, Count<1>{}, i * V, (int64_t)0);
+        if (np * V + i0 < n) step(Count<1>{}, Count<1>{}, np * V + i0, (int64_t)0);
+    } else {
+        for (; i + 3 * stride < n; i += 4 * stride) step(Count<1>{}, Count<4>{}, i, stride);
+        for (; i < n; i += stride) step(Count<1>{}, Count<1>{}, i, (int64_t)0);
+    }
+}
+template <typename... P>
+__device__ __forceinline__ bool aligned16(const P *...p) {
+    return (((uintptr_t)p | ...) & 15) == 0;
+}
+
 // U = b, and (n-space) X = 0, W = 0; the sum of b^2 and the start of the recurrence.
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict__ b, T *__restrict__ U, int64_t m,
@@ -184,20 +211,18 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict
     grid_start(b);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     SumSq<T> s;
-    int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i + 3 * stride < m; i += 4 * stride) {
-        T v[4];
+    lsqr_each<T>(m, aligned16(b, U), (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride,
+                 [&](auto vc, auto gc, int64_t i, int64_t gap) {
+        constexpr int V = decltype(vc)::value, G = decltype(gc)::value;
+        Pack<T, V> v[G];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = b[i + k * stride];
+        for (int g = 0; g < G; ++g) v[g] = ldp<T, V>(b + i + g * gap);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) U[i + k * stride] = v[k];
-        s.add(v);
-    }
-    for (; i < m; i += stride) {
-        const T v[1] = {b[i]};
-        U[i] = v[0];
-        s.add(v);
-    }
+        for (int g = 0; g < G; ++g) {
+            stp<T, V>(U + i + g * gap, v[g]);
+            s.add(v[g].v);
+        }
+    });
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         X[i] = T(0);
         W[i] = T(0);
@@ -223,30 +248,25 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_axpby(const T *__restrict
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     SumSq<T> s, s2;
-    int64_t i = i0;
-    // four independent elements in flight per thread
-    for (; i + 3 * stride < n; i += 4 * stride) {
-        T x[4], y[4];
+    lsqr_each<T>(n, aligned16(Xin, Y, W), i0, stride, [&](auto vc, auto gc, int64_t i, int64_t gap) {
+        constexpr int V = decltype(vc)::value, G = decltype(gc)::value;
+        Pack<T, V> x[G], y[G], w[G];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { x[k] = Xin[i + k * stride]; y[k] = Y[i + k * stride]; }
+        for (int g = 0; g < G; ++g) {
+            x[g] = ldp<T, V>(Xin + i + g * gap);
+            y[g] = ldp<T, V>(Y + i + g * gap);
+            if (W) w[g] = ldp<T, V>(W + i + g * gap);
+        }
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            y[k] = bb == T(0) ? a * x[k] : fma(a, x[k], bb * y[k]);
-            Y[i + k * stride] = y[k];
+        for (int g = 0; g < G; ++g) {
+#pragma unroll
+            for (int k = 0; k < V; ++k)
+                y[g].v[k] = bb == T(0) ? a * x[g].v[k] : fma(a, x[g].v[k], bb * y[g].v[k]);
+            stp<T, V>(Y + i + g * gap, y[g]);
+            s.add(y[g].v);
+            if (W) s2.add(w[g].v);
         }
-        s.add(y);
-    }
-    for (; i < n; i += stride) {
-        const T r[1] = {bb == T(0) ? a * Xin[i] : fma(a, Xin[i], bb * Y[i])};
-        Y[i] = r[0];
-        s.add(r);
-    }
-    if (W) {
-        for (int64_t j = i0; j < n; j += stride) {
-            const T w[1] = {W[j]};
-            s2.add(w);
-        }
-    }
+    });
     lsqr_finish<T>(L, s.get(), s2.get(), W != nullptr, phase);
 }
 
@@ -435,11 +455,27 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_xw(const T *__restrict__ 
         if (threadIdx.x < 32 && L.st->estimate) lsqr_estimate<T>(L);
         return;
     }
-    for (int64_t i = (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const T w = W[i];
-        X[i] = fma(t1, w, X[i]);
-        W[i] = fma(ia, V[i], t2 * w);
-    }
+    lsqr_each<T>(n, aligned16(V, W, X), (int64_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x, stride,
+                 [&](auto vc, auto gc, int64_t i, int64_t gap) {
+        constexpr int N = decltype(vc)::value, G = decltype(gc)::value;
+        Pack<T, N> w[G], x[G], v[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            w[g] = ldp<T, N>(W + i + g * gap);
+            x[g] = ldp<T, N>(X + i + g * gap);
+            v[g] = ldp<T, N>(V + i + g * gap);
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                x[g].v[k] = fma(t1, w[g].v[k], x[g].v[k]);
+                w[g].v[k] = fma(ia, v[g].v[k], t2 * w[g].v[k]);
+            }
+            stp<T, N>(X + i + g * gap, x[g]);
+            stp<T, N>(W + i + g * gap, w[g]);
+        }
+    });
 }
 
 }  // namespace

@@ -80,9 +80,8 @@ inline void launch_fwd_axis0_t(const AxisPass &p, cudaStream_t s) {
         const int64_t z = want_y / grid.y;
         grid.z = gdim(z < p.nch + 1 ? z : p.nch + 1, kMaxGridYZ);
     }
-    launch(k_fwd_axis0<D, TX, T, MODE>, grid, kThreads, 0, s,
-           p.idx, (const T *)p.B, p.ns, p.d, (const TX *)p.X, (const T *)p.w, p.n, p.Q, p.nch,
-        (T *)p.Y);
+    launch(k_fwd_axis0<D, TX, T, MODE>, grid, kThreads, 0, s, p.idx, (const T *)p.B, p.ns, p.d, (const TX *)p.X,
+           (const T *)p.w, p.n, p.Q, p.nch, (T *)p.Y);
 }
 
 template <typename T, typename TX, int MODE>
@@ -112,8 +111,8 @@ inline void launch_fwd0_warp(const AxisPass &p, cudaStream_t s) {
     SC = SC < 32 ? 32 : SC;
     const int64_t tasks = groups * ((p.ns + SC - 1) / SC);
     const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    launch(k_fwd0_warp<D, T>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s,
-           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.n, Qy, SC, (T *)p.Y);
+    launch(k_fwd0_warp<D, T>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s, p.idx, (const T *)p.B, p.ns, p.d,
+           (const T *)p.X, p.n, Qy, SC, (T *)p.Y);
 }
 
 template <typename T, typename TX>
@@ -149,9 +148,8 @@ inline void launch_fwd_axis_t(const AxisPass &p, cudaStream_t s) {
         const int64_t jb = c0 * kChunk;
         const int64_t jcount = (p.ns - jb < cn * kChunk) ? p.ns - jb : cn * kChunk;
         dim3 grid(gx, (unsigned)cn, gdim(p.Q, kMaxGridYZ));
-        launch(k_fwd_axis<D, T, VEC, FINAL, ST>, grid, kThreads, 0, s,
-           p.idx + jb, (const T *)p.B + jb, p.ns, jcount, p.d, (const T *)p.X, p.M, p.n, p.Q,
-            (T *)p.Y + p.M * jb);
+        launch(k_fwd_axis<D, T, VEC, FINAL, ST>, grid, kThreads, 0, s, p.idx + jb, (const T *)p.B + jb, p.ns,
+               jcount, p.d, (const T *)p.X, p.M, p.n, p.Q, (T *)p.Y + p.M * jb);
     }
 }
 
@@ -180,13 +178,13 @@ inline void launch_fwd_warp(const AxisPass &p, cudaStream_t s) {
     const int64_t total = p.M * p.ns * Q;
     if (NC == 0 && total <= kThreadFwdValues) {
         launch(k_fwd_thread<D, T>, (unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s,
-           p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
-            (T *)p.Y);
+               p.idx, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n,
+               (uint32_t)total, (T *)p.Y);
         return;
     }
-    launch(k_fwd_warp<D, T, ST, FINAL, NC>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s,
-           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, Q, NC > 0 ? (int)p.nch : 0, gxw,
-        (p.ns + rows - 1) / rows, rows, (T *)p.Y);
+    launch(k_fwd_warp<D, T, ST, FINAL, NC>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s, p.idx, (const T *)p.B,
+           p.ns, p.d, (const T *)p.X, p.M, p.n, Q, NC > 0 ? (int)p.nch : 0, gxw, (p.ns + rows - 1) / rows, rows,
+           (T *)p.Y);
 }
 
 template <typename T, int D, int VEC, bool ST>
@@ -227,8 +225,8 @@ template <typename T>
 inline void launch_fwd_axis(const AxisPass &p, cudaStream_t s) {
     if (p.mode == kRational && (p.nch + 1 > 4 || p.d > 3)) {
         dim3 grid((unsigned)((p.M + kThreads - 1) / kThreads), gdim(p.ns, kMaxGridYZ));
-        launch(k_fwd_axis_rational_generic<T>, grid, kThreads, 0, s,
-           p.idx, (const T *)p.B, p.ns, p.d, (const T *)p.X, p.M, p.n, p.nch, (T *)p.Y);
+        launch(k_fwd_axis_rational_generic<T>, grid, kThreads, 0, s, p.idx, (const T *)p.B, p.ns, p.d,
+               (const T *)p.X, p.M, p.n, p.nch, (T *)p.Y);
         return;
     }
     switch (p.d) {
@@ -265,10 +263,8 @@ inline void launch_adj_axis_t(const AxisPass &p, cudaStream_t s) {
                              smem);
         attr_set = true;
     }
-    launch(k_adj_axis<D, T, VEC, ST>, grid, kThreads, smem, s,
-           p.idx, p.perm, p.lb, (const T *)p.B, p.ns,
-                                                     p.d, (const T *)p.X, p.M, p.n, p.Q, (int)CC,
-                                                     (T *)p.Y);
+    launch(k_adj_axis<D, T, VEC, ST>, grid, kThreads, smem, s, p.idx, p.perm, p.lb, (const T *)p.B, p.ns, p.d,
+           (const T *)p.X, p.M, p.n, p.Q, (int)CC, (T *)p.Y);
 }
 
 // One thread per output (sg_ring.cuh).
@@ -276,9 +272,9 @@ template <typename T, int D>
 inline void launch_adj_thread(const AxisPass &p, cudaStream_t s) {
     const int64_t total = p.M * p.n * p.Q;
     if (total == 0) return;
-    launch(k_adj_thread<D, T>, (unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s,
-           p.perm, p.lb, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
-        (T *)p.Y);
+    launch(k_adj_thread<D, T>, (unsigned)((total + kThreadBlock - 1) / kThreadBlock), kThreadBlock, 0, s, p.perm,
+           p.lb, (const T *)p.B, (uint32_t)p.ns, (const T *)p.X, (uint32_t)p.M, (uint32_t)p.n, (uint32_t)total,
+           (T *)p.Y);
 }
 
 // Cotangent values up to which a pass over an axis k >= 1 runs one thread per output: it
@@ -321,8 +317,8 @@ inline void launch_adj_ring(const AxisPass &p, cudaStream_t s) {
     if (per_chunk == 0) return;
     const int64_t CC = adj_chunk(p, per_chunk, kRingLat, kRingPer);
     const int64_t chunks = (p.n + CC - 1) / CC;
-    launch(k_adj_ring<D, T>, (unsigned)(per_chunk * chunks), 32, (ring_smem<D, T>()), s,
-           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, (T *)p.Y);
+    launch(k_adj_ring<D, T>, (unsigned)(per_chunk * chunks), 32, (ring_smem<D, T>()), s, p.perm, p.lb,
+           (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, (T *)p.Y);
 }
 template <typename T, int D>
 inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
@@ -332,8 +328,8 @@ inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
     const int64_t CC = sizeof(T) == 4 ? adj_chunk(p, per_chunk, kColsLat, kColsPer)
                                       : adj_chunk(p, per_chunk, 64 * D + kColsLat, 64 * D);
     const int64_t chunks = (p.n + CC - 1) / CC, units = per_chunk * chunks;
-    launch(k_adj_cols<D, T, 8>, (unsigned)((units + kColsWarps - 1) / kColsWarps), 32 * kColsWarps, 0, s,
-           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
+    launch(k_adj_cols<D, T, 8>, (unsigned)((units + kColsWarps - 1) / kColsWarps), 32 * kColsWarps, 0, s, p.perm,
+           p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
 }
 
 template <typename T, int D>
@@ -384,10 +380,8 @@ inline void launch_adj_axis0_t(const AxisPass &p, cudaStream_t s) {
                              (int)adj_axis0_smem_bytes<D, T>(32));
         attr_set = true;
     }
-    launch(k_adj_axis0<D, T>, grid, kAdj0Threads, smem, s,
-           p.idx, p.perm, p.lb, (const T *)p.B,
-                                                       p.ns, p.d, (const T *)p.X, p.n, p.Q, QT,
-                                                       (T *)p.Y);
+    launch(k_adj_axis0<D, T>, grid, kAdj0Threads, smem, s, p.idx, p.perm, p.lb, (const T *)p.B, p.ns, p.d,
+           (const T *)p.X, p.n, p.Q, QT, (T *)p.Y);
 }
 
 // degrees <= 5: shared-memory tiles of 32 columns x kA0Cp control points, or one thread
@@ -403,9 +397,8 @@ inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
         return;
     }
     const int smem = a0_smem<D, T>();
-    launch(k_adj0_tile<D, T>, (unsigned)tiles, 32 * kA0Warps, smem, s,
-           p.perm, p.lb, (const T *)p.B, p.ns, (const T *)p.X,
-                                                                   p.n, p.Q, groups, (T *)p.Y);
+    launch(k_adj0_tile<D, T>, (unsigned)tiles, 32 * kA0Warps, smem, s, p.perm, p.lb, (const T *)p.B, p.ns,
+           (const T *)p.X, p.n, p.Q, groups, (T *)p.Y);
 }
 
 // Higher degrees (runtime-degree path) run as CTA tiles.

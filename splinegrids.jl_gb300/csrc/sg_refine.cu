@@ -532,10 +532,8 @@ static void launch_mult_nd(const MultArgs &a, const void *X, void *Y, int64_t N,
     }
     const unsigned blocks = (unsigned)((N + kMultThreads - 1) / kMultThreads);
     const bool small = N <= 0xffffffffLL;
-    if (ADJ) launch(k_mult_adjoint_nd<T, ND>, blocks, kMultThreads, 0, s,
-           p, (const T *)X, (T *)Y, N, small);
-    else launch(k_mult_nd<T, ND>, blocks, kMultThreads, 0, s,
-           p, a, (const T *)X, (T *)Y, N, small);
+    if (ADJ) launch(k_mult_adjoint_nd<T, ND>, blocks, kMultThreads, 0, s, p, (const T *)X, (T *)Y, N, small);
+    else launch(k_mult_nd<T, ND>, blocks, kMultThreads, 0, s, p, a, (const T *)X, (T *)Y, N, small);
 }
 
 template <typename T, bool ADJ>
@@ -544,10 +542,8 @@ static void launch_mult(const MultArgs &a, const void *X, void *Y, int64_t N, cu
     if (a.ndims == 2 && one_launch) launch_mult_nd<T, 2, ADJ>(a, X, Y, N, s);
     else if (a.ndims == 3 && one_launch) launch_mult_nd<T, 3, ADJ>(a, X, Y, N, s);
     else if (a.ndims == 4 && one_launch) launch_mult_nd<T, 4, ADJ>(a, X, Y, N, s);
-    else if (ADJ) launch(k_mult_adjoint<T>, grid_for(N, 256), 256, 0, s,
-           a, (const T *)X, (T *)Y, N);
-    else launch(k_mult<T>, grid_for(N, 256), 256, 0, s,
-           a, (const T *)X, (T *)Y, N);
+    else if (ADJ) launch(k_mult_adjoint<T>, grid_for(N, 256), 256, 0, s, a, (const T *)X, (T *)Y, N);
+    else launch(k_mult<T>, grid_for(N, 256), 256, 0, s, a, (const T *)X, (T *)Y, N);
 }
 
 extern "C" int sg_mult(int32_t dtype, int32_t ndims, const int64_t *size_Y,
@@ -617,15 +613,11 @@ extern "C" int sg_local_refinement(int32_t dtype, int32_t nin, int32_t nout,
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned g = (unsigned)((n_refined + 255) / 256);
     if (dtype == SG_F32)
-        launch(k_local_refinement<float>, g, 256, 0, s,
-           r, nout, n_refined, refinement_indices,
-                                                    (const float *)refinement_values,
-                                                    (float *)control_points, ncp);
+        launch(k_local_refinement<float>, g, 256, 0, s, r, nout, n_refined, refinement_indices,
+               (const float *)refinement_values, (float *)control_points, ncp);
     else
-        launch(k_local_refinement<double>, g, 256, 0, s,
-           r, nout, n_refined, refinement_indices,
-                                                     (const double *)refinement_values,
-                                                     (double *)control_points, ncp);
+        launch(k_local_refinement<double>, g, 256, 0, s, r, nout, n_refined, refinement_indices,
+               (const double *)refinement_values, (double *)control_points, ncp);
     return cuda_check(cudaGetLastError(), "k_local_refinement launch");
 }
 
@@ -643,14 +635,10 @@ extern "C" int sg_local_refinement_adjoint(int32_t dtype, int32_t nin, int32_t n
     cudaStream_t s = (cudaStream_t)stream;
     const unsigned g = (unsigned)((n_refined + 255) / 256);
     if (dtype == SG_F32)
-        launch(k_local_refinement_adjoint<float>, g, 256, 0, s,
-           r, nout, n_refined, refinement_indices,
-                                                            (float *)refinement_values,
-                                                            (float *)control_points, ncp);
+        launch(k_local_refinement_adjoint<float>, g, 256, 0, s, r, nout, n_refined, refinement_indices,
+               (float *)refinement_values, (float *)control_points, ncp);
     else
-        launch(k_local_refinement_adjoint<double>, g, 256, 0, s,
-           r, nout, n_refined, refinement_indices,
-                                                             (double *)refinement_values,
-                                                             (double *)control_points, ncp);
+        launch(k_local_refinement_adjoint<double>, g, 256, 0, s, r, nout, n_refined, refinement_indices,
+               (double *)refinement_values, (double *)control_points, ncp);
     return cuda_check(cudaGetLastError(), "k_local_refinement_adjoint launch");
 }

@@ -363,7 +363,9 @@ k_adj_cols(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
 // shared memory in segments (cp.async, coalesced along the samples; the CTAs of an SM
 // overlap one another's waits); lane = column (odd row stride: no bank conflicts), warp =
 // control point.  Results leave through shared memory, eight consecutive control points
-// of a column at a time: a warp's own 32 results lie n apart.  SG_A0_FIGURES
+// of a column at a time: a warp's own 32 results lie n apart.  Bound by the chain of shared
+// loads and FMAs of each control point.  ((1999, 131) x 3: warp tasks with transpose tiles 18 us,
+// these tiles 8.)
 // ---------------------------------------------------------------------------------
 constexpr int kA0Warps = 8;
 constexpr int kA0Cp = 8;                        // control points per CTA, one per warp

@@ -396,9 +396,15 @@ inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
         launch_adj_thread<T, D>(p, s);
         return;
     }
-    const int smem = a0_smem<D, T>();
-    launch(k_adj0_tile<D, T>, (unsigned)tiles, 32 * kA0Warps, smem, s, p.perm, p.lb, (const T *)p.B, p.ns,
-           (const T *)p.X, p.n, p.Q, groups, (T *)p.Y);
+    if constexpr (sizeof(T) == 4) {
+        if (!p.perm && p.ns % 4 == 0 && (uintptr_t)p.X % 16 == 0 && (uintptr_t)p.B % 16 == 0) {
+            launch(k_adj0_tile<D, T, true>, (unsigned)tiles, 32 * kA0Warps, (a0_smem<D, T, true>()), s, p.perm, p.lb,
+                   (const T *)p.B, p.ns, (const T *)p.X, p.n, p.Q, groups, (T *)p.Y);
+            return;
+        }
+    }
+    launch(k_adj0_tile<D, T, false>, (unsigned)tiles, 32 * kA0Warps, (a0_smem<D, T, false>()), s, p.perm, p.lb,
+           (const T *)p.B, p.ns, (const T *)p.X, p.n, p.Q, groups, (T *)p.Y);
 }
 
 // Higher degrees (runtime-degree path) run as CTA tiles.

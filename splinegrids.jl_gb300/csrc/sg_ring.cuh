@@ -363,79 +363,112 @@ k_adj_cols(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
 // shared memory in segments (cp.async, coalesced along the samples; the CTAs of an SM
 // overlap one another's waits); lane = column (odd row stride: no bank conflicts), warp =
 // control point.  Results leave through shared memory, eight consecutive control points
-// of a column at a time: a warp's own 32 results lie n apart.  Bound by the chain of shared
-// loads and FMAs of each control point.  ((1999, 131) x 3: warp tasks with transpose tiles 18 us,
-// these tiles 8.)
+// of a column at a time: a warp's own 32 results lie n apart.  ((1999, 131) x 3: warp
+// tasks with transpose tiles 18 us, these tiles 8.)
 // ---------------------------------------------------------------------------------
 constexpr int kA0Warps = 8;
-constexpr int kA0Cp = 8;                        // control points per CTA, one per warp
+constexpr int kA0Cp = kA0Warps;  // control points per CTA, one per warp
 template <typename T>
 __host__ __device__ constexpr int a0_seg() { return sizeof(T) == 4 ? 192 : 96; }  // samples per segment
-template <int D, typename T>
+// Row stride of the staged columns: odd for single values; 4 past a multiple of 32 banks for
+// 16-byte loads (eight lanes of a load then cover all banks).
+template <typename T, bool V4>
+__host__ __device__ constexpr int a0_stride() { return a0_seg<T>() + (V4 ? 4 : 1); }
+template <int D, typename T, bool V4>
 __host__ __device__ constexpr int a0_smem() {
-    return (int)(align16(32 * (a0_seg<T>() + 1) * (int64_t)sizeof(T)) + align16(a0_seg<T>() * D * (int64_t)sizeof(T)));
+    return (int)(align16(32 * a0_stride<T, V4>() * (int64_t)sizeof(T)) + align16(a0_seg<T>() * D * (int64_t)sizeof(T)));
 }
 
-template <int D, typename T>
+// V4 (Float32, sorted samples, ns a multiple of 4, X and B on 16-byte boundaries): samples are
+// copied and read four at a time, from the multiple of 4 at or before the first.  The tiles are
+// bound by the issue of their instructions: 256 control points, 4096 samples, 768 columns, degree
+// 3: 1063 a warp and 12.3 us with single values, 767 and 9.3 us so.
+template <int D, typename T, bool V4>
 __global__ void __launch_bounds__(32 * kA0Warps)
 k_adj0_tile(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns,
             const T *__restrict__ X, int64_t n, int64_t Q, int64_t groups, T *__restrict__ Y) {
+    static_assert(!V4 || sizeof(T) == 4, "16-byte groups of four");
     constexpr int d = D - 1;
-    constexpr int SEG = a0_seg<T>();
-    constexpr int PER = kA0Cp / kA0Warps;
+    constexpr int SEG = a0_seg<T>(), STR = a0_stride<T, V4>();
     extern __shared__ __align__(16) unsigned char smem[];
-    T *xs = reinterpret_cast<T *>(smem);  // [32][SEG + 1]
-    T *bs = reinterpret_cast<T *>(smem + align16(32 * (SEG + 1) * (int64_t)sizeof(T)));  // [D][SEG]
+    T *xs = reinterpret_cast<T *>(smem);  // [32][STR]
+    T *bs = reinterpret_cast<T *>(smem + align16(32 * STR * (int64_t)sizeof(T)));  // [D][SEG]
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t tile = blockIdx.x + grid_start();
     const int64_t q0 = (tile % groups) * 32;
     const int c0 = (int)(tile / groups) * kA0Cp;
     const int c1 = c0 + kA0Cp < n ? c0 + kA0Cp : (int)n;
-    const int s_lo = lb[c0], s_hi = lb[c1 + d];
-    T acc[PER];
+    const int c = c0 + w;  // this warp's control point
+    const int s_hi = lb[c1 + d], s_lo = V4 ? lb[c0] & ~3 : lb[c0];
+    int bd[D + 1];  // support starts c - d .. c, one span each: span i holds the samples whose
+                    // basis value i belongs to c, [bd[d - i], bd[d - i + 1])
 #pragma unroll
-    for (int p = 0; p < PER; ++p) acc[p] = T(0);
+    for (int i = 0; i <= D; ++i) bd[i] = c < c1 ? lb[c + i] : 0;
+    T acc = T(0);
     for (int sb = s_lo; sb < s_hi; sb += SEG) {
         const int nb = s_hi - sb < SEG ? s_hi - sb : SEG;
         if (sb != s_lo) __syncthreads();
         for (int k = w; k < 32; k += kA0Warps) {
             if (q0 + k < Q) {
                 const T *xc = X + ns * (q0 + k);
-                T *xd = xs + k * (SEG + 1);
-                for (int t = lane; t < nb; t += 32)
-                    cp_async<(int)sizeof(T)>(xd + t, xc + (perm ? perm[sb + t] : sb + t));
+                T *xd = xs + k * STR;
+                if constexpr (V4) {  // whole groups: the last may end past s_hi, not past ns
+                    for (int t = 4 * lane; t < nb; t += 128) cp_async<16>(xd + t, xc + sb + t);
+                } else {
+                    for (int t = lane; t < nb; t += 32)
+                        cp_async<(int)sizeof(T)>(xd + t, xc + (perm ? perm[sb + t] : sb + t));
+                }
             }
         }
-        for (int t = threadIdx.x; t < nb; t += 32 * kA0Warps) {
-            const int64_t j = perm ? perm[sb + t] : sb + t;
+        if constexpr (V4) {
+            for (int t = 4 * lane; w < D && t < nb; t += 128) cp_async<16>(bs + w * SEG + t, B + ns * w + sb + t);
+        } else {
+            for (int t = threadIdx.x; t < nb; t += 32 * kA0Warps) {
+                const int64_t j = perm ? perm[sb + t] : sb + t;
 #pragma unroll
-            for (int i = 0; i < D; ++i) cp_async<(int)sizeof(T)>(bs + i * SEG + t, B + j + ns * i);
+                for (int i = 0; i < D; ++i) cp_async<(int)sizeof(T)>(bs + i * SEG + t, B + j + ns * i);
+            }
         }
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
-        const T *xl = xs + lane * (SEG + 1) - sb;
+        const T *xl = xs + lane * STR - sb;
 #pragma unroll
-        for (int p = 0; p < PER; ++p) {
-            const int c = c0 + w * PER + p;
-            if (c >= c1) break;
-            // support starts c - d .. c, one span each: span i holds the samples whose
-            // basis value i belongs to c
-#pragma unroll
-            for (int i = D - 1; i >= 0; --i) {
-                int a = lb[c - i + d], z = lb[c - i + d + 1];
-                a = a > sb ? a : sb;
-                z = z < sb + nb ? z : sb + nb;
-                const T *bi = bs + i * SEG - sb;
+        for (int i = D - 1; i >= 0; --i) {
+            const int a = bd[d - i] > sb ? bd[d - i] : sb;
+            const int z = bd[d - i + 1] < sb + nb ? bd[d - i + 1] : sb + nb;
+            const T *bi = bs + i * SEG - sb;
+            if constexpr (V4) {
+                int g = a & ~3;
+                auto part = [&]() {  // the samples of group g inside [a, z)
+                    const float4 x = *reinterpret_cast<const float4 *>(xl + g);
+                    const float4 v = *reinterpret_cast<const float4 *>(bi + g);
+                    if (g >= a) acc = ::fma(v.x, x.x, acc);  // (g < z)
+                    if (g + 1 >= a && g + 1 < z) acc = ::fma(v.y, x.y, acc);
+                    if (g + 2 >= a && g + 2 < z) acc = ::fma(v.z, x.z, acc);
+                    if (g + 3 < z) acc = ::fma(v.w, x.w, acc);  // (g + 3 >= a)
+                    g += 4;
+                };
+                if (a < z && g < a) part();
+#pragma unroll 4
+                for (; g + 4 <= z; g += 4) {
+                    const float4 x = *reinterpret_cast<const float4 *>(xl + g);
+                    const float4 v = *reinterpret_cast<const float4 *>(bi + g);
+                    acc = ::fma(v.x, x.x, acc);
+                    acc = ::fma(v.y, x.y, acc);
+                    acc = ::fma(v.z, x.z, acc);
+                    acc = ::fma(v.w, x.w, acc);
+                }
+                if (a < z && g < z) part();
+            } else {
 #pragma unroll 8
-                for (int s = a; s < z; ++s) acc[p] = ::fma(bi[s], xl[s], acc[p]);
+                for (int s = a; s < z; ++s) acc = ::fma(bi[s], xl[s], acc);
             }
         }
     }
     // out through shared memory: kA0Cp consecutive control points of a column per store group
     __syncthreads();
-#pragma unroll
-    for (int p = 0; p < PER; ++p) xs[lane * (kA0Cp + 1) + w * PER + p] = acc[p];
+    xs[lane * (kA0Cp + 1) + w] = acc;
     __syncthreads();
     for (int t = threadIdx.x; t < 32 * kA0Cp; t += 32 * kA0Warps) {
         const int k = t / kA0Cp, c = c0 + t % kA0Cp;

@@ -385,14 +385,25 @@ inline void launch_adj_axis0_t(const AxisPass &p, cudaStream_t s) {
 }
 
 // degrees <= 5: shared-memory tiles of 32 columns x kA0Cp control points, or one thread
-// per output when half of a tile's lanes would idle or the tiles leave most SMs idle
-// ((1999, 131) x 3: tiles 8 us against 18; (50, 10, 5) x 4: one thread per output 6 against 8)
+// per output when half of a tile's lanes would idle or the tiles leave most SMs idle, and
+// that is the shorter: with S samples a control point, a tile's warp issues some 3 S + 300
+// instructions (425 a cycle on the whole chip) and then waits 8 cycles a sample; a thread reads
+// its samples eight at a time from L2, 88 cycles a sample, or is bound by its instructions.
+// Measured on axis 0 of (100, 10) x (100, 50), S = 4: one thread per output 6.2 us for both
+// passes, tiles 6.6; (10, 10) x (200, 50), S = 60: 13.8 and 7.9; (5, 5) x (2749, 25), S = 1649: 330
+// and 43.6.
 constexpr int64_t kA0Tiles = 64;
+inline bool a0_thread_is_shorter(const AxisPass &p, int64_t groups) {
+    const double S = (double)p.ns * (p.d + 1) / (double)p.n;
+    const double tile = (double)p.n * groups * (3 * S + 300) / 425 + 8 * S + 3000;
+    const double instr = (double)p.n * p.Q * S * 10 / (32 * 425);
+    return (88 * S > instr ? 88 * S : instr) + 2200 <= tile;
+}
 template <typename T, int D>
 inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
     const int64_t groups = (p.Q + 31) / 32, tiles = groups * ((p.n + kA0Cp - 1) / kA0Cp);
     if (tiles == 0) return;
-    if ((p.Q < 16 || tiles < kA0Tiles) && p.n * p.Q <= INT32_MAX) {
+    if ((p.Q < 16 || tiles < kA0Tiles) && p.n * p.Q <= INT32_MAX && a0_thread_is_shorter(p, groups)) {
         launch_adj_thread<T, D>(p, s);
         return;
     }

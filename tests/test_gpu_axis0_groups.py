@@ -36,3 +36,32 @@ def test_axis0_tiles_have_the_fused_bits(sg, deg0, n0, ns0):
         got.append(gr)
     assert torch.isfinite(got[0]).sum() > 0.9 * got[0].numel()
     assert torch.equal(torch.nan_to_num(got[0], nan=1.5), torch.nan_to_num(got[1], nan=1.5))
+
+
+@pytest.mark.parametrize("dtype_name", ["f32", "f64"])
+@pytest.mark.parametrize("n0,ns0,n1,nout", [
+    (5, 1000, 4, 1),     # four columns, supports of 600 samples and more: a tile
+    (5, 1001, 5, 2),
+    (300, 600, 4, 1),    # supports of six: one thread per output
+    (900, 1500, 4, 1),
+    (40, 900, 4, 5),     # 20 columns of one tile
+])
+def test_few_columns_have_the_fused_bits(sg, n0, ns0, n1, nout, dtype_name):
+    import torch
+    dt = torch.float64 if dtype_name == "f64" else torch.float32
+    g = sg.SplineGrid((sg.SplineDimension(n0, 2, ns0, float_type=dt),
+                       sg.SplineDimension(n1, 1, 30, float_type=dt)), nout)
+    plan = g.plan(dt)
+    gen = torch.Generator(device="cuda").manual_seed(n0 + n1)
+    cot = sg.arrays.empty((ns0, 30, nout), dt)
+    cot.copy_(torch.randn((ns0, 30, nout), generator=gen, device="cuda", dtype=dt))
+    got = []
+    for strategy in ("fused", "separable"):
+        plan.set_strategy(strategy)
+        gr = sg.arrays.empty((n0, n1, nout), dt)
+        gr.fill_(float("nan"))
+        sg.evaluate_adjoint_(g, control_points=gr, eval=cot)
+        plan.check()
+        got.append(gr)
+    assert torch.isfinite(got[0]).all()
+    assert torch.equal(got[0], got[1])

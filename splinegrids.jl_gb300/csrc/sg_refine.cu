@@ -171,11 +171,10 @@ __global__ void k_mult_adjoint(MultArgs a, const T *__restrict__ Y, T *__restric
 // the unrolled one for the widest band of its warp (2 to 5 terms a dimension, factors in
 // registers, independent loads) or plain loops for wider ones: bound by the terms'
 // instructions, so one sum for all widths up to 5, 25 predicated terms a plane, took 2 to 4
-// times as long.  Terms and factors keep their order, so only the contraction of the last
-// product with the sum can change a bit.  Measured, us, general kernels / one sum for all /
-// now: (58, 58, 26) -> (114, 114, 50), bands of 2, Float32: mult! 46 / 22 / 11.7, mult_adjoint! 79
-// / 17 / 12.6; bands of 3: 122 / - / 14.7, 231 / 286 / 39.6; (257, 257) x 3 -> (512, 512) x 3, bands of
-// 3, Float64: 54 / 75 / 39.6, 72 / 114 / 67.5.
+// times as long.  Terms, factors and roundings are those of the general kernels.  Measured, us,
+// general kernels / one sum for all / now: (58, 58, 26) -> (114, 114, 50), bands of 2, Float32:
+// mult! 46 / 22 / 11.8, mult_adjoint! 79 / 17 / 12.6; bands of 3: 122 / - / 15, 231 / 286 / 39;
+// (257, 257) x 3 -> (512, 512) x 3, bands of 3, Float64: 54 / 75 / 43, 73 / 114 / 65.
 // ---------------------------------------------------------------------------------
 constexpr int kMultThreads = 128;
 
@@ -217,6 +216,10 @@ __device__ __forceinline__ void nd_decode(const int64_t (&size)[ND], int64_t lin
     }
 }
 
+// a + b, not contracted with the product b may be: the bits of the general function.
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
 // The sum of x at k_d < n[d], stride st[d] (0 fastest), times the factors f(d, k) of dimension d at
 // term k, over the first NR dimensions.  n[d] <= C: the factors sit in registers, the loads of a
 // k2 are independent.
@@ -251,27 +254,33 @@ __device__ __forceinline__ T nd_sum_c(const T *__restrict__ x, const int (&n)[ND
                     T t = v[k1][k0] * w[0][k0];
                     if constexpr (NR > 1) t = t * w[1][k1];
                     if constexpr (NR > 2) t = t * w2;
-                    acc += t;
+                    acc = add_rn(acc, t);
                 }
         if constexpr (NR > 2) x += st[2];
     }
     return acc;
 }
 
-// Bands of any width, all ND dimensions.
-template <typename T, int ND, typename F>
+// Bands of any width, the first NR dimensions.
+template <int NR, typename T, int ND, typename F>
 __device__ __forceinline__ T nd_sum_any(const T *__restrict__ X, const int (&n)[ND], const int64_t (&st)[ND], F f) {
     T acc = T(0);
-    const int n1 = n[1], n2 = ND > 2 ? n[ND > 2 ? 2 : 0] : 1, n3 = ND > 3 ? n[ND > 3 ? 3 : 0] : 1;
+    const int n1 = NR > 1 ? n[1] : 1, n2 = NR > 2 ? n[NR > 2 ? 2 : 0] : 1, n3 = NR > 3 ? n[NR > 3 ? 3 : 0] : 1;
     for (int k3 = 0; k3 < n3; ++k3) {
-        const T w3 = ND > 3 ? f(3, k3) : T(1);
+        const T w3 = NR > 3 ? f(3, k3) : T(1);
         for (int k2 = 0; k2 < n2; ++k2) {
-            const T w2 = ND > 2 ? f(2, k2) : T(1);
+            const T w2 = NR > 2 ? f(2, k2) : T(1);
             for (int k1 = 0; k1 < n1; ++k1) {
-                const T w1 = f(1, k1);
-                const T *x = X + k1 * st[1] + (ND > 2 ? k2 * st[ND > 2 ? 2 : 0] : 0) + (ND > 3 ? k3 * st[ND > 3 ? 3 : 0] : 0);
+                const T w1 = NR > 1 ? f(1, k1) : T(1);
+                const T *x = X + k1 * st[1] + (NR > 2 ? k2 * st[NR > 2 ? 2 : 0] : 0) + (NR > 3 ? k3 * st[NR > 3 ? 3 : 0] : 0);
 #pragma unroll 4
-                for (int k0 = 0; k0 < n[0]; ++k0) acc += x[k0] * f(0, k0) * w1 * w2 * w3;
+                for (int k0 = 0; k0 < n[0]; ++k0) {
+                    T t = x[k0] * f(0, k0);
+                    if constexpr (NR > 1) t = t * w1;
+                    if constexpr (NR > 2) t = t * w2;
+                    if constexpr (NR > 3) t = t * w3;
+                    acc = add_rn(acc, t);
+                }
             }
         }
     }
@@ -281,7 +290,8 @@ __device__ __forceinline__ T nd_sum_any(const T *__restrict__ X, const int (&n)[
 // The narrowest of the sums that holds every band of the warp's threads (the vote keeps the
 // warp in one of them): a term that a thread does not have costs it as much as one it has.
 // A row of a bisected dimension has degree / 2 + 1 columns at most, a column degree + 2 rows.
-// last: the last dimension is refined (Nout is not: no factors of one are multiplied).
+// last: the last dimension is refined (Nout is not: no factors of one are multiplied); that takes
+// the loops, for the unrolled sums of ND dimensions as well would cost the kernel registers.
 template <int NR, typename T, int ND, typename F>
 __device__ __forceinline__ T nd_sum_n(const T *__restrict__ x, const int (&n)[ND], const int64_t (&st)[ND], F f) {
     int widest = n[0];
@@ -292,7 +302,7 @@ __device__ __forceinline__ T nd_sum_n(const T *__restrict__ x, const int (&n)[ND
     if (cap <= 3) return nd_sum_c<3, NR>(x, n, st, f);
     if (cap <= 4) return nd_sum_c<4, NR>(x, n, st, f);
     if (cap <= 5) return nd_sum_c<5, NR>(x, n, st, f);
-    return nd_sum_any(x, n, st, f);
+    return nd_sum_any<NR>(x, n, st, f);
 }
 template <typename T, int ND, typename F>
 __device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)[ND], const int (&n)[ND],
@@ -301,12 +311,11 @@ __device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)
 #pragma unroll
     for (int d = 0; d < ND; ++d) x += lo[d] * st[d];
     if (!last) return nd_sum_n<ND - 1>(x, n, st, f);
-    if constexpr (ND < 4) return nd_sum_n<ND>(x, n, st, f);
-    else return nd_sum_any(x, n, st, f);
+    return nd_sum_any<ND>(x, n, st, f);
 }
 
 template <typename T, int ND>
-__global__ void __launch_bounds__(kMultThreads)
+__global__ void __launch_bounds__(kMultThreads, sizeof(T) == 4 ? 6 : 4)
 k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, int64_t NY, bool small) {
     const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NY) return;
@@ -344,7 +353,7 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
 }
 
 template <typename T, int ND>
-__global__ void __launch_bounds__(kMultThreads)
+__global__ void __launch_bounds__(kMultThreads, sizeof(T) == 4 ? 6 : 4)
 k_mult_adjoint_nd(MultNd<ND> p, const T *__restrict__ Y, T *__restrict__ B, int64_t NB, bool small) {
     const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NB) return;

@@ -128,14 +128,14 @@ int sg_grid_plan_enable_timing(sg_grid_plan *plan, int32_t enable);
 int sg_grid_plan_pass_times(sg_grid_plan *plan, float *ms, int32_t *n_passes);
 
 /* Status of the plan's earlier launches on `stream` (no counterpart in the reference,
- * whose kernels have no device-side waits).  The adjoint passes over axes k >= 1 wait
- * on shared-memory barriers for their bulk copies; each wait gives up after a bounded
+ * whose kernels have no device-side waits).  The fused adjoint waits
+ * on shared-memory barriers for its bulk copies; each wait gives up after a bounded
  * time and records SG_ERR_TIMEOUT in the plan's status word instead of hanging.
  * Synchronizes `stream`, returns that status and clears it. */
 int sg_grid_plan_check(sg_grid_plan *plan, sg_stream_t stream);
 
 /* Measured tuning of the adjoint: for every pass over an axis k >= 1 the plan times
- * candidate chunk sizes of the bulk-copy stream (8..64 control points per tile, three
+ * candidate chunk sizes (8..64 control points per unit, three
  * runs each, on `stream`, with the caller's cotangent eval_bar and gradient buffer
  * control_points_bar as scratch) and keeps the fastest for later sg_evaluate_adjoint
  * calls; chosen[k] (optional, SG_MAX_NIN entries) receives the choice (0: the built-in
@@ -157,7 +157,7 @@ int sg_grid_plan_untune(sg_grid_plan *plan);
  * being captured or another stream is still using the plan's intermediate.
  * sg_grid_plan_set_strategy(FUSED) on a grid outside it returns
  * SG_ERR_UNSUPPORTED; sg_grid_plan_paths reports the path each direction takes.  On
- * the fused path sg_grid_plan_tune times adjoint tile sizes instead of stream chunks
+ * the fused path sg_grid_plan_tune times adjoint tile sizes instead of chunks
  * (chosen[1] = axis-1 control points per tile). */
 #define SG_STRATEGY_AUTO 0
 #define SG_STRATEGY_SEPARABLE 1

@@ -86,9 +86,9 @@ struct sg_grid_plan {
     // below c (offsets of the fused adjoint's weight list); device, n_basis[0] + 1 values
     int32_t *off0 = nullptr;
     int64_t line_support = 0;  // Nin = 1 with long supports (adj_line_*): the longest; else 0
-    // device status word: SG_ERR_TIMEOUT when a bounded wait of a streaming pass gave up
+    // device status word: SG_ERR_TIMEOUT when a bounded wait gave up
     int *status = nullptr;
-    // adjoint stream chunk size per axis chosen by sg_grid_plan_tune (0: heuristic)
+    // adjoint chunk size per axis chosen by sg_grid_plan_tune (0: heuristic)
     int32_t tuned_cc[SG_MAX_NIN] = {};
     // Nin = 2: the fused single-launch path (sg_fused2d.cuh) when the grid fits it
     int32_t strategy = SG_STRATEGY_AUTO;
@@ -447,7 +447,6 @@ static AxisPass axis_pass(const sg_grid_desc &d, const sg_grid_plan *p, int k,
     a.idx = d.sample_indices[k];
     a.perm = p->perm[k];
     a.lb = p->lb[k];
-    a.status = p->status;
     a.ns = d.n_samples[k];
     a.d = d.degree[k];
     a.n = d.n_basis[k];
@@ -768,7 +767,7 @@ extern "C" int sg_evaluate_adjoint(sg_grid_plan *p, const int32_t *derivative_or
     return rc;
 }
 
-// Measured choice of the adjoint stream's chunk size per axis k >= 1: each candidate
+// Measured choice of the adjoint's chunk size per axis k >= 1: each candidate
 // runs the pass three times on the caller's arrays (events on `stream`), the fastest
 // median wins.  The results do not depend on the chunk size (every control point sums
 // its samples in the same order), only the time does.

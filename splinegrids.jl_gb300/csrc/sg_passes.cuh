@@ -28,7 +28,6 @@ struct AxisPass {
     int mode = kPlain;
     bool final_pass = false;        // writes eval
     int x_dtype = SG_F32;           // element type of X on the axis-0 forward pass
-    int *status = nullptr;          // device status word of bounded waits
     int cc = 0;                     // adjoint: control points per chunk (0: heuristic)
     int64_t support = 0;            // Nin = 1 adjoint: samples in the longest support (adj_line_*)
 };

@@ -1,7 +1,7 @@
 // sg_stream.cuh -- the adjoint pass over an axis k >= 1 as a warp-specialized stream:
 // one producer warp moves whole row segments into a shared-memory ring with bulk
 // copies (cp.async.bulk) and stages each stage's basis rows beside them; eight
-// consumer warps sum them.
+// consumer warps sum them.  The batch's pass queue (sg_batch.cu) runs it.
 //
 // The pass reads its input X[M, ns, Q] (for the first adjoint pass: the cotangent on
 // eval, the largest array of the adjoint) exactly once and spends d+1 FMAs per value,

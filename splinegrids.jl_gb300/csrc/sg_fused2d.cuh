@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "sg_contract.cuh"
+#include "sg_divide.h"
 #include "sg_mbar.cuh"
 
 namespace sg {
@@ -47,6 +48,7 @@ constexpr int kF2PhaseBPerStage = 1;  // adjoint: pending phase-B items a thread
 constexpr int kF2BarBytes = ((2 * kF2NS * 8 + 15) / 16) * 16;  // full + empty mbarriers
 constexpr int kF2MaxG = 32;        // adjoint: channels per tile at most (one bulk copy each)
 constexpr int kF2Cps = 512;        // adjoint: axis-0 control points of a tile whose supports are staged
+static_assert(kF2Cps * kF2MaxG <= 65536, "work items divided by small_quotient");
 
 // Adjoint tiles: (sample, channel) pairs per tile; four pairs per consumer thread for
 // Float32 (two register pairs), two for Float64.
@@ -615,11 +617,10 @@ __device__ __forceinline__ bool f2_adjoint_tile(const F2Grid &g, const F2Tile &t
     // two outputs share every weight load and run as one packed FMA chain (one output
     // when pb_nc is odd and the pair is the last).
     int pb_col0 = 0, pb_nc = 0, pb_sh = 0, pb_o = 0, pb_n = 0;
-    // r / K0 for r < K0 G: exact by a 32-bit reciprocal while K0 and K0 G are small
-    const uint32_t k0_inv = (uint32_t)((0x100000000ull + K0 - 1) / (uint32_t)K0);
+    const uint32_t k0_inv = small_reciprocal((uint32_t)K0);  // staged: K0 <= kF2Cps, items < 32 K0
     auto b_item = [&](int o) {
         const int hp = o & pb_sh, r2 = o >> pb_sh;
-        const int cl = G == 1 ? 0 : (c0_staged ? (int)__umulhi((uint32_t)r2, k0_inv) : r2 / K0);
+        const int cl = G == 1 ? 0 : (c0_staged ? (int)small_quotient((uint32_t)r2, k0_inv) : r2 / K0);
         const int ci = r2 - cl * K0, c0 = C0a + ci;
         int sb, wb, m;
         if (c0_staged) {

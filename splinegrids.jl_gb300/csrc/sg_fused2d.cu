@@ -15,13 +15,13 @@ static int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 template <typename T, typename TX>
 __global__ void __launch_bounds__(kF2Lanes * kF2FwdWarps, 3)
 k_f2_fwd_grid(F2Grid g, F2Tiling tiling) {
-    grid_start();
+    const uint32_t block = blockIdx.x + grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ F2Grid s_g;
     if (threadIdx.x == 0) s_g = g;
     __syncthreads();
     const int w = threadIdx.x / kF2Lanes;
-    const int64_t task = (int64_t)blockIdx.x * kF2FwdWarps + w;
+    const int64_t task = (int64_t)block * kF2FwdWarps + w;
     if (task >= tiling.count()) return;
     const F2Tile tl = tiling.tile(task, 0, g.nch, g.ns0, g.ns1);
     f2_run_forward<T, TX>(s_g, tl, smem + w * f2_fwd_warp_smem<T>());
@@ -31,9 +31,12 @@ k_f2_fwd_grid(F2Grid g, F2Tiling tiling) {
 template <typename T, typename TX>
 __global__ void __launch_bounds__(kF2TileWarps * 32, sizeof(T) == 4 ? 5 : 4)
 k_f2_fwdt_grid(F2Grid g, F2Tiling tiling) {
-    grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
-    const F2Tile t = tiling.tile((int64_t)blockIdx.x, 2, g.nch, g.ns0, g.ns1);
+    F2Tile t = tiling.tile((int64_t)blockIdx.x, 2, g.nch, g.ns0, g.ns1);  // (its divisions, before the wait)
+    const uint32_t zero = grid_start();  // every address follows from the tile's corner
+    t.a_lo += zero;
+    t.b_lo += zero;
+    t.c_lo += zero;
     f2_run_forward_tile<T, TX>(g, t, smem);
 }
 
@@ -53,7 +56,6 @@ k_f2_fwdt_batch(const F2Grid *__restrict__ grids, const F2Tile *__restrict__ til
 template <typename T>
 __global__ void __launch_bounds__(kF2AdjThreads, 2)
 k_f2_adj_grid(F2Grid g, F2Tiling tiling, int *status) {
-    grid_start();
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ F2Grid s_g;
     __shared__ F2Tile s_t;
@@ -61,6 +63,12 @@ k_f2_adj_grid(F2Grid g, F2Tiling tiling, int *status) {
         s_g = g;
         s_t = tiling.tile((int64_t)blockIdx.x, 1, g.nch, g.n0, g.n1);
         f2_adj_init<T>(smem);
+    }
+    const uint32_t zero = grid_start();
+    if (threadIdx.x == 0) {  // as above; the tile is read behind the barrier
+        s_t.a_lo += zero;
+        s_t.b_lo += zero;
+        s_t.c_lo += zero;
     }
     __syncthreads();
     uint32_t gstage = 0;

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_start(const T *__restrict
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_axpby(const T *__restrict__ Xin, T *__restrict__ Y, int64_t n,
                                                 const T *__restrict__ W, int phase, LsqrShared L) {
-    grid_start(Xin, W);
+    grid_start(Xin, Y, W);
     const LsqrState *st = L.st;
     if (st->done) {  // the solve has stopped: leave every vector as it is
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -447,7 +447,7 @@ __device__ void lsqr_estimate(const LsqrShared &L) {
 template <typename T>
 __global__ void __launch_bounds__(kLsqrThreads) k_lsqr_xw(const T *__restrict__ V, T *__restrict__ W, T *__restrict__ X,
                                              int64_t n, LsqrShared L) {
-    grid_start(V);
+    grid_start(V, W, X);
     if (*L.skip_xw) return;
     const T t1 = (T)L.st->t1, t2 = (T)L.st->t2, ia = (T)L.st->inv_alpha;
     const int64_t stride = (int64_t)(gridDim.x - 1) * blockDim.x;

@@ -446,8 +446,7 @@ __device__ __forceinline__ bool ref_linear(const RefIdx &r, const int32_t *ridx,
 template <typename T>
 __global__ void k_local_refinement(RefIdx r, int nout, int64_t n_ref, const int32_t *ridx,
                                    const T *vals, T *cp, int64_t ncp) {
-    grid_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x + grid_start();
     if (i >= n_ref) return;
     int64_t lin;
     if (!ref_linear(r, ridx, n_ref, i, lin)) { g_bad_refinement_index = 1; return; }
@@ -458,8 +457,7 @@ __global__ void k_local_refinement(RefIdx r, int nout, int64_t n_ref, const int3
 template <typename T>
 __global__ void k_local_refinement_adjoint(RefIdx r, int nout, int64_t n_ref,
                                            const int32_t *ridx, T *vals, T *cp, int64_t ncp) {
-    grid_start();
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x + grid_start();
     if (i >= n_ref) return;
     int64_t lin;
     if (!ref_linear(r, ridx, n_ref, i, lin)) { g_bad_refinement_index = 1; return; }

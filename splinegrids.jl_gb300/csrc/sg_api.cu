@@ -840,6 +840,8 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
         cudaEventDestroy(e1);
         return rc;
     }
+    ScratchLease lease(p, s, false);  // another stream's adjoint may be reading the intermediate
+    if (!rc) rc = lease.rc;
     const void *X = eval_bar;
     int buf = 0;
     static const int kCand[] = {8, 12, 16, 24, 32, 48, 64};
@@ -883,6 +885,8 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
                           : (k > 0 ? adj_axis_f32(a, s) : adj_axis0_f32(a, s));
         X = a.Y;
     }
+    const int rc2 = lease.end();
+    if (!rc) rc = rc2;
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (!rc) rc = cuda_check(cudaStreamSynchronize(s), "tune: sync");

@@ -519,7 +519,14 @@ struct ScratchLease {
         lock = std::unique_lock<std::mutex>(p->scratch_mutex);
         if (p->scratch_used && id != p->scratch_stream) {
             if (may_fail) {
+                // (a query is among the calls that a capture on another thread forbids this one,
+                // and is ended by; the event is never recorded in a capture, so nothing conflicts)
+                cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+                rc = cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "plan: capture mode");
+                if (rc) return;
                 const cudaError_t e = cudaEventQuery(p->scratch_done);
+                rc = cuda_check(cudaThreadExchangeStreamCaptureMode(&mode), "plan: capture mode");
+                if (rc) return;
                 if (e == cudaErrorNotReady) {
                     (void)cudaGetLastError();  // not an error
                     return;

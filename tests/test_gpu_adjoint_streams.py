@@ -45,3 +45,50 @@ def test_tuning_waits_for_another_streams_adjoints(sg):
     torch.cuda.synchronize()
     assert torch.equal(queued[0], want)
     g.plan(torch.float32).untune()
+
+
+@pytest.mark.parametrize("busy", [False, True])
+def test_another_threads_capture_survives_the_adjoint(sg, busy):
+    """An adjoint on a second stream asks whether the first one's is done; asking must neither fail
+    nor end a capture (torch's default, global mode) that another thread has under way."""
+    import threading
+
+    import torch
+    g, cot, want = _large(sg)
+    got = sg.arrays.zeros(N + (NOUT,), torch.float32)
+    first = sg.arrays.zeros(N + (NOUT,), torch.float32)
+    a, b, s = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()
+    x = torch.zeros(1000, device="cuda")
+    with torch.cuda.stream(b):
+        x.add_(0)  # the streams exist before the capture
+    torch.cuda.synchronize()
+    errors = []
+
+    def on_b():
+        try:
+            with torch.cuda.stream(b):
+                sg.evaluate_adjoint_(g, eval=cot, control_points=got)
+        except Exception as e:  # reported by the main thread
+            errors.append(e)
+
+    with torch.cuda.stream(a):
+        if busy:
+            torch.cuda._sleep(20_000_000)
+        sg.evaluate_adjoint_(g, eval=cot, control_points=first)
+    if not busy:
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        graph.capture_begin(capture_error_mode="global")
+        x.add_(1)
+        t = threading.Thread(target=on_b)
+        t.start()
+        t.join()
+        x.add_(1)
+        graph.capture_end()
+    assert not errors, errors
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and torch.equal(first, want)
+    assert float(x[0]) == 2.0 and float(x[-1]) == 2.0

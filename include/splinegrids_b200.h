@@ -135,11 +135,11 @@ int sg_grid_plan_pass_times(sg_grid_plan *plan, float *ms, int32_t *n_passes);
 int sg_grid_plan_check(sg_grid_plan *plan, sg_stream_t stream);
 
 /* Measured tuning of the adjoint: for every pass over an axis k >= 1 the plan times
- * candidate chunk sizes (8..64 control points per unit, three
- * runs each, on `stream`, with the caller's cotangent eval_bar and gradient buffer
+ * the chunk size of the built-in heuristic and fixed ones (8..64 control points per unit;
+ * three runs each, on `stream`, with the caller's cotangent eval_bar and gradient buffer
  * control_points_bar as scratch) and keeps the fastest for later sg_evaluate_adjoint
  * calls; chosen[k] (optional, SG_MAX_NIN entries) receives the choice (0: the built-in
- * heuristic, e.g. for axis 0).  Results are bitwise the same for every choice.
+ * heuristic, always for axis 0).  Results are bitwise the same for every choice.
  * Synchronizes `stream`.  sg_grid_plan_untune returns to the heuristic. */
 int sg_grid_plan_tune(sg_grid_plan *plan, const int32_t *derivative_order, const void *eval_bar,
                       void *control_points_bar, sg_stream_t stream, int32_t *chosen);

@@ -851,7 +851,7 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
     if (!rc) rc = lease.rc;
     const void *X = eval_bar;
     int buf = 0;
-    static const int kCand[] = {8, 12, 16, 24, 32, 48, 64};
+    static const int kCand[] = {0, 8, 12, 16, 24, 32, 48, 64};  // 0: the size chosen without tuning
     for (int k = d.nin - 1; k >= 0 && !rc; --k) {
         AxisPass a = axis_pass(d, p, k, derivative_order);
         a.X = X;
@@ -866,7 +866,7 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
             float best = 3.4e38f;
             int best_cc = 0;
             for (int c = 0; c < (int)(sizeof(kCand) / sizeof(kCand[0])) && !rc; ++c) {
-                if (kCand[c] > a.n && c > 0) break;
+                if (kCand[c] > a.n && c > 1) break;
                 a.cc = kCand[c];
                 float ms[3];
                 for (int r = 0; r < 3 && !rc; ++r) {

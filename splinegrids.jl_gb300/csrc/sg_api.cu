@@ -704,11 +704,18 @@ extern "C" int sg_evaluate_multi(sg_grid_plan *p, int32_t n_orders, const int32_
     return rc ? rc : rc2;
 }
 
+// The adjoint pass over axis k.
+static int adjoint_pass(const sg_grid_plan *p, const AxisPass &a, int k, cudaStream_t s) {
+    const bool f64 = p->desc.dtype == SG_F64;
+    if (k > 0) return f64 ? adj_axis_f64(a, s) : adj_axis_f32(a, s);
+    if (p->line_support) return f64 ? adj_line_f64(a, s) : adj_line_f32(a, s);
+    return f64 ? adj_axis0_f64(a, s) : adj_axis0_f32(a, s);
+}
+
 // The passes of evaluate_adjoint!, last axis first, through scratch[0] and scratch[1].
 static int separable_adjoint(sg_grid_plan *p, const int32_t *derivative_order, const void *eval_bar,
                              void *control_points_bar, void *const *scratch, cudaStream_t s, PassTimer &timer) {
     const sg_grid_desc &d = p->desc;
-    const bool f64 = d.dtype == SG_F64;
     int rc = SG_OK;
     const void *X = eval_bar;
     int buf = 0;
@@ -723,9 +730,7 @@ static int separable_adjoint(sg_grid_plan *p, const int32_t *derivative_order, c
         a.M = M;
         a.Q = Q;
         timer.begin();
-        if (k > 0) rc = f64 ? adj_axis_f64(a, s) : adj_axis_f32(a, s);
-        else if (p->line_support) rc = f64 ? adj_line_f64(a, s) : adj_line_f32(a, s);
-        else rc = f64 ? adj_axis0_f64(a, s) : adj_axis0_f32(a, s);
+        rc = adjoint_pass(p, a, k, s);
         timer.end();
         if (rc) return rc;
         X = a.Y;
@@ -837,7 +842,6 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
     if (!eval_bar || !control_points_bar)
         return set_error(SG_ERR_INVALID_ARGUMENT, "sg_grid_plan_tune: NULL array");
     cudaStream_t s = (cudaStream_t)stream;
-    const bool f64 = d.dtype == SG_F64;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     rc = cuda_check(cudaEventCreate(&e0), "tune: event");
     if (!rc) rc = cuda_check(cudaEventCreate(&e1), "tune: event");
@@ -871,7 +875,7 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
                 float ms[3];
                 for (int r = 0; r < 3 && !rc; ++r) {
                     rc = cuda_check(cudaEventRecord(e0, s), "tune: record");
-                    if (!rc) rc = f64 ? adj_axis_f64(a, s) : adj_axis_f32(a, s);
+                    if (!rc) rc = adjoint_pass(p, a, k, s);
                     if (!rc) rc = cuda_check(cudaEventRecord(e1, s), "tune: record");
                     if (!rc) rc = cuda_check(cudaEventSynchronize(e1), "tune: sync");
                     if (!rc) rc = cuda_check(cudaEventElapsedTime(&ms[r], e0, e1), "tune: time");
@@ -888,8 +892,7 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
         }
         if (chosen) chosen[k] = p->tuned_cc[k];
         // leave this pass's output in place for the next axis
-        if (!rc) rc = f64 ? (k > 0 ? adj_axis_f64(a, s) : adj_axis0_f64(a, s))
-                          : (k > 0 ? adj_axis_f32(a, s) : adj_axis0_f32(a, s));
+        if (!rc) rc = adjoint_pass(p, a, k, s);
         X = a.Y;
     }
     const int rc2 = lease.end();

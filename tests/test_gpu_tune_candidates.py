@@ -14,3 +14,18 @@ def test_tuning_can_keep_the_untuned_chunks(sg):
     cot = sg.arrays.zeros(ns + (1,), torch.float32)
     grad = sg.arrays.empty(n + (1,), torch.float32)
     assert any(sg.tune_adjoint_(g, eval=cot, control_points=grad)[2] == 0 for _ in range(3))
+
+
+@pytest.mark.parametrize("dtype_name", ["f32", "f64"])
+def test_tuning_a_curve_runs_its_adjoint(sg, dtype_name):
+    """A curve with long supports sums them with a kernel of its own, in another order than the
+    passes over several columns do; the gradient that tuning leaves behind has its bits."""
+    import torch
+    dt = torch.float64 if dtype_name == "f64" else torch.float32
+    g = sg.SplineGrid((sg.SplineDimension(15, 3, 6001, float_type=dt),), 2)
+    gen = torch.Generator().manual_seed(5)
+    cot = sg.arrays.from_any(torch.randn((6001, 2), generator=gen, dtype=torch.float64), dt)
+    want, left = sg.arrays.empty((15, 2), dt), sg.arrays.empty((15, 2), dt)
+    sg.evaluate_adjoint_(g, eval=cot, control_points=want)
+    assert sg.tune_adjoint_(g, eval=cot, control_points=left) == [0]
+    assert torch.equal(left, want)

@@ -158,7 +158,8 @@ int sg_grid_plan_untune(sg_grid_plan *plan);
  * sg_grid_plan_set_strategy(FUSED) on a grid outside it returns
  * SG_ERR_UNSUPPORTED; sg_grid_plan_paths reports the path each direction takes.  On
  * the fused path sg_grid_plan_tune times adjoint tile sizes instead of chunks
- * (chosen[1] = axis-1 control points per tile). */
+ * (chosen[1] = axis-1 control points per tile); for large grids under AUTO it times both,
+ * and chosen holds the chunks. */
 #define SG_STRATEGY_AUTO 0
 #define SG_STRATEGY_SEPARABLE 1
 #define SG_STRATEGY_FUSED 2
@@ -478,7 +479,7 @@ int sg_fit_losses(sg_fit_plan *p, sg_stream_t stream, double *latest, int64_t *c
 
 /* ------------------------------------------------------------------ test hooks */
 
-/* For tests of the failure paths only; the defaults are restored by passing -1 / 0.
+/* For tests (of the failure paths, but for the last) only; the defaults are restored by passing -1 / 0.
  * sg_test_fail_allocations: every device allocation of a plan or handle after the next
  *   `after` ones fails with SG_ERR_OUT_OF_MEMORY (after < 0: none fails);
  *   sg_test_live_allocations counts the live ones, to show that a failed create leaks
@@ -490,11 +491,14 @@ int sg_fit_losses(sg_fit_plan *p, sg_stream_t stream, double *latest, int64_t *c
  *   one tile more than its pass has (it can never complete); fused_first_stage != 0
  *   makes the fused adjoint's producer withhold its arrival on each CTA's first stage.
  *   Either way the bounded waits run out, the kernels return, and sg_batch_check /
- *   sg_grid_plan_check report SG_ERR_TIMEOUT. */
+ *   sg_grid_plan_check report SG_ERR_TIMEOUT.
+ * sg_test_fused_adjoint_launches: fused adjoints of single grids launched so far, to
+ *   show which path a call took. */
 int sg_test_fail_allocations(int64_t after);
 int64_t sg_test_live_allocations(void);
 int sg_test_set_wait_limits(int64_t batch_spin_limit, int64_t mbar_wait_cycles);
 int sg_test_block_waits(int32_t batch_dependency, int32_t fused_first_stage);
+int64_t sg_test_fused_adjoint_launches(void);
 
 #ifdef __cplusplus
 }

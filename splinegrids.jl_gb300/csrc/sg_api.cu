@@ -897,6 +897,10 @@ extern "C" int sg_grid_plan_tune(sg_grid_plan *p, const int32_t *derivative_orde
     }
     const int rc2 = lease.end();
     if (!rc) rc = rc2;
+    // AUTO calls that cannot have the intermediate (captured ones, and those beside another
+    // stream's) take the fused tiles, so these are tuned as well
+    if (!rc && use_fused(p, p->f2_adj_ok))
+        rc = tune_fused_adjoint(p, derivative_order, eval_bar, control_points_bar, s, e0, e1, nullptr);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     if (!rc) rc = cuda_check(cudaStreamSynchronize(s), "tune: sync");

@@ -2,6 +2,7 @@
 // (sg_fused2d.cuh): one launch per evaluate! / evaluate_adjoint! of a 2D grid, and the
 // batch kernels that run the fused units of many 2D grids.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "sg_fused2d_host.h"
@@ -290,6 +291,8 @@ static void set_smem(K kernel, int64_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+static std::atomic<int64_t> g_adj_launches{0};  // per-grid fused adjoints so far (a test hook reads it)
+
 template <typename T, typename TX>
 static int launch_grid_t(const F2Grid &g, const F2Tiling &t, int kind, int *status, cudaStream_t s) {
     const int64_t n = t.count();
@@ -310,6 +313,7 @@ static int launch_grid_t(const F2Grid &g, const F2Tiling &t, int kind, int *stat
         launch(k_f2_fwd_grid<T, TX>, (unsigned)blocks, kF2Lanes * kF2FwdWarps, (size_t)f2_fwd_smem<T>(), s, g, t);
     } else if constexpr (std::is_same<T, TX>::value) {
         if (n > 0x7fffffffLL) return set_error(SG_ERR_UNSUPPORTED, "fused 2D: too many tiles");
+        g_adj_launches.fetch_add(1, std::memory_order_relaxed);
         launch(k_f2_adj_grid<T>, (unsigned)n, kF2AdjThreads, (size_t)f2_adj_smem<T>(), s, g, t, status);
     }
     return cuda_check(cudaGetLastError(), "fused 2D launch");
@@ -408,3 +412,5 @@ int f2_set_withhold_first_stage(bool on) {
 }
 
 }  // namespace sg
+
+extern "C" int64_t sg_test_fused_adjoint_launches(void) { return sg::g_adj_launches.load(); }

@@ -139,6 +139,7 @@ SIGNATURES = {
     "sg_test_live_allocations": (C.c_int64, []),
     "sg_test_set_wait_limits": (C.c_int, [_i64, _i64]),
     "sg_test_block_waits": (C.c_int, [_i32, _i32]),
+    "sg_test_fused_adjoint_launches": (C.c_int64, []),
 }
 
 _lib = None

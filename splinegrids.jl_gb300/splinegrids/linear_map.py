@@ -34,22 +34,25 @@ def _copy_levels(control_points, x: torch.Tensor, out: bool) -> None:
     """Between x (flat, [n_control_points, Nout] column-major) and the levels' values, which
     are its consecutive rows; one column of one level is one copy, all issued by one
     library call."""
-    ncp, nout = control_points.n_control_points(), control_points.nout
-    vals = [lr.refinement_values for lr in control_points.local_refinements]
-    if nout * len(vals) > 64 or any(v.dtype != x.dtype or not v.is_cuda or not arrays.is_colmajor(v)
-                                    for v in vals):
+    nout = control_points.nout
+    levels = [(lr.refinement_values, lr.n_refined) for lr in control_points.local_refinements]
+    ncp = sum(n for _, n in levels)
+    assert x.numel() == ncp * nout, "the vector must hold every level's refinement values"
+    dt = x.dtype
+    if nout * len(levels) > 64 or any(v.dtype != dt or not v.is_cuda or v.shape != (n, nout)
+                                      or not arrays.is_colmajor(v) for v, n in levels):
         xm = arrays.reshape(x, (ncp, nout))
         r = 0
-        for v in vals:
-            rows = xm[r:r + v.shape[0]]
+        for v, n in levels:
+            rows = xm[r:r + n]
             (rows if out else v).copy_(v if out else rows)
-            r += v.shape[0]
+            r += n
         return
     es, x0 = x.element_size(), x.data_ptr()
     xs, vs, nb = [], [], []
     r = 0
-    for v in vals:
-        n, v0 = v.shape[0], v.data_ptr()
+    for v, n in levels:
+        v0 = v.data_ptr()
         if n:
             for o in range(nout):
                 xs.append(x0 + es * (r + ncp * o))

@@ -169,7 +169,8 @@ class LSQRSolver:
     n), applies A and A' once so that every plan the operator needs exists, and (with
     ``graph=True``) captures the solve: prologue, then one iteration as the body of a
     device-side while loop.  ``solve(b)`` then copies b into the solver's buffer and
-    launches the graph once; the host waits only when it reads the result.  Defaults
+    launches the graph once; the host waits only when it reads the result.  A solve after
+    the grid's refresh_plans() captures again.  Defaults
     follow IterativeSolvers' lsqr: atol = btol = sqrt(eps), conlim = 1/sqrt(eps),
     maxiter = max(m, n)."""
 
@@ -213,6 +214,7 @@ class LSQRSolver:
             self._V, self._G = (arrays.reshape(v, tuple(cps.shape)) for v in (self.V, self.G))
             self._F, self._U = (arrays.reshape(v, tuple(A.grid.eval.shape)) for v in (self.F, self.U))
         self.graph = False
+        self._refreshes = A.grid._refreshes
         if graph:
             self._capture()
             self.graph = True
@@ -272,6 +274,15 @@ class LSQRSolver:
                 _lib.check(lib.sg_lsqr_capture_end(self.handle, s))
         torch.cuda.current_stream(self.A.device).wait_stream(cs)
 
+    def _follow_refresh(self) -> None:
+        """The grid's plans were refreshed: so is the solver's own, and the graph, which holds
+        the addresses of the tables that the refresh replaced, is captured again."""
+        if self._adj_plan is not None:
+            self._adj_plan.refresh()
+        if self.graph:
+            self._capture()
+        self._refreshes = self.A.grid._refreshes
+
     def info(self) -> dict:
         """Iterations, stop code and the solver's norm estimates (synchronizes)."""
         counts = (C.c_int64 * 3)()
@@ -289,6 +300,8 @@ class LSQRSolver:
         if b.dim() != 1:
             b = arrays.vec(b)
         self.A._check(b, self.A.shape[0], "b")
+        if self._refreshes != self.A.grid._refreshes:
+            self._follow_refresh()
         self.B.copy_(b)
         lib = _lib.load()
         s = _lib.stream_handle()

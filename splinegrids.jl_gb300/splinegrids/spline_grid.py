@@ -59,6 +59,10 @@ class _Plan:
         self.handle = h
         self._fin = weakref.finalize(self, _lib.load().sg_grid_plan_destroy, h)
 
+    def refresh(self) -> None:
+        """Re-read the grid's sample indices."""
+        _lib.check(_lib.load().sg_grid_plan_refresh(self.handle, _lib.stream_handle()))
+
     def workspace_bytes(self) -> int:
         return int(_lib.load().sg_grid_plan_workspace_bytes(self.handle))
 
@@ -133,6 +137,7 @@ class SplineGrid:
         self.weights = weights
         self.eval = eval
         self._plans = {}
+        self._refreshes = 0  # holders of plans of their own, or of captured calls, compare it
 
     @classmethod
     def from_parts(cls, spline_dimensions, control_points, weights, eval):
@@ -182,7 +187,8 @@ class SplineGrid:
     def refresh_plans(self) -> None:
         """Re-read sample indices after set_sample_indices_ changed them."""
         for p in self._plans.values():
-            _lib.check(_lib.load().sg_grid_plan_refresh(p.handle, _lib.stream_handle()))
+            p.refresh()
+        self._refreshes += 1
 
     def __repr__(self):
         kind = "NURBSGrid" if self.is_nurbs() else "SplineGrid"

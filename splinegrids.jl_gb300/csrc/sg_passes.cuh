@@ -276,21 +276,16 @@ inline void launch_adj_thread(const AxisPass &p, cudaStream_t s) {
            (T *)p.Y);
 }
 
-// Cotangent values up to which a pass over an axis k >= 1 runs one thread per output: it
-// reads every value d + 1 times, so it loses once the pass is long enough to be bound by
-// memory ((2048, 2048): 31 us against 14; (50, 50, 25) x 4 values: 24 against 50).
-constexpr int64_t kThreadAdjValues = 1 << 20;
-
 // Control points per chunk of an adjoint pass whose units are warps (k_adj_ring,
 // k_adj_cols): per_chunk units per chunk.  A unit walks the rows of CC + d knot spans (the
 // d last ones are read again by the next chunk), every row costs it at least `lat` cycles,
 // and `per` cycles of its SM sub-partition (each has its own FP64 pipe and a quarter of the
 // SM's share of the memory bandwidth), where ceil(units / sub-partitions) units share it.
-// The chunk count with the smallest (CC + d) * max(lat, units per sub-partition * per).
+// The chunk count with the smallest (CC + d) * max(lat, units per sub-partition * per); beyond
+// 512 chunks in steps of 3 %.
 inline int64_t adj_chunk(const AxisPass &p, int64_t per_chunk, int64_t lat, int64_t per) {
     int64_t best = p.n, best_cost = INT64_MAX, prev = 0;
-    const int64_t kmax = p.n < 512 ? p.n : 512;
-    for (int64_t k = 1; k <= kmax; ++k) {
+    for (int64_t k = 1; k <= p.n; k += k < 512 ? 1 : k / 32) {
         const int64_t CC = (p.n + k - 1) / k;
         if (CC == prev) continue;
         prev = CC;
@@ -331,19 +326,87 @@ inline void launch_adj_cols(const AxisPass &p, cudaStream_t s) {
            p.lb, (const T *)p.B, p.ns, (const T *)p.X, p.M, p.n, (int)CC, gxw, chunks, units, (T *)p.Y);
 }
 
+// Warp tasks of 128 (Float64: 64) values of m x CC control points (sg_warp.cuh).
+template <typename T, int D, bool ST>
+inline void launch_adj_warp(const AxisPass &p, cudaStream_t s) {
+    const int64_t gxw = (p.M + warp_width<T>() - 1) / warp_width<T>();
+    const int64_t per_chunk = gxw * p.Q;  // tasks per chunk
+    if (per_chunk == 0) return;
+    const int64_t want_chunks = (kNumSMs * 32 * 2 + per_chunk - 1) / per_chunk;
+    int64_t CC = (p.n + want_chunks - 1) / want_chunks;
+    CC = CC < 8 ? 8 : (CC > 64 ? 64 : CC);
+    const int64_t chunks = (p.n + CC - 1) / CC;
+    const int64_t blocks = (per_chunk * chunks + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    launch(k_adj_warp<D, T, ST>, (unsigned)blocks, 32 * kWarpsPerBlock, 0, s, p.idx, p.perm, p.lb, (const T *)p.B,
+           p.ns, p.d, (const T *)p.X, p.M, p.n, p.Q, (int)CC, gxw, chunks, (T *)p.Y);
+}
+
+// The kernel of an adjoint pass over an axis k >= 1, degrees 0 to 5; all give the same bits.  S:
+// samples a control point sums.  The lines were drawn through 4500 measured passes (0.5 to 80
+// samples a control point, 2^13 to 2^25 values, rows of 1 to 10^7); us, Float32 unless said:
+//  * Rows below 24 values leave a quarter of a warp's lanes and more idle in every other kernel: one
+//    thread per output ((8, 1104301) x 2, 361168 control points, degree 3: 122, rings 299).  But a
+//    few thousand outputs with long sums leave the SMs idle: rings ((16, 5104), 112, degree 4: 21,
+//    threads 47).  And where a control point has hardly a sample, threads read each row d + 1
+//    times from far apart: warp tasks ((16, 1339501), 1079800, degree 2: 172, threads 185; (24,
+//    1068033), 1087384: 150 and 241).
+//  * Short sums (S < 9) never make up for the ring's 800 cycles a completed control point: warp tasks
+//    ((1104, 17941), 33274, degree 1: 41, rings 56; (51332, 141) x 4 Float64, 94, degree 0: 80,
+//    columns 293), or, small, one thread per output.
+//  * Float64, up to 2^13 values a row and 2^23 in all, or few values: one thread per output fills the
+//    FP64 pipe more evenly than units do ((40, 39431), 1287, degree 2: 28, columns 41).
+//  * Many columns of few samples: four warp tasks a CTA start faster than rings ((268872, 11) x 4, 4,
+//    degree 3: 19 and 23).
+//  * Unsorted samples leave rows in no order that caches like: warp tasks, which keep more of them in
+//    flight ((4792, 5542) Float64, 454, degree 1: 125, columns 418).
+//  * The others: rings (Float32 rows of 16-byte multiples; (220, 74811), 1273, degree 1: 22, warp
+//    tasks 79), columns.
+enum AdjKernel { kAdjThread, kAdjWarp, kAdjLong, kAdjGeneric };
+template <typename T>
+inline AdjKernel adj_axis_kernel(const AxisPass &p) {
+    constexpr bool f64 = sizeof(T) == 8;
+    const double S = (double)p.ns * (p.d + 1) / (double)p.n;
+    const int64_t MQ = p.M * p.Q, O = MQ * p.n, V = MQ * p.ns;
+    const bool warp = p.d <= 3, rings = !f64 && vec_width<T>(p) == 16 / (int)sizeof(T);
+    if (O > INT32_MAX || p.ns > INT32_MAX) return kAdjLong;  // k_adj_thread counts in 32 bits
+    if (p.M < 24) {
+        if (O < 12288 && S >= 32) return kAdjLong;
+        if (warp && p.M >= 8 && (f64 ? S < 2 && O >= 1 << 18 : S < 4 && O >= 1 << 20)) return kAdjWarp;
+        return kAdjThread;
+    }
+    if (S < 9) {
+        if (O < 1 << 18 && MQ < 1 << 16) return kAdjThread;
+        return warp ? kAdjWarp : kAdjLong;
+    }
+    if (f64 && (V < 1 << 18 || (MQ < 1 << 13 && V < 1 << 23))) return kAdjThread;
+    if (warp && MQ >= 1 << 18 && p.ns < 24) return kAdjWarp;
+    if (warp && !f64 && !rings && MQ >= 1 << 14 && S < 16) return kAdjWarp;
+    if (warp && p.perm && (f64 ? V >= 1 << 22 : O >= 3 << 19)) return kAdjWarp;
+    return kAdjLong;
+}
+
 template <typename T, int D>
 inline void launch_adj_axis_d(const AxisPass &p, cudaStream_t s) {
     if constexpr (D == 0) {
         launch_adj_axis_t<T, D, 1, false>(p, s);  // runtime degree: one value a thread
     } else {
-        if (p.M * p.ns * p.Q <= kThreadAdjValues && p.M * p.n * p.Q <= INT32_MAX) {
+        const bool aligned = vec_width<T>(p) == 16 / (int)sizeof(T);
+        const AdjKernel k = adj_axis_kernel<T>(p);
+        if (k == kAdjThread) {
             launch_adj_thread<T, D>(p, s);
             return;
+        }
+        if constexpr (D <= 4) {
+            if (k == kAdjWarp) {
+                if (aligned) launch_adj_warp<T, D, false>(p, s);
+                else launch_adj_warp<T, D, true>(p, s);
+                return;
+            }
         }
         if constexpr (sizeof(T) == 4) {
             // rings copy 16 bytes per lane; Float64 passes are bound by the FP64 pipe, which
             // the finer units of k_adj_cols fill more evenly
-            if (vec_width<T>(p) == 16 / (int)sizeof(T)) {
+            if (aligned) {
                 launch_adj_ring<T, D>(p, s);
                 return;
             }
@@ -383,28 +446,89 @@ inline void launch_adj_axis0_t(const AxisPass &p, cudaStream_t s) {
            (const T *)p.X, p.n, p.Q, QT, (T *)p.Y);
 }
 
-// degrees <= 5: shared-memory tiles of 32 columns x kA0Cp control points, or one thread
-// per output when half of a tile's lanes would idle or the tiles leave most SMs idle, and
-// that is the shorter: with S samples a control point, a tile's warp issues some 3 S + 300
-// instructions (425 a cycle on the whole chip) and then waits 8 cycles a sample; a thread reads
-// its samples eight at a time from L2, 88 cycles a sample, or is bound by its instructions.
-// Measured on axis 0 of (100, 10) x (100, 50), S = 4: one thread per output 6.2 us for both
-// passes, tiles 6.6; (10, 10) x (200, 50), S = 60: 13.8 and 7.9; (5, 5) x (2749, 25), S = 1649: 330
-// and 43.6.
-constexpr int64_t kA0Tiles = 64;
-inline bool a0_thread_is_shorter(const AxisPass &p, int64_t groups) {
-    const double S = (double)p.ns * (p.d + 1) / (double)p.n;
-    const double tile = (double)p.n * groups * (3 * S + 300) / 425 + 8 * S + 3000;
-    const double instr = (double)p.n * p.Q * S * 10 / (32 * 425);
-    return (88 * S > instr ? 88 * S : instr) + 2200 <= tile;
+// degrees <= 3: warp tasks of 32 columns x a chunk of control points (sg_warp.cuh); few
+// columns get short chunks (at least 4 control points) so the tasks fill the GPU
+template <typename T, int D>
+inline void launch_adj0_warp(const AxisPass &p, cudaStream_t s) {
+    const int64_t groups = (p.Q + 31) / 32;
+    if (groups == 0 || p.n == 0) return;
+    const int64_t want = (kAxis0Tasks + groups - 1) / groups;  // chunks wanted
+    int64_t CC = (p.n + want - 1) / want;
+    CC = CC < 4 ? 4 : CC;
+    const int64_t tasks = groups * ((p.n + CC - 1) / CC);
+    const int64_t blocks = (tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    const int smem = kWarpsPerBlock * warp_adj0_smem<D, T>();
+    static bool attr_set = false;  // one instance per template instantiation
+    if (!attr_set) {
+        cudaFuncSetAttribute(k_adj0_warp<D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        attr_set = true;
+    }
+    launch(k_adj0_warp<D, T>, (unsigned)blocks, 32 * kWarpsPerBlock, smem, s, p.idx, p.perm, p.lb, (const T *)p.B,
+           p.ns, p.d, (const T *)p.X, p.n, p.Q, CC, (T *)p.Y);
 }
+
+// The kernel of the adjoint pass over axis 0, degrees 0 to 5 (all give the same bits); the lines were
+// drawn through the same measurements as adj_axis_kernel's.  A tile (32 columns x kA0Cp control
+// points; kAdjLong) pays some 300 instructions a warp and a wait a segment, whatever it sums:
+//  * Short sums (S < 18, Float64 9): one thread per output (4 samples, 1748157 columns, 2 control
+//    points, degree 1: 29, tiles 149; 84462, 52, 14594: 16 and 22).  With very many outputs the
+//    threads' loads are too scattered at degrees 2 and 3, and where a control point has hardly a
+//    sample: warp tasks (12, 625777, 6, degree 3: 36 and 69; 13, 1477950, 16, degree 1: 122, 155).
+//  * Fewer than 16 columns leave half of a tile's lanes idle: one thread per output, unless its sum
+//    is long or there are few of them (Float64 182592, 3, 96247, degree 5: 16, tiles 65; 741545,
+//    12, 16121, degree 3, S = 184: 188 and 62).
+//  * Very many columns of few samples: warp tasks (20, 305766, 3, degree 2: 22, tiles 34).
+//  * Unsorted samples: warp tasks, Float32 (67104, 300, 2615, degree 2: 157, tiles 454); the
+//    CTA tiles of the runtime-degree path for degrees 4 and 5 (303904, 56, 56499, degree 4: 198, 450).
+//  * The others: tiles (10168, 192, 137, degree 3: 18, threads 75).
+template <typename T>
+inline AdjKernel adj_axis0_kernel(const AxisPass &p) {
+    constexpr bool f64 = sizeof(T) == 8;
+    const double S = (double)p.ns * (p.d + 1) / (double)p.n;
+    const int64_t O = p.n * p.Q;
+    const bool warp = p.d <= 3;
+    if (O > INT32_MAX || p.ns > INT32_MAX) return kAdjLong;  // k_adj_thread counts in 32 bits
+    const int64_t V = p.ns * p.Q;
+    if (p.perm && O >= 1 << 16 && V >= 1 << 19 && p.ns >= 12 && p.d >= 1) {
+        if (warp && !f64) return kAdjWarp;
+        if (!warp && V >= 1 << 22) return kAdjGeneric;
+    }
+    if constexpr (f64) {
+        if (S < 9) return warp && p.Q >= 16 && O >= 150000 ? kAdjWarp : kAdjThread;
+        if (p.Q < 16) return O >= 8192 && S < 4096 ? kAdjThread : kAdjLong;
+        return warp && p.ns < 16 && O >= 80000 ? kAdjWarp : kAdjLong;
+    } else {
+        if (S < 18) {
+            if (O < 12288 && S >= 8) return kAdjLong;
+            const bool scattered = (p.d >= 2 && S >= 5) || 4 * p.ns < 5 * p.n;
+            if (warp && scattered && O >= 1 << 20 && p.Q >= 32) return kAdjWarp;
+            if (warp && p.d >= 2 && p.Q >= 1 << 16) return kAdjWarp;
+            return kAdjThread;
+        }
+        if (warp && ((p.ns < 64 && p.Q >= 1 << 15) || (p.ns < 128 && p.Q >= 1 << 16))) return kAdjWarp;
+        return p.Q < 16 && O >= 1 << 17 && S < 64 ? kAdjThread : kAdjLong;
+    }
+}
+
 template <typename T, int D>
 inline void launch_adj0(const AxisPass &p, cudaStream_t s) {
     const int64_t groups = (p.Q + 31) / 32, tiles = groups * ((p.n + kA0Cp - 1) / kA0Cp);
     if (tiles == 0) return;
-    if ((p.Q < 16 || tiles < kA0Tiles) && p.n * p.Q <= INT32_MAX && a0_thread_is_shorter(p, groups)) {
+    const AdjKernel k = adj_axis0_kernel<T>(p);
+    if (k == kAdjThread) {
         launch_adj_thread<T, D>(p, s);
         return;
+    }
+    if constexpr (D <= 4) {
+        if (k == kAdjWarp) {
+            launch_adj0_warp<T, D>(p, s);
+            return;
+        }
+    } else {
+        if (k == kAdjGeneric) {
+            launch_adj_axis0_t<T, 0>(p, s);
+            return;
+        }
     }
     if constexpr (sizeof(T) == 4) {
         if (!p.perm && p.ns % 4 == 0 && (uintptr_t)p.X % 16 == 0 && (uintptr_t)p.B % 16 == 0) {

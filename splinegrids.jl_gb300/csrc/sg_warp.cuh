@@ -595,6 +595,38 @@ fwd0_warp(int64_t q0, int64_t s_begin, int64_t s_end, int lane, unsigned char *w
 // ---------------------------------------------------------------------------------
 constexpr int kWarpsPerBlock = 4;
 
+template <int D, typename T, bool ST>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+k_adj_warp(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
+           const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
+           const T *__restrict__ X, int64_t M, int64_t n, int64_t Q, int CC, int64_t gxw,
+           int64_t chunks, T *__restrict__ Y) {
+    __shared__ __align__(16) unsigned char smem[kWarpsPerBlock * warp_adj_smem<D, T>()];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w + grid_start();
+    if (task >= gxw * chunks * Q) return;
+    const int64_t mw = task % gxw, r = task / gxw;
+    adj_axis_warp<D, T, ST>(mw, r % chunks, r / chunks, lane, smem + w * warp_adj_smem<D, T>(), idx,
+                            perm, lb, B, ns, d, X, M, n, CC, Y);
+}
+
+// task = column group (fastest) x chunk of CC control points
+template <int D, typename T>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+k_adj0_warp(const int32_t *__restrict__ idx, const int32_t *__restrict__ perm,
+            const int32_t *__restrict__ lb, const T *__restrict__ B, int64_t ns, int d,
+            const T *__restrict__ X, int64_t n, int64_t Q, int64_t CC, T *__restrict__ Y) {
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t task = (int64_t)blockIdx.x * kWarpsPerBlock + w + grid_start();
+    const int64_t groups = (Q + 31) / 32, chunks = (n + CC - 1) / CC;
+    if (task >= groups * chunks) return;
+    const int64_t cg = task % groups, c_lo = (task / groups) * CC;
+    const int64_t c_hi = c_lo + CC < n ? c_lo + CC : n;
+    adj0_warp<D, T>(cg * 32, c_lo, c_hi, lane, s_dyn + w * warp_adj0_smem<D, T>(), idx, perm, lb,
+                    B, ns, d, X, n, Q, Y);
+}
+
 // task = column group (fastest) x chunk of SC samples
 template <int D, typename T>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)

@@ -153,8 +153,9 @@ int sg_grid_plan_untune(sg_grid_plan *plan);
  * in device memory (its adjoint also needs sorted samples on both axes).  Both give
  * bitwise identical results.  SG_STRATEGY_AUTO (the default) takes the fused path
  * wherever it applies, but for the adjoint of large grids with long rows (2^21 values
- * and more, rows of two adjoint tiles and more), which runs separably unless its call is
- * being captured or another stream is still using the plan's intermediate.
+ * and more, rows of two adjoint tiles and more) that is estimated to be faster in two
+ * passes, and then runs so unless its call is being captured or another stream is still
+ * using the plan's intermediate.
  * sg_grid_plan_set_strategy(FUSED) on a grid outside it returns
  * SG_ERR_UNSUPPORTED; sg_grid_plan_paths reports the path each direction takes.  On
  * the fused path sg_grid_plan_tune times adjoint tile sizes instead of chunks

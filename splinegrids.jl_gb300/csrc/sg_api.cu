@@ -180,6 +180,50 @@ static int validate_desc(const sg_grid_desc *d) {
 // axis-0 supports that fit a tile.  The grid runs alone, so the tilings are sized for
 // whole waves of the resident units.
 constexpr int64_t kSeparableAdjValues = 1 << 21;
+
+// Estimates, in us, of a large grid's adjoint as fused tiles (chunks along axis 0, one channel a
+// tile) and as two passes.  The terms are what bounds each part; the factors were fitted to 2700
+// measured grids of 2^21 to 2^26 values, 1.3 to 150 samples a control point along either axis
+// (standard deviation of the quotient 12 to 19 %).
+//   Fused, a wave of tiles after the other: a tile's set-up, its rows (a fixed latency each, and the
+//   FMAs; Float64: the pipe), its halves of four columns (a barrier, and the longest chain of a
+//   thread's sums) and the other sums; or the bytes that all tiles read.
+//   Separable: the units of the first pass (adj_chunk's cycles a row) or its bytes; of the second
+//   the tiles' waves, the samples a tile stages, the longest sum, and the intermediate's bytes and FMAs.
+static double fused_adjoint_us(const sg_grid_desc &d, const std::vector<int32_t> &lb0, const F2Tiling &t, int slots) {
+    const bool f64 = d.dtype == SG_F64;
+    const double ns0 = (double)d.n_samples[0], ns1 = (double)d.n_samples[1], r1 = ns1 / (double)d.n_basis[1];
+    const double S0 = std::min(ns0, ns0 * (d.degree[0] + 1) / (double)d.n_basis[0]);
+    const double rows = std::min(ns1, (t.kb + d.degree[1]) * r1);
+    const double waves = (double)((t.count() + slots - 1) / slots), halves = (double)((t.kb + 3) / 4);
+    const double chain = S0 * std::max(1.0, 2.0 * t.ka / 256), sums = t.kb * (double)t.ka * S0 / 256;
+    double samples = 0;  // of axis 0, read by all chunks
+    for (int64_t a = 0; a < d.n_basis[0]; a += t.ka)
+        samples += lb0[std::min<int64_t>(a + t.ka, d.n_basis[0]) + d.degree[0]] - lb0[a];
+    const double mb = samples * rows * t.nbb * d.nout * (f64 ? 8e-6 : 4e-6);
+    const double tile = f64 ? 0.72 + rows * (0.009 + 0.254 * (d.degree[1] + 1)) + halves * (0.58 + 0.071 * chain) + 0.0885 * sums
+                            : 2.0 + rows * (0.113 + 0.0158 * (d.degree[1] + 1)) + halves * (0.43 + 0.0084 * chain) + 0.0225 * sums;
+    return (f64 ? 3.4 : 2.7) + std::max(waves * tile, mb / 5.5);
+}
+static double separable_adjoint_us(const sg_grid_desc &d) {
+    const bool f64 = d.dtype == SG_F64;
+    const double ns0 = (double)d.n_samples[0], ns1 = (double)d.n_samples[1], n0 = (double)d.n_basis[0];
+    AxisPass a;
+    a.n = d.n_basis[1];
+    a.d = d.degree[1];
+    const int64_t per_chunk = d.nout * (f64 ? (d.n_samples[0] + 31) / 32 : (d.n_samples[0] + 127) / 128);
+    const int D1 = d.degree[1] + 1;
+    int64_t cycles = 0;
+    adj_chunk(a, per_chunk, f64 ? 64 * D1 + kColsLat : kRingLat, f64 ? 64 * D1 : kRingPer, &cycles);
+    const double pass1 = (double)cycles * ns1 / (double)d.n_basis[1] / 2000 * (f64 ? 1.07 : 1.0);
+    const double S0 = ns0 * (d.degree[0] + 1) / n0, staged = S0 + (kA0Cp - 1) * ns0 / n0;
+    const int64_t Q = d.n_basis[1] * d.nout, tiles = (Q + 31) / 32 * ((d.n_basis[0] + kA0Cp - 1) / kA0Cp);
+    const double waves = (double)((tiles + kNumSMs * 6 - 1) / (kNumSMs * 6)), mid = ns0 * (double)Q * 1e-6;
+    const double pass2 = f64 ? (waves * (61 * staged + 2300) + 141 * S0) / 2000 + mid * (1.25 + 1.07 * (d.degree[0] + 1))
+                             : (waves * (7.2 * staged + 3100) + 40 * S0) / 2000 + mid * (1.09 + 0.25 * (d.degree[0] + 1));
+    return (f64 ? 5.3 : 2.8) + std::max(pass1, ns0 * ns1 * d.nout * (f64 ? 8e-6 : 4e-6) / 5.5) + pass2;
+}
+
 static void plan_fused_tilings(sg_grid_plan *p) {
     const sg_grid_desc &d = p->desc;
     p->f2_fwd_ok = p->f2_adj_ok = p->f2_adj_skip = false;
@@ -205,13 +249,23 @@ static void plan_fused_tilings(sg_grid_plan *p) {
                                          f2_align_elems(dt), p->f2_adj_target,
                                          p->f2_adj_target > 0 ? 0 : f2_slots(dt, 1),
                                          p->f2_adj);
-    // AUTO: rows of two tiles and more would be cut into chunks, and chunks along both axes
-    // re-read (and re-sum) their neighbours' boundary spans.  From kSeparableAdjValues on,
-    // two passes are faster: their axis-1 units have a halo along one axis only, and the
-    // intermediate (n1 / ns1 of the cotangent) stays in L2.  (4096, 4096) x 3: Float32 52 us
-    // against 66, Float64 460 against 527; (2048, 2048): 12 against 23.
-    p->f2_adj_skip = p->f2_adj_ok && d.n_samples[0] >= 2 * np &&
-                     d.n_samples[0] * d.n_samples[1] * d.nout >= kSeparableAdjValues;
+    // AUTO: rows of two tiles and more are cut into chunks, and chunks along both axes re-read (and
+    // re-sum) their neighbours' boundary spans.  From kSeparableAdjValues on, two passes, whose
+    // axis-1 units have a halo along one axis only, are often faster: (4096, 4096) x 3, 256 control
+    // points an axis, degree 3: Float32 49 us, fused 59; Float64 466 and 522.  They lose where the
+    // intermediate (n1 / ns1 of the cotangent) is a large part of it, or a control point has many
+    // samples on axis 0 and few on axis 1: (32768, 1024), (8192, 256), degree 2: 62 and 37; (4096,
+    // 513), (40, 171), degree 3: 23 and 16.  By the estimates 100 of 2364 such Float32 grids and 74
+    // of 1136 Float64 are more than 10 % slower than the other way (two passes for all: 615 and
+    // 111, tiles for all: 1194 and 772).
+    p->f2_adj_skip = false;
+    if (p->f2_adj_ok && d.n_samples[0] >= 2 * np && d.n_samples[0] * d.n_samples[1] * d.nout >= kSeparableAdjValues) {
+        F2Tiling t = p->f2_adj;  // untuned, so that tuning does not change the path
+        if (p->f2_adj_target > 0)
+            f2_adjoint_tiling(p->lb0_host.data(), d.n_basis[0], d.degree[0], d.n_samples[0], d.n_basis[1], d.degree[1],
+                              d.n_samples[1], d.nout, np, f2_align_elems(dt), 0, f2_slots(dt, 1), t);
+        p->f2_adj_skip = separable_adjoint_us(d) < fused_adjoint_us(d, p->lb0_host, t, f2_slots(dt, 1));
+    }
     if (p->f2_adj_skip && !p->scratch_done &&
         cudaEventCreateWithFlags(&p->scratch_done, cudaEventDisableTiming) != cudaSuccess) {
         (void)cudaGetLastError();

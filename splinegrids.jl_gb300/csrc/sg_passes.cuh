@@ -282,8 +282,8 @@ inline void launch_adj_thread(const AxisPass &p, cudaStream_t s) {
 // and `per` cycles of its SM sub-partition (each has its own FP64 pipe and a quarter of the
 // SM's share of the memory bandwidth), where ceil(units / sub-partitions) units share it.
 // The chunk count with the smallest (CC + d) * max(lat, units per sub-partition * per); beyond
-// 512 chunks in steps of 3 %.
-inline int64_t adj_chunk(const AxisPass &p, int64_t per_chunk, int64_t lat, int64_t per) {
+// 512 chunks in steps of 3 %.  cost_out: that product.
+inline int64_t adj_chunk(const AxisPass &p, int64_t per_chunk, int64_t lat, int64_t per, int64_t *cost_out = nullptr) {
     int64_t best = p.n, best_cost = INT64_MAX, prev = 0;
     for (int64_t k = 1; k <= p.n; k += k < 512 ? 1 : k / 32) {
         const int64_t CC = (p.n + k - 1) / k;
@@ -297,6 +297,7 @@ inline int64_t adj_chunk(const AxisPass &p, int64_t per_chunk, int64_t lat, int6
             best = CC;
         }
     }
+    if (cost_out) *cost_out = best_cost;
     return p.cc > 0 && per_chunk * ((p.n + p.cc - 1) / p.cc) <= INT32_MAX ? p.cc : best;  // cc: measured by sg_grid_plan_tune
 }
 // Cycles of adj_chunk's model, fitted to sweeps on (256, 256) x (4096, 4096) x 3,

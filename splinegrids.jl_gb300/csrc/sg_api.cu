@@ -238,7 +238,7 @@ static void plan_fused_tilings(sg_grid_plan *p) {
                                d.nout, f2_tile_cols(dt), 0, f2_slots(dt, 2), p->f2_fwd)) {
         p->f2_fwd_ok = true;
         p->f2_fwd_kind = 2;
-        p->f2_fwd_stage = !p->perm[0] && p->f2_fwd.count() > f2_slots(dt, 2);
+        p->f2_fwd_stage = dt == SG_F64 && !p->perm[0] && p->f2_fwd.count() > f2_slots(dt, 2);
     } else {
         p->f2_fwd_ok = f2_forward_tiling(d.n_samples[0], d.n_samples[1], d.nout, 0, f2_slots(dt, 0),
                                          p->f2_fwd);

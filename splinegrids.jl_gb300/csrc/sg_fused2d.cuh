@@ -108,8 +108,11 @@ struct F2Grid {
     int64_t ns0, ns1, n0, n1;
     int32_t d0, d1, nch;
     // forward tiles: stage the tile's control points (axis-0 samples sorted, and more tiles
-    // than fit the GPU at once, so that loads wait behind other tiles' stores; a single
-    // wave loses 0.4 us to the extra barrier)
+    // than fit the GPU at once, so that loads wait behind other tiles' stores).  One grid alone:
+    // Float64 only ((60556, 278), 4409 x 107 control points: 88 us per sample, 84 staged; (4096, 4096)
+    // x 3 390 and 388).  In Float32, with launches that overlap their set-up, the staging's
+    // barrier costs 1 to 3 % of tiles of many rows and up to 25 % of tiles of few ((4096, 4096) x 3
+    // 31.6 and 32.0 us, from bfloat16 31.8 and 32.4; (679264, 5) x 3 44 and 58).
     int32_t stage;
 };
 
@@ -835,7 +838,7 @@ __device__ __forceinline__ void f2_forward_tile(const F2Grid &g, const F2Tile &t
     // its columns, a few hundred values when axis 0 is sorted), its axis-0 basis rows and the
     // rows' headers are all fetched at once, and Y is formed from the staged block.  Larger
     // blocks and unsorted samples read the control points per sample instead.  Measured, per
-    // sample against staged: (4096, 4096) x 3 35.7 and 32.1 us; 32 grids x 16 sets 292 and 280.
+    // sample against staged: 32 grids x 16 sets 292 and 280 us; one grid alone at F2Grid::stage.
     const int pa = tl.na > 0 ? tl.pa : (g.stage ? (int)support_start(g.idx0[tl.a_lo], g.d0, (int)g.n0) : 0);
     const int na = tl.na > 0 ? tl.na
                  : g.stage ? (int)support_start(g.idx0[tl.a_lo + tl.a_len - 1], g.d0, (int)g.n0) + g.d0 + 1 - pa : 0;

@@ -34,7 +34,7 @@ __device__ __forceinline__ void row_extent(const MultArgs &a, int r, int64_t i, 
 // product of the row bands in the reference's order (first dim fastest) with the factors
 // multiplied in dim order.
 template <typename T>
-__device__ __noinline__ T mult_entry(const MultArgs &a, const T *__restrict__ B, int64_t lin) {
+__device__ __forceinline__ T mult_entry(const MultArgs &a, const T *__restrict__ B, int64_t lin) {
     int64_t c0[kMaxDims], nc[kMaxDims], z0[kMaxDims], Jb[kMaxDims];
     int64_t rem = lin, tot = 1;
     for (int dd = 0; dd < a.ndims; ++dd) {
@@ -73,6 +73,12 @@ __device__ __noinline__ T mult_entry(const MultArgs &a, const T *__restrict__ B,
     return out;
 }
 
+// The same as a call: what a kernel falls back on costs it no registers.
+template <typename T>
+__device__ __noinline__ T mult_entry_call(const MultArgs &a, const T *__restrict__ B, int64_t lin) {
+    return mult_entry(a, B, lin);
+}
+
 // refinement_matrix_array_mul_kernel (src/refinement_matrix.jl:365-403): one thread per
 // entry of Y.
 template <typename T>
@@ -109,7 +115,7 @@ __device__ __forceinline__ void rows_covering(const MultArgs &a, int r, int64_t 
 // Y[I] prod A[I_d, J_d] over the rows I whose bands cover J, in a fixed order (first dim
 // fastest).
 template <typename T>
-__device__ __noinline__ T mult_adjoint_entry(const MultArgs &a, const T *__restrict__ Y, int64_t lin) {
+__device__ __forceinline__ T mult_adjoint_entry(const MultArgs &a, const T *__restrict__ Y, int64_t lin) {
     int64_t J[kMaxDims], lo[kMaxDims], cnt[kMaxDims], Ib[kMaxDims];
     int64_t rem = lin, tot = 1;
     for (int dd = 0; dd < a.ndims; ++dd) {
@@ -174,7 +180,7 @@ __global__ void k_mult_adjoint(MultArgs a, const T *__restrict__ Y, T *__restric
 // times as long.  Terms, factors and roundings are those of the general kernels.  Measured, us,
 // general kernels / one sum for all / now: (58, 58, 26) -> (114, 114, 50), bands of 2, Float32:
 // mult! 46 / 22 / 11.8, mult_adjoint! 79 / 17 / 12.6; bands of 3: 122 / - / 15, 231 / 286 / 39;
-// (257, 257) x 3 -> (512, 512) x 3, bands of 3, Float64: 54 / 75 / 43, 73 / 114 / 65.
+// (257, 257) x 3 -> (511, 511) x 3, bands of 3, Float64, general / now: 51 / 39, 56 / 41.
 // ---------------------------------------------------------------------------------
 constexpr int kMultThreads = 128;
 
@@ -287,35 +293,55 @@ __device__ __forceinline__ T nd_sum_any(const T *__restrict__ X, const int (&n)[
     return acc;
 }
 
-// The narrowest of the sums that holds every band of the warp's threads (the vote keeps the
-// warp in one of them): a term that a thread does not have costs it as much as one it has.
-// A row of a bisected dimension has degree / 2 + 1 columns at most, a column degree + 2 rows.
+// The narrowest of the unrolled sums that holds every band of the warp's threads, or the loops (the
+// vote keeps the warp in one of them).  A row of a bisected dimension has degree / 2 + 1 columns at
+// most, a column degree + 2 rows.
+//  * Float32: unrolled, also where bands of other widths leave terms out ((50, 40, 54) x 2, degrees 2, 3,
+//    2: 30 us, loops 45).
+//  * Float64: a term that a thread does not have costs it as much as one it has, on a pipe that is the
+//    bound.  mult! (ROWS) takes the loops ((33, 55, 50) x 3, degrees 1, 0, 4: 114 us, unrolled 407;
+//    equal bands of 2 and 3: 8 and 8); mult_adjoint!, whose factors' look-ups are longer, the unrolled
+//    sums while at most half of their terms are missing ((32, 59, 65) x 2, degrees 0, 1, 3: loops 74,
+//    unrolled 240; (12, 12, 12) x 2, degrees 2, 3, 3: 44 and 27).
 // last: the last dimension is refined (Nout is not: no factors of one are multiplied); that takes
 // the loops, for the unrolled sums of ND dimensions as well would cost the kernel registers.
-template <int NR, typename T, int ND, typename F>
+template <int NR, bool ROWS, typename T, int ND, typename F>
 __device__ __forceinline__ T nd_sum_n(const T *__restrict__ x, const int (&n)[ND], const int64_t (&st)[ND], F f) {
-    int widest = n[0];
+    if constexpr (sizeof(T) == 8 && ROWS) {
+        return nd_sum_any<NR>(x, n, st, f);
+    } else {
+        unsigned widest = n[0], terms = n[0];
 #pragma unroll
-    for (int d = 1; d < NR; ++d) widest = n[d] > widest ? n[d] : widest;
-    const int cap = (int)__reduce_max_sync(__activemask(), (unsigned)widest);
-    if (cap <= 2) return nd_sum_c<2, NR>(x, n, st, f);
-    if (cap <= 3) return nd_sum_c<3, NR>(x, n, st, f);
-    if (cap <= 4) return nd_sum_c<4, NR>(x, n, st, f);
-    if (cap <= 5) return nd_sum_c<5, NR>(x, n, st, f);
-    return nd_sum_any<NR>(x, n, st, f);
+        for (int d = 1; d < NR; ++d) {
+            widest = (unsigned)n[d] > widest ? n[d] : widest;
+            terms *= n[d];
+        }
+        const unsigned cap = __reduce_max_sync(__activemask(), widest);
+        if constexpr (sizeof(T) == 8) {
+            unsigned all = cap;
+#pragma unroll
+            for (int d = 1; d < NR; ++d) all *= cap;
+            if (cap > 5 || all > 2 * __reduce_max_sync(__activemask(), terms)) return nd_sum_any<NR>(x, n, st, f);
+        }
+        if (cap <= 2) return nd_sum_c<2, NR>(x, n, st, f);
+        if (cap <= 3) return nd_sum_c<3, NR>(x, n, st, f);
+        if (cap <= 4) return nd_sum_c<4, NR>(x, n, st, f);
+        if (cap <= 5) return nd_sum_c<5, NR>(x, n, st, f);
+        return nd_sum_any<NR>(x, n, st, f);
+    }
 }
-template <typename T, int ND, typename F>
+template <bool ROWS, typename T, int ND, typename F>
 __device__ __forceinline__ T nd_sum(const T *__restrict__ X, const int64_t (&lo)[ND], const int (&n)[ND],
                                     const int64_t (&st)[ND], bool last, F f) {
     const T *x = X;
 #pragma unroll
     for (int d = 0; d < ND; ++d) x += lo[d] * st[d];
-    if (!last) return nd_sum_n<ND - 1>(x, n, st, f);
+    if (!last) return nd_sum_n<ND - 1, ROWS>(x, n, st, f);
     return nd_sum_any<ND>(x, n, st, f);
 }
 
 template <typename T, int ND>
-__global__ void __launch_bounds__(kMultThreads, sizeof(T) == 4 ? 6 : 4)
+__global__ void __launch_bounds__(kMultThreads, 6)
 k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, int64_t NY, bool small) {
     const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NY) return;
@@ -339,7 +365,7 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
         }
     }
     if (!fits) {
-        Y[lin] = mult_entry(a, B, lin);
+        Y[lin] = mult_entry_call(a, B, lin);
         return;
     }
     auto f = [&](int d, int k) {
@@ -349,11 +375,11 @@ k_mult_nd(MultNd<ND> p, MultArgs a, const T *__restrict__ B, T *__restrict__ Y, 
             if (e == d && p.rp[e]) r = ((const T *)p.nz[e])[z0[e] + k];
         return r;
     };
-    Y[lin] = nd_sum(B, c0, n, st, p.rp[ND - 1] != nullptr, f);
+    Y[lin] = nd_sum<true>(B, c0, n, st, p.rp[ND - 1] != nullptr, f);
 }
 
 template <typename T, int ND>
-__global__ void __launch_bounds__(kMultThreads, sizeof(T) == 4 ? 6 : 4)
+__global__ void __launch_bounds__(kMultThreads, 6)
 k_mult_adjoint_nd(MultNd<ND> p, const T *__restrict__ Y, T *__restrict__ B, int64_t NB, bool small) {
     const int64_t lin = blockIdx.x * (int64_t)kMultThreads + threadIdx.x + grid_start();
     if (lin >= NB) return;
@@ -416,7 +442,7 @@ k_mult_adjoint_nd(MultNd<ND> p, const T *__restrict__ Y, T *__restrict__ B, int6
             }
         return r;
     };
-    B[lin] = nd_sum(Y, lo, n, st, p.rp[ND - 1] != nullptr, f);
+    B[lin] = nd_sum<false>(Y, lo, n, st, p.rp[ND - 1] != nullptr, f);
 }
 
 struct RefIdx {

@@ -1,5 +1,6 @@
-// sg_ring.cuh -- per-grid adjoint passes: an axis k >= 1 as warp-private cp.async rings,
-// axis 0 as shared-memory tiles, and one thread per output for the small ones.
+// sg_ring.cuh -- per-grid adjoint passes: an axis k >= 1 as warp-private cp.async rings or columns,
+// axis 0 as shared-memory tiles, and one thread per output for short sums and small passes.
+// (Which runs, and where the warp tasks of sg_warp.cuh do: adj_axis_kernel, adj_axis0_kernel.)
 //
 // Unless said otherwise they sum the samples of a control point from zero in increasing
 // view order, one FMA per sample: the order (and so the bits) of the other adjoint kernels.
@@ -23,7 +24,7 @@ namespace sg {
 // halo, read twice) stay a small part of it.  Support starts come from the support
 // table (the position where the next control point completes is a register compare per
 // row); basis rows are staged 32 at a time, one per lane.
-// Measured on (256, 256) -> (4096, 4096), 3 channels, Float32 (201 MB): 40 us, 5.0 TB/s plus
+// Measured on (256, 256) -> (4096, 4096), 3 channels, Float32 (201 MB): 42 us, 5.4 TB/s with
 // the halo's 12 % (the 1024-wide stream tiles of the batch queue: 56 us; a copy: 30 us).
 // What is left is the rows around completed control points and the halo.
 // ---------------------------------------------------------------------------------
@@ -549,9 +550,9 @@ k_adj_line(const int32_t *__restrict__ perm, const int32_t *__restrict__ lb, con
 }
 
 // ---------------------------------------------------------------------------------
-// Small passes, one thread per output: no staging, no windows, every load independent.
-// With few outputs the warp tasks of sg_warp.cuh leave most SMs idle and each warp is a
-// chain of dependent steps.  The adjoint form takes any axis (M = 1 for axis 0).
+// One thread per output: no staging, no windows, every load independent.  With few outputs the
+// warp tasks of sg_warp.cuh leave most SMs idle and each warp is a chain of dependent steps; with
+// short sums or short rows there is little for any staging to share.  The adjoint form takes any axis (M = 1 for axis 0).
 // Measured on the (10, 10, 5) -> (50, 50, 25) x 4 volume, Float64: forward 24 -> 7 us, adjoint
 // 50 -> 24 us (three passes each).
 // ---------------------------------------------------------------------------------

@@ -82,8 +82,10 @@ class _Plan:
         _lib.check(_lib.load().sg_grid_plan_check(self.handle, _lib.stream_handle()))
 
     def tune(self, derivative_order, eval_bar: torch.Tensor, control_points_bar: torch.Tensor):
-        """Time the adjoint stream's chunk-size candidates on these arrays (scratch) and
-        keep the fastest per axis; returns the choice per axis (0: heuristic)."""
+        """Time the adjoint's candidate chunk sizes (separable passes), tile sizes (fused) or both
+        (a large 2D grid under "auto") on these arrays, which serve as scratch, and keep the
+        fastest.  Returns the chunk size per axis (0: the heuristic's), or for a fused adjoint
+        the axis-1 control points per tile."""
         chosen = (C.c_int32 * _lib.SG_MAX_NIN)()
         _lib.check(_lib.load().sg_grid_plan_tune(
             self.handle, _lib.i32_array(derivative_order), arrays.ptr(eval_bar, "eval"),
@@ -96,12 +98,16 @@ class _Plan:
     STRATEGIES = {"auto": 0, "separable": 1, "fused": 2}
 
     def set_strategy(self, strategy: str) -> None:
-        """"auto" (fused wherever it applies), "separable" (one launch per axis) or
-        "fused" (Nin = 2: both axes in one launch); results are bitwise the same."""
+        """"separable" (one launch per axis), "fused" (Nin = 2: both axes in one launch) or "auto";
+        results are bitwise the same.  "auto" is fused wherever that applies, but for the
+        adjoint of grids of 2^21 values and more, with rows of two adjoint tiles and more, that is
+        estimated to be faster in two passes.  Such an adjoint still runs fused while it is
+        being captured into a CUDA graph, and while another stream uses the plan's intermediate."""
         _lib.check(_lib.load().sg_grid_plan_set_strategy(self.handle, self.STRATEGIES[strategy]))
 
     def paths(self) -> tuple:
-        """The path ("separable" / "fused") of evaluate and of evaluate_adjoint."""
+        """The path ("separable" / "fused") of evaluate and of evaluate_adjoint.  Under "auto" a
+        separable adjoint is that of an ordinary call: see ``set_strategy`` for the others."""
         f, a = C.c_int32(), C.c_int32()
         _lib.check(_lib.load().sg_grid_plan_paths(self.handle, C.byref(f), C.byref(a)))
         names = {1: "separable", 2: "fused"}

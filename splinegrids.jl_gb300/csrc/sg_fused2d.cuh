@@ -108,11 +108,14 @@ struct F2Grid {
     int64_t ns0, ns1, n0, n1;
     int32_t d0, d1, nch;
     // forward tiles: stage the tile's control points (axis-0 samples sorted, and more tiles
-    // than fit the GPU at once, so that loads wait behind other tiles' stores).  One grid alone:
-    // Float64 only ((60556, 278), 4409 x 107 control points: 88 us per sample, 84 staged; (4096, 4096)
-    // x 3 390 and 388).  In Float32, with launches that overlap their set-up, the staging's
-    // barrier costs 1 to 3 % of tiles of many rows and up to 25 % of tiles of few ((4096, 4096) x 3
-    // 31.6 and 32.0 us, from bfloat16 31.8 and 32.4; (679264, 5) x 3 44 and 58).
+    // than fit the GPU at once, so that loads wait behind other tiles' stores).  One grid alone,
+    // with launches that overlap their set-up: all such Float64 grids ((60556, 278), 4409 x 107
+    // control points: 88 us per sample, 84 staged; (4096, 4096) x 3 390 and 388).  In Float32 the
+    // extra barrier costs tiles of few columns and rows up to 25 % ((679264, 5) x 3 44 and 58), blocks
+    // too large to be staged 2 %, and rows off the 16-byte boundaries 2 %; tiles of 32
+    // columns and more of aligned rows gain up to 10 % ((5688, 1912) x 8, 107 x 1610: 106 and 96;
+    // three orders of (6000, 300) x 4, 200 x 200: 30.5 and 28.7).  From bfloat16 it gains nothing
+    // ((4096, 4096) x 3 31.8 and 32.4).
     int32_t stage;
 };
 

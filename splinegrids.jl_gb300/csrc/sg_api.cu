@@ -239,8 +239,7 @@ static void plan_fused_tilings(sg_grid_plan *p) {
         p->f2_fwd_ok = true;
         p->f2_fwd_kind = 2;
         // (see F2Grid::stage; a tile's columns, and the control points along axis 0 of its samples)
-        const double cols = std::min<double>(f2_tile_cols(dt), p->f2_fwd.kb * (double)d.n_basis[1] / (double)d.n_samples[1] +
-                                                                   d.degree[1] + 1);
+        const double cols = p->f2_fwd.kb * (double)d.n_basis[1] / (double)d.n_samples[1] + d.degree[1] + 1;
         const double along = kF2TileS0 * (double)d.n_basis[0] / (double)d.n_samples[0] + d.degree[0] + 1;
         const bool gains = d.dtype == SG_F64 || (d.dtype == SG_F32 && d.n_samples[0] % 4 == 0 && cols >= 32 &&
                                                  cols * along <= 1.05 * kF2TileBlock);  // (the kernel decides by the tile)

@@ -241,7 +241,8 @@ static void plan_fused_tilings(sg_grid_plan *p) {
         // (see F2Grid::stage; a tile's columns, and the control points along axis 0 of its samples)
         const double cols = p->f2_fwd.kb * (double)d.n_basis[1] / (double)d.n_samples[1] + d.degree[1] + 1;
         const double along = kF2TileS0 * (double)d.n_basis[0] / (double)d.n_samples[0] + d.degree[0] + 1;
-        const bool gains = d.dtype == SG_F64 || (d.dtype == SG_F32 && d.n_samples[0] % 4 == 0 && cols >= 32 &&
+        const bool gains = d.dtype == SG_F64 || (d.dtype == SG_F32 && d.n_samples[0] % 4 == 0 &&
+                                                 cols >= (p->f2_fwd.kb >= 180 ? 16 : 32) &&
                                                  cols * along <= 1.05 * kF2TileBlock);  // (the kernel decides by the tile)
         p->f2_fwd_stage = gains && !p->perm[0] && p->f2_fwd.count() > f2_slots(dt, 2);
     } else {

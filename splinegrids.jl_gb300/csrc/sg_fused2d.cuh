@@ -113,7 +113,9 @@ struct F2Grid {
     // control points: 88 us per sample, 84 staged; (4096, 4096) x 3 390 and 388).  In Float32 the
     // extra barrier costs tiles of few columns and rows up to 25 % ((679264, 5) x 3 44 and 58), blocks
     // too large to be staged 2 %, and rows off the 16-byte boundaries 2 %; tiles of 32
-    // columns and more of aligned rows gain up to 10 % ((5688, 1912) x 8, 107 x 1610: 106 and 96).
+    // columns and more of aligned rows gain up to 10 % ((5688, 1912) x 8, 107 x 1610: 106 and 96).  With 180
+    // rows and more, 16 columns are enough: as fast alone, and what follows is faster (three orders
+    // both ways of (4096, 4096) x 3 255.7 and 253.3).
     // From bfloat16 it gains nothing ((4096, 4096) x 3 31.8 and 32.4).
     int32_t stage;
 };

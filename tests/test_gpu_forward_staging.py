@@ -10,6 +10,7 @@ SHAPES = [
     ((100, 1600), (3, 2), (5600, 1900), 1, True),
     ((64, 2300), (2, 0), (2228, 3800), 3, True),
     ((64, 2300), (2, 0), (2229, 3800), 3, True),  # rows off the 16-byte boundaries
+    ((256, 256), (3, 3), (4096, 4096), 1, True),   # long tiles of some 20 columns
     ((2000, 600), (3, 2), (4096, 1000), 1, True),  # blocks too large
     ((200, 200), (3, 3), (6000, 300), 4, False),
     ((300, 3), (2, 2), (200000, 5), 1, True),     # few rows
